@@ -89,7 +89,11 @@ typedef struct ptw_walk_stats {
     float total_ms;    /* device time of the whole call, copies included */
 } ptw_walk_stats;
 
-/* Launch parameters of the walk kernels (chosen by ptw_autotune). */
+/* Launch parameters of the walk kernels (chosen by ptw_autotune).  A graph is
+ * built with block 256, ilp 2, chunk 256, paths_ilp 2, cache_hints 1,
+ * paths_named 1 and zeros; while the fields that count and endpoint walks
+ * read have these values, the library picks kernel, column layout and launch
+ * of those walks by their number of walkers. */
 typedef struct ptw_tune {
     int32_t block;         /* threads per block (multiple of 32) */
     int32_t ilp;           /* walkers held per thread: 1, 2 or 4 */

@@ -289,7 +289,9 @@ int check_cfg(const ptw_graph *g, const ptw_walk_cfg *cfg, bool needs_sp)
 }
 
 // Maps source names to internal ids and uploads them to the scratch table.
-int upload_sources(ptw_graph *g, const ptw_walk_cfg *cfg)
+// With `only`, a single source's id is stored there instead (it travels as a
+// kernel argument, without a copy to wait for).
+int upload_sources(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *only = nullptr)
 {
     if (cfg->start_mode != PTW_START_SOURCES) return PTW_OK;
     const uint32_t n = g->dg.n;
@@ -300,6 +302,10 @@ int upload_sources(ptw_graph *g, const ptw_walk_cfg *cfg)
         if (p == g->h_names + n || *p != nm)
             return fail(PTW_EINVAL, "source " + std::to_string(nm) + " is not a vertex of the graph");
         ids[i] = g->h_idx2int[p - g->h_names];
+    }
+    if (only && ids.size() == 1) {
+        *only = ids[0];
+        return PTW_OK;
     }
     if (g->sc.sources_cap < cfg->n_sources) {
         cudaFree(g->sc.sources);
@@ -328,9 +334,10 @@ int stage_bytes(ptw_graph *g, size_t bytes, void **out)
     return PTW_OK;
 }
 
-WalkLaunch make_launch(const ptw_walk_cfg *cfg)
+WalkLaunch make_launch(const ptw_walk_cfg *cfg, uint32_t source0 = 0)
 {
     WalkLaunch wl;
+    wl.source0 = source0;
     wl.w_begin = cfg->first_walker;
     wl.w_end = wl.w_begin + cfg->n_walkers;
     wl.thr = stop_threshold(cfg->sp);
@@ -358,39 +365,48 @@ int finish_stats(ptw_graph *g, ptw_walk_stats *stats, uint64_t walkers, bool cou
     return PTW_OK;
 }
 
-// Runs the count walk into g->sc.counts and scatters the result by name
-// into d_by_name.  Events: ev0 before, ev1 after the kernel.
-int run_count(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_by_name)
+// Records one of the graph's events for the statistics of a call that asked
+// for them.
+cudaError_t mark(ptw_graph *g, int ev, bool timed)
 {
-    int rc = upload_sources(g, cfg);
+    return timed ? cudaEventRecord(g->ev[ev], g->stream) : cudaSuccess;
+}
+
+// Runs the count walk into g->sc.counts and scatters the result by name
+// into d_by_name.  Events (timed): ev3 first, ev0 before, ev1 after the kernel.
+int run_count(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_by_name, bool timed)
+{
+    uint32_t source0 = 0;
+    int rc = upload_sources(g, cfg, &source0);
     if (rc) return rc;
     // on extended columns the walk counts by name into d_by_name itself;
     // otherwise by internal id into the scratch, scattered by name after
-    const bool by_name = cfg->n_walkers && count_walk_by_name(g, g->tune);
-    PTW_CUDA(cudaEventRecord(g->ev[3], g->stream));
+    const bool by_name = cfg->n_walkers && count_walk_by_name(g, g->tune, cfg->n_walkers);
+    PTW_CUDA(mark(g, 3, timed));
     if (by_name) PTW_CUDA(cudaMemsetAsync(d_by_name, 0, (uint64_t)g->dg.id_bound * 4, g->stream));
     else PTW_CUDA(cudaMemsetAsync(g->sc.counts, 0, (uint64_t)g->dg.n * 4, g->stream));
-    PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
+    PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers) {
-        WalkLaunch wl = make_launch(cfg);
+        WalkLaunch wl = make_launch(cfg, source0);
         if (by_name) wl.by_name = d_by_name;
         rc = launch_walk(g, wl, g->tune);
         if (rc) return rc;
     } else {
         PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 2 * sizeof(unsigned long long), g->stream));
     }
-    PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
+    PTW_CUDA(mark(g, 1, timed));
     return by_name ? PTW_OK : launch_counts_by_name(g, d_by_name);
 }
 
-int run_endpoint(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_pairs)
+int run_endpoint(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_pairs, bool timed)
 {
-    int rc = upload_sources(g, cfg);
+    uint32_t source0 = 0;
+    int rc = upload_sources(g, cfg, &source0);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[3], g->stream));
-    PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
+    PTW_CUDA(mark(g, 3, timed));
+    PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers) {
-        WalkLaunch wl = make_launch(cfg);
+        WalkLaunch wl = make_launch(cfg, source0);
         wl.endpoint = true;
         wl.pairs = d_pairs;
         rc = launch_walk(g, wl, g->tune);
@@ -398,7 +414,7 @@ int run_endpoint(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_pairs)
     } else {
         PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 2 * sizeof(unsigned long long), g->stream));
     }
-    PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
+    PTW_CUDA(mark(g, 1, timed));
     return PTW_OK;
 }
 
@@ -814,9 +830,9 @@ try {
     if (rc) return rc;
     if (!d_counts) return fail(PTW_EINVAL, "null counts buffer");
     PTW_CUDA(cudaSetDevice(g->device));
-    rc = run_count(g, cfg, d_counts);
+    rc = run_count(g, cfg, d_counts, stats != nullptr);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     if ((rc = check_word_status(g))) return rc;
     return finish_stats(g, stats, cfg->n_walkers, true);
 } catch (...) {
@@ -832,11 +848,11 @@ try {
     if (!h_counts) return fail(PTW_EINVAL, "null counts buffer");
     PTW_CUDA(cudaSetDevice(g->device));
     if (!g->sc.by_name) PTW_CUDA(device_malloc(&g->sc.by_name, (uint64_t)g->dg.id_bound * 4));
-    rc = run_count(g, cfg, g->sc.by_name);
+    rc = run_count(g, cfg, g->sc.by_name, stats != nullptr);
     if (rc) return rc;
     PTW_CUDA(cudaMemcpyAsync(h_counts, g->sc.by_name, (uint64_t)g->dg.id_bound * 4,
                              cudaMemcpyDeviceToHost, g->stream));
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     PTW_CUDA(cudaStreamSynchronize(g->stream));
     if ((rc = check_word_status(g))) return rc;
     return finish_stats(g, stats, cfg->n_walkers, true);
@@ -870,7 +886,7 @@ try {
         PTW_CUDA(cudaStreamWaitEvent(g->stream, a->ev_copy, 0));
     }
     PTW_CUDA(cudaEventRecord(a->ev_start, g->stream));
-    rc = run_count(g, cfg, a->by_name);
+    rc = run_count(g, cfg, a->by_name, false);
     if (rc) return rc;
     PTW_CUDA(cudaMemcpyAsync(a->h_moves, g->sc.ctrl + 1, sizeof(unsigned long long), cudaMemcpyDeviceToHost,
                              g->stream));
@@ -923,9 +939,9 @@ try {
     if (!d_pairs && cfg->n_walkers) return fail(PTW_EINVAL, "null pairs buffer");
     if ((uintptr_t)d_pairs % 8) return fail(PTW_EINVAL, "pairs buffer must be 8-byte aligned");
     PTW_CUDA(cudaSetDevice(g->device));
-    rc = run_endpoint(g, cfg, d_pairs);
+    rc = run_endpoint(g, cfg, d_pairs, stats != nullptr);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     if ((rc = check_word_status(g))) return rc;
     return finish_stats(g, stats, cfg->n_walkers, false);
 } catch (...) {
@@ -942,11 +958,11 @@ try {
     void *stage = nullptr;
     rc = stage_bytes(g, cfg->n_walkers * 8, &stage);
     if (rc) return rc;
-    rc = run_endpoint(g, cfg, (uint32_t *)stage);
+    rc = run_endpoint(g, cfg, (uint32_t *)stage, stats != nullptr);
     if (rc) return rc;
     if (cfg->n_walkers)
         PTW_CUDA(cudaMemcpyAsync(h_pairs, stage, cfg->n_walkers * 8, cudaMemcpyDeviceToHost, g->stream));
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     PTW_CUDA(cudaStreamSynchronize(g->stream));
     if ((rc = check_word_status(g))) return rc;
     return finish_stats(g, stats, cfg->n_walkers, false);
@@ -1110,7 +1126,7 @@ try {
     if (!g->sc.by_name) PTW_CUDA(device_malloc(&g->sc.by_name, std::max<uint64_t>((uint64_t)g->dg.id_bound * 4, 4)));
     auto time_walk = [&](const ptw_tune &t, int reps, float *med) -> int {
         std::vector<float> ms(reps);
-        const bool by_name = count_walk_by_name(g, t);
+        const bool by_name = count_walk_by_name(g, t, cfg.n_walkers);
         WalkLaunch twl = wl;
         if (by_name) twl.by_name = g->sc.by_name;
         for (int rep = -1; rep < reps; ++rep) {

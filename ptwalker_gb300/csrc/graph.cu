@@ -146,6 +146,18 @@ __global__ void k_adj(const uint32_t *int_deg, const uint32_t *int_off, uint32_t
         adj[i] = make_uint2(int_off[i], int_deg[i]);
 }
 
+// Appends {id, first column, degree} of every vertex that starts a run of
+// equal degree (unordered; run[0].x counts them, also beyond max_runs).
+__global__ void k_row_runs(const uint2 *adj, uint32_t n, uint32_t max_runs, uint4 *run)
+{
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 r = adj[i];
+        if (i != 0 && adj[i - 1].y == r.y) continue;
+        const uint32_t p = atomicAdd(&run[0].x, 1u);
+        if (p < max_runs) run[1 + p] = make_uint4(i, r.x, r.y, 0u);
+    }
+}
+
 // Scatter canonical edges into internal rows.  Edge e belongs to canonical
 // row si[e]; its rank inside the row is e - row_ptr[si[e]].
 __global__ void k_fill_col(const uint32_t *si, const uint32_t *di, const uint32_t *row_ptr,
@@ -326,15 +338,7 @@ int graph_init_handle(ptw_graph *g)
     PTW_CUDA(cudaStreamCreateWithFlags(&g->own_stream, cudaStreamNonBlocking));
     g->stream = g->own_stream;
     for (auto &e : g->ev) PTW_CUDA(cudaEventCreate(&e));
-    g->tune.block = 256;
-    g->tune.ilp = 2;
-    g->tune.chunk = 256;
-    g->tune.hot_k = 0;
-    g->tune.blocks_per_sm = 0;
-    g->tune.min_blocks = 0;
-    g->tune.paths_ilp = 2;
-    g->tune.cache_hints = 1;
-    g->tune.paths_named = 1;
+    g->tune = default_tune();
     return PTW_OK;
 }
 
@@ -351,6 +355,7 @@ void graph_release(ptw_graph *g)
     cudaFree(g->dg.col_named);
     cudaFree(g->dg.col_ext);
     cudaFree(g->dg.vtx_ext);
+    cudaFree(g->dg.rows);
     cudaFree(g->dg.edge_filter);
     cudaFree(g->sc.counts);
     cudaFree(g->sc.ctrl);
@@ -447,6 +452,43 @@ int csr_to_device_edges(const uint64_t *h_row_ptr, const uint32_t *h_col, const 
     *d_dst = dst;
     return PTW_OK;
 }
+
+namespace {
+
+// Builds the row table from the runs of equal degree (k_row_runs); none when
+// there are more than kMaxRowRuns of them.
+int build_row_table(ptw_graph *g, const std::vector<uint4> &found)
+{
+    const uint32_t runs = found[0].x, n = g->dg.n;
+    if (runs > kMaxRowRuns) return PTW_OK;
+    std::vector<uint4> run(found.begin() + 1, found.begin() + 1 + runs);
+    std::sort(run.begin(), run.end(), [](const uint4 &x, const uint4 &y) { return x.x < y.x; });
+    std::vector<uint32_t> img(row_words(runs, n), 0u);
+    for (uint32_t k = 0; k < runs; ++k) {
+        img[k] = run[k].x;
+        img[row_pairs_at(runs) + 2 * k] = run[k].y - run[k].x * run[k].z;
+        img[row_pairs_at(runs) + 2 * k + 1] = run[k].z;
+    }
+    img[runs] = img[runs + 1] = ~0u;
+    img[row_pairs_at(runs) + 2 * runs] = img[row_pairs_at(runs) + 2 * runs - 2];
+    img[row_pairs_at(runs) + 2 * runs + 1] = img[row_pairs_at(runs) + 2 * runs - 1];
+    uint16_t *bucket = reinterpret_cast<uint16_t *>(img.data() + row_buckets_at(runs));
+    uint32_t next = 0;  // first bucket whose run is not set yet
+    for (uint32_t k = 0; k < runs; ++k) {
+        // run k holds the ids [run[k].x, end); it is the run of every bucket whose first id is among them
+        const uint32_t end = k + 1 < runs ? run[k + 1].x : n;
+        const uint32_t last = row_bucket(end - 1);
+        for (; next <= last; ++next) bucket[next] = (uint16_t)k;
+    }
+    PTW_CUDA(device_malloc(&g->dg.rows, img.size() * 4));
+    PTW_CUDA(cudaMemcpyAsync(g->dg.rows, img.data(), img.size() * 4, cudaMemcpyHostToDevice, g->stream));
+    PTW_CUDA(cudaStreamSynchronize(g->stream));  // img is read until then
+    g->dg.row_runs = runs;
+    g->device_bytes += img.size() * 4;
+    return PTW_OK;
+}
+
+}  // namespace
 
 int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m,
                                   bool as_undirected, bool clean, bool compact_names)
@@ -598,15 +640,22 @@ int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst
 
     // Scratch reused by every walk.
     PTW_CUDA(device_malloc(&g->sc.counts, (uint64_t)n * 4));
-    PTW_CUDA(device_malloc(&g->sc.ctrl, 8 * sizeof(unsigned long long)));
-    PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 8 * sizeof(unsigned long long), st));  // [7]: index checks
+    PTW_CUDA(device_malloc(&g->sc.ctrl, 16 * sizeof(unsigned long long)));
+    PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 16 * sizeof(unsigned long long), st));  // [7]: index checks
+    uint4 *d_run = nullptr;
+    std::vector<uint4> h_run(1 + kMaxRowRuns);
+    PTW_CUDA(tmp.alloc(&d_run, h_run.size()));
+    PTW_CUDA(cudaMemsetAsync(d_run, 0, sizeof(uint4), st));
+    k_row_runs<<<grid_for(n), kThreads, 0, st>>>(dg.adj, n, kMaxRowRuns, d_run);
+    PTW_CUDA(cudaGetLastError());
+    PTW_CUDA(cudaMemcpyAsync(h_run.data(), d_run, h_run.size() * sizeof(uint4), cudaMemcpyDeviceToHost, st));
     PTW_CUDA(cudaStreamSynchronize(st));
     dg.max_degree = h_maxdeg;
     // symmetrised, self-loops dropped and duplicates removed: simple and
     // symmetric by construction (node2vec then skips its check)
     dg.simple_symmetric = as_undirected && clean ? 1 : -1;
     g->device_bytes = (uint64_t)n * (8 + 4 * 4 + 4) + mm * 4 + 64;
-    return PTW_OK;
+    return build_row_table(g, h_run);
 }
 
 }  // namespace ptw

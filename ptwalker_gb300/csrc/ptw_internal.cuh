@@ -16,6 +16,8 @@
 #include "../../include/ptw.h"
 #include <nvtx3/nvToolsExt.h>
 
+#include "row_table.cuh"
+
 // Philox counter words that separate the purposes of a draw.
 #define PTW_TAG_WALK 0x57414C4Bu  // "WALK": one draw per move
 #define PTW_TAG_START 0x53545254u // "STRT": start-vertex draw
@@ -254,6 +256,8 @@ struct DeviceGraph {
     uint4 *col_ext = nullptr;     // [m] {neighbour id, its first column, its degree, its name};
                                   // built on the first walk with tune.ext_columns
     uint4 *vtx_ext = nullptr;     // [n] {id, first column, degree, name} by canonical index, built with col_ext
+    uint32_t *rows = nullptr;     // row table (row_table.cuh); null when the graph has too many distinct degrees
+    uint32_t row_runs = 0;        // runs of equal degree in it
     uint32_t *edge_filter = nullptr; // blocked Bloom filter of the directed edges (u, v): blocks of
                                      // 8 words; built on the first node2vec walk
     uint64_t filter_blocks = 0;      // a power of two
@@ -264,7 +268,7 @@ struct DeviceGraph {
 // Scratch owned by a graph handle and reused by every call.
 struct Scratch {
     uint32_t *counts = nullptr;           // [n] visit counts by internal id
-    unsigned long long *ctrl = nullptr;   // [8]: walker cursor, moves, error flags
+    unsigned long long *ctrl = nullptr;   // [16]: walker cursor, moves, error flags
     uint32_t *sources = nullptr;          // source internal ids
     uint32_t sources_cap = 0;
     uint32_t *by_name = nullptr;          // [id_bound] staging for host-output calls
@@ -330,15 +334,22 @@ struct WalkLaunch {
     uint64_t seed = 0;
     int start_mode = 0;
     uint32_t n_sources = 0;
+    uint32_t source0 = 0;      // the only source's internal id (n_sources == 1: no list on the device)
     uint32_t max_moves = 0;
     bool endpoint = false;     // RWR endpoint app instead of counting
     uint32_t *pairs = nullptr; // endpoint output by walker (names)
     uint32_t *by_name = nullptr; // count walks: count straight into this by-name array (extended
                                  // columns; see count_walk_by_name), else into the graph's scratch
 };
-// True when the count walk under tune t reads the extended columns (built
-// here if needed) and can count by name directly.
-bool count_walk_by_name(ptw_graph *g, const ptw_tune &t);
+// The launch parameters a graph is built with.
+ptw_tune default_tune();
+// True when the fields of t that count and endpoint walks read are the ones
+// a graph is built with: the library then picks kernel and launch itself.
+bool walk_launch_is_auto(const ptw_tune &t);
+// True when a count walk of n_walk walkers under tune t counts straight into
+// the caller's by-name array: on the extended columns (built here if needed),
+// or in a launch of the library's own choice that is short on walkers.
+bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk);
 int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t);
 int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
                  int start_mode, uint32_t n_sources, int32_t *paths);

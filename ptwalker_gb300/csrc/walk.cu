@@ -21,6 +21,9 @@
 // gather: the walker keeps {off, deg} of its vertex in registers and loads a
 // row record only at its start vertex.
 //
+// A graph that still has the launch parameters it was built with walks in
+// k_walk_queued (walk_queued.cuh) instead.
+//
 // K3 k_paths: DeepWalk (src/core/deepwalk.cpp:25-28) on the plain or
 // name-paired columns.  One walker per lane, all walks the same length, so a
 // warp stays converged.  Each warp stages the next 32 path positions of its
@@ -45,11 +48,13 @@ struct WalkArgs {
     const uint4 *__restrict__ vtx_ext;       // {id, first column, degree, name} by canonical index
     const uint32_t *__restrict__ start_map;  // canonical index -> internal
     const uint32_t *__restrict__ int2idx;    // internal -> canonical index
-    const uint32_t *__restrict__ sources;    // internal ids
+    const uint32_t *__restrict__ sources;    // internal ids (more than one source)
     const uint32_t *__restrict__ int2name;
+    const uint32_t *__restrict__ rows;       // k_walk_queued: row table (row_table.cuh)
     uint32_t *__restrict__ counts;
     uint32_t *__restrict__ pairs;            // endpoint app: [2 * walkers] names
-    unsigned long long *__restrict__ ctrl;   // [0] cursor, [1] moves
+    unsigned long long *__restrict__ ctrl;   // [0] cursor, [1] moves; k_walk_queued: [8] cursor, [9] moves so far,
+                                             // [10] blocks that ended
     uint64_t w_begin;
     uint64_t n_walk;
     uint64_t thr;
@@ -57,9 +62,11 @@ struct WalkArgs {
     uint32_t n;
     uint32_t key0, key1;
     uint32_t n_sources;
+    uint32_t source0;  // the only source
     uint32_t max_moves;
     uint32_t chunk;
     uint32_t hot_k;
+    uint32_t row_runs, row_words;
     int start_mode;
     int hints;  // L2 eviction priorities on (see l2_policy)
     int by_name;  // EXT count walks: counts[] is indexed by vertex name (the caller's output)
@@ -67,11 +74,13 @@ struct WalkArgs {
 
 __device__ __forceinline__ uint32_t start_vertex(const WalkArgs &a, uint64_t wid)
 {
+    if (a.start_mode == PTW_START_SOURCES && a.n_sources == 1) return a.source0;
     return walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
 }
 
 __device__ __forceinline__ uint32_t start_index(const WalkArgs &a, uint64_t wid)
 {
+    if (a.start_mode == PTW_START_SOURCES && a.n_sources == 1) return a.int2idx[a.source0];
     return walker_start_index(a.start_mode, a.int2idx, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
 }
 
@@ -676,14 +685,43 @@ void *pick_walk(bool endpoint, int ilp, bool hot, int min_blocks, int block, boo
 }
 
 }  // namespace
+}  // namespace ptw
 
-// Builds the extended column copy on first use; false (and no error) when
-// it does not fit in device memory, so the caller walks without it.
-bool count_walk_by_name(ptw_graph *g, const ptw_tune &t)
+#include "walk_queued.cuh"
+
+namespace ptw {
+
+// Walkers of one wave of k_walk_queued.
+static uint64_t queued_lanes(const ptw_graph *g) { return (uint64_t)g->num_sms * kQueuedBlock; }
+
+ptw_tune default_tune()
 {
+    ptw_tune t{};
+    t.block = 256;
+    t.ilp = 2;
+    t.chunk = 256;
+    t.paths_ilp = 2;
+    t.cache_hints = 1;
+    t.paths_named = 1;
+    return t;
+}
+
+bool walk_launch_is_auto(const ptw_tune &t)
+{
+    const ptw_tune d = default_tune();
+    return t.block == d.block && t.ilp == d.ilp && t.chunk == d.chunk && t.hot_k == d.hot_k &&
+           t.blocks_per_sm == d.blocks_per_sm && t.min_blocks == d.min_blocks && t.cache_hints == d.cache_hints &&
+           !(t.ext_columns & 1) && t.gather_slots == d.gather_slots && t.warp_agg == d.warp_agg;
+}
+
+bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
+{
+    if (walk_launch_is_auto(t)) return n_walk <= queued_lanes(g);
     return !t.gather_slots && !t.warp_agg && (t.ext_columns & 1) && ensure_ext_columns(g);
 }
 
+// Builds the extended column copy on first use; false (and no error) when
+// it does not fit in device memory, so the caller walks without it.
 bool ensure_ext_columns(ptw_graph *g)
 {
     if (g->dg.col_ext) return true;
@@ -764,12 +802,12 @@ int check_tune(const ptw_tune &t)
     return PTW_OK;
 }
 
-int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
+namespace {
+
+WalkArgs walk_args(ptw_graph *g, const WalkLaunch &wl)
 {
-    int rc = check_tune(t);
-    if (rc) return rc;
     const DeviceGraph &dg = g->dg;
-    WalkArgs a;
+    WalkArgs a{};
     a.adj = dg.adj;
     a.col = dg.col;
     a.start_map = dg.idx2int;
@@ -787,11 +825,57 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     a.key0 = (uint32_t)wl.seed;
     a.key1 = (uint32_t)(wl.seed >> 32);
     a.n_sources = wl.n_sources;
+    a.source0 = wl.source0;
     a.max_moves = wl.max_moves;
+    a.start_mode = wl.start_mode;
+    return a;
+}
+
+// The launch of a graph with the launch parameters it was built with.  Up to
+// one walker per lane of 1,024 threads on every SM: as few threads per SM as
+// that takes, so that all SMs share the walkers.
+int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
+{
+    WalkArgs a = walk_args(g, wl);
+    a.chunk = 32;
+    if (wl.by_name) a.counts = wl.by_name;
+    const bool one_wave = a.n_walk <= queued_lanes(g);
+    const uint64_t per_sm = (a.n_walk + g->num_sms - 1) / g->num_sms;
+    const int block = (int)std::min<uint64_t>(kQueuedBlock, (per_sm + 31) / 32 * 32);
+    const uint64_t grid = std::min<uint64_t>(g->num_sms, (a.n_walk + block - 1) / block);
+    const bool group = wl.start_mode == PTW_START_SOURCES && !wl.endpoint;
+    // Hot counters pay once their flush (hot_k words per block) is small
+    // beside the visits: scale 14 (12,557 walkers) is quicker without any,
+    // scale 16 (45,000) with 1,024, from one wave on 8,192 and 4,096 are alike.
+    if (!wl.endpoint)
+        a.hot_k = std::min<uint32_t>(!one_wave ? 8192u : a.n_walk >= 24576 ? 1024u : 0u, g->dg.n);
+    const bool rows = !one_wave && g->dg.rows;
+    if (rows) {
+        a.rows = g->dg.rows;
+        a.row_runs = g->dg.row_runs;
+        a.row_words = row_words(g->dg.row_runs, g->dg.n);
+    }
+    void *fn = pick_walk_queued(wl.endpoint, a.hot_k > 0, one_wave, group, rows);
+    const size_t smem = ((size_t)a.hot_k + a.row_words) * 4;
+    if (smem > 48 * 1024)
+        PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    void *args[] = {&a};
+    PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::max<uint64_t>(grid, 1)), dim3(block), args, smem, g->stream));
+    return PTW_OK;
+}
+
+}  // namespace
+
+int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
+{
+    int rc = check_tune(t);
+    if (rc) return rc;
+    if (walk_launch_is_auto(t)) return launch_walk_queued(g, wl);
+    const DeviceGraph &dg = g->dg;
+    WalkArgs a = walk_args(g, wl);
     a.chunk = (uint32_t)t.chunk;
     const bool hot = !wl.endpoint && t.hot_k > 0;
     a.hot_k = hot ? std::min<uint32_t>((uint32_t)t.hot_k, dg.n) : 0;
-    a.start_mode = wl.start_mode;
     a.hints = t.cache_hints;
 
     const bool slots = t.gather_slots != 0 && ensure_ext_columns(g);
