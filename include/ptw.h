@@ -315,7 +315,8 @@ typedef struct ptw_batch_tune {
     uint32_t dense_ratio;   /* a query counts into a dense array of n counters when that takes
                                at most this many times its hash table's bytes; 0 = 1 */
     int32_t ext_columns;    /* 1 = walk the extended column copy, 2 = the plain columns,
-                               0 = as bit 0 of the graph's walk tune */
+                               0 = the plain columns, or, on a graph with more than 8192
+                               distinct degrees, as bit 0 of the graph's walk tune */
 } ptw_batch_tune;
 int ptw_graph_set_batch_tune(ptw_graph *g, const ptw_batch_tune *t);
 int ptw_graph_get_batch_tune(const ptw_graph *g, ptw_batch_tune *t);

@@ -130,7 +130,7 @@ constexpr uint64_t kMaxBudget = 1ull << 28;
 // Effective batch launch parameters (zero fields of ptw_batch_tune take the
 // defaults).
 struct BatchTune {
-    uint32_t desc_walkers, blocks_per_sm, dense_ratio;
+    uint32_t desc_walkers, blocks_per_sm, dense_ratio;  // desc_walkers 0: by the number of walkers
     uint64_t group_bytes;
     bool ext;
 };
@@ -139,11 +139,13 @@ BatchTune effective_tune(const ptw_graph *g)
 {
     const ptw_batch_tune &t = g->btune;
     BatchTune e;
-    e.desc_walkers = t.desc_walkers ? t.desc_walkers : kDescWalkers;
+    e.desc_walkers = t.desc_walkers;
     e.blocks_per_sm = t.blocks_per_sm;
     e.dense_ratio = t.dense_ratio ? t.dense_ratio : 1u;
     e.group_bytes = t.group_bytes == 0 ? kGroupBytes : t.group_bytes == ~0ull ? 0ull : t.group_bytes;
-    e.ext = t.ext_columns == 1 ? true : t.ext_columns == 2 ? false : (g->tune.ext_columns & 1) != 0;
+    // by itself, the graph's walk tune decides only where there is no row table
+    // (which is quicker than the extended columns on every graph measured)
+    e.ext = t.ext_columns == 1 ? true : t.ext_columns == 2 || g->dg.rows ? false : (g->tune.ext_columns & 1) != 0;
     return e;
 }
 
@@ -384,10 +386,10 @@ uint64_t interleave_descriptors(const std::vector<uint64_t> &j0, const std::vect
 
 void interleave_descriptors(const std::vector<uint64_t> &j0, const std::vector<uint64_t> &count,
                             const std::vector<uint64_t> &table_bytes, uint64_t group_bytes,
-                            std::vector<uint3> &desc)
+                            std::vector<uint3> &desc, uint32_t desc_walkers)
 {
     std::unique_ptr<uint3[]> buf;
-    const uint64_t n = interleave_descriptors(j0, count, table_bytes, group_bytes, buf, 1, kDescWalkers);
+    const uint64_t n = interleave_descriptors(j0, count, table_bytes, group_bytes, buf, 1, desc_walkers);
     desc.assign(buf.get(), buf.get() + n);
 }
 
@@ -423,9 +425,11 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     std::unique_ptr<uint3[]> h_desc;
     std::vector<uint64_t> tbytes(nq);
     for (uint32_t i = 0; i < nq; ++i) tbytes[i] = wq[i].cap * 8;
+    uint64_t walkers = 0;
+    for (uint64_t c : cnt) walkers += c;
     const uint64_t nd = interleave_descriptors(j0, cnt, tbytes, bt.group_bytes, h_desc,
                                                std::min(16u, std::max(1u, std::thread::hardware_concurrency())),
-                                               bt.desc_walkers);
+                                               bt.desc_walkers ? bt.desc_walkers : desc_walkers_for(g, walkers));
     t_plan = clk();
     ph->plan_ms += 1e3 * (t_plan - t_enter);
     const uint64_t n_slots = h_tab[nq];
@@ -456,11 +460,10 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
         t_setup = clk();
     }
 
-    BatchArgs a;
+    BatchArgs a{};
     a.adj = g->dg.adj;
     a.col = g->dg.col;
     const bool ext = bt.ext && ensure_ext_columns(g);
-    a.col_ext = g->dg.col_ext;
     a.int2idx = g->dg.int2idx;
     a.ext_idx = g->dg.id_bound == g->dg.n ? 1u : 0u;  // names 0..n-1
     a.desc = d_desc;
@@ -483,13 +486,10 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     a.max_moves = cfg->max_moves;
     a.app = cfg->app;
     if (nd >= (1ull << 32)) return fail(PTW_EINVAL, "wave too large");
-    int per_sm = 0;
-    const void *kfn = ext ? (const void *)k_batch<true> : (const void *)k_batch<false>;
-    PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kfn, 256, 0));
-    per_sm = std::max(per_sm, 1);
-    if (bt.blocks_per_sm) per_sm = std::min<int>(per_sm, (int)bt.blocks_per_sm);
-    uint64_t grid = (uint64_t)g->num_sms * per_sm;
-    grid = std::min<uint64_t>(grid, std::max<uint64_t>(1, (nd + 7) / 8));
+    BatchLaunch bl;
+    if (const int rc0 = batch_launch(g, ext, a, bl)) return rc0;
+    if (bt.blocks_per_sm) bl.per_sm = std::min<int>(bl.per_sm, (int)bt.blocks_per_sm);
+    const unsigned grid = batch_grid(g, bl, nd);
     // Full lists: host buffers of an estimated size are faulted in on host
     // threads while the walk runs (about 1.1 distinct entries per walker on
     // R-MAT at sp 0.2; 1.5 leaves room); compaction adopts them if the lists
@@ -530,7 +530,7 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     const int sp_walk = ph->begin(PhaseTimer::kWalk, st);
     {
         void *kargs[] = {&a};
-        PTW_CUDA(cudaLaunchKernel(kfn, dim3((unsigned)grid), dim3(256), kargs, 0, st));
+        PTW_CUDA(cudaLaunchKernel(bl.fn, dim3(grid), dim3(bl.block), kargs, bl.smem, st));
     }
     ph->end(sp_walk, st);
     PTW_CUDA(cudaEventRecord(g->ev[1], st));

@@ -56,9 +56,9 @@ __device__ __forceinline__ void tab_add(unsigned long long *slots, uint32_t mask
 // kDenseMask) one fire-and-forget reduction at v's canonical index idx,
 // else a hash-table insert of v.
 __device__ __forceinline__ void count_add(unsigned long long *tab, uint32_t mask, uint32_t v, uint32_t idx,
-                                          uint32_t inc, uint32_t *flag, uint32_t n, unsigned long long *check)
+                                          uint32_t inc, uint32_t *flag, uint32_t n, unsigned long long *check, uint64_t pol)
 {
-    if (mask == kDenseMask) atomicAdd(reinterpret_cast<uint32_t *>(tab) + PTW_IDX(idx, n, check, kCheckTable), inc);
+    if (mask == kDenseMask) red_add_hint(reinterpret_cast<uint32_t *>(tab) + PTW_IDX(idx, n, check, kCheckTable), inc, pol);
     else tab_add(tab, mask, v, inc, flag);
     (void)n;
     (void)check;
@@ -75,6 +75,8 @@ __device__ __forceinline__ void count_add(unsigned long long *tab, uint32_t mask
 struct BatchArgs {
     const uint2 *__restrict__ adj;
     const uint32_t *__restrict__ col;
+    const uint32_t *__restrict__ rows;     // row table (row_table.cuh)
+    uint32_t row_runs, row_words;
     const uint4 *__restrict__ col_ext;     // EXT: {id, first column, degree, name} per entry
     const uint32_t *__restrict__ int2idx;  // internal id -> canonical index (dense tables)
     uint32_t ext_idx;  // 1: names are 0..n-1, so an extended column's name is the canonical index
@@ -96,38 +98,74 @@ struct BatchArgs {
     int app;
 };
 
-// Walker ranks per descriptor (host side splits queries into chunks of it).
+// Walker ranks per descriptor at most (host side splits queries into chunks of it).
 constexpr uint32_t kDescWalkers = 256;
-
-constexpr int kBatchIlp = 2;
+// A move that leaves a vertex of at most this degree may meet other walkers of
+// its query at its end.
+constexpr uint32_t kCrowdDegree = 32;
 
 // Counts one visit of key v (canonical index idx, used by dense tables) in
-// query entry q's table, aggregated over the lanes of the warp that visit
-// the same (query, vertex) now.
-__device__ __forceinline__ void visit_agg(unsigned mask_active, bool on, uint32_t q, uint32_t v, uint32_t idx,
-                                          unsigned long long *tab, uint32_t tmask, uint32_t *flag, uint32_t lane,
-                                          const BatchArgs &a)
+// query entry q's table for every lane with `on` (the whole warp calls it).
+// Visits of one vertex among the lanes with `crowd` are merged into one update:
+// a query's walkers meet on the first moves and around vertices of low degree,
+// and without merging there the counters of those few vertices are the bound
+// (R-MAT scale 22, 512 uniform sources: 8.7 against 14.6 ms).  Elsewhere two
+// lanes hardly ever visit one vertex, and __match_any_sync costs an SM 2 cycles
+// per distinct 32-bit key (4 per 64-bit key), so that matching every move of a
+// warp was 60% of the kernel's time on a graph in L2 (scale 16: 3.5 ms with all
+// lanes matched on 64 bits, 2.4 on 32, 1.9 with the crowded ones only).
+__device__ __forceinline__ void visit_merged(bool on, bool crowd, uint32_t q, uint32_t v, uint32_t idx,
+                                             unsigned long long *tab, uint32_t tmask, uint32_t *flag, uint32_t lane,
+                                             const BatchArgs &a, uint64_t pol)
 {
-    const unsigned m = __ballot_sync(mask_active, on);
-    if (!on) return;
-    const unsigned long long key = ((unsigned long long)q << 32) | v;
-    const unsigned grp = __match_any_sync(m, key);
-    if ((grp & ((1u << lane) - 1u)) == 0) count_add(tab, tmask, v, idx, __popc(grp), flag, a.n, a.check);
+    unsigned left = __ballot_sync(kBFull, on && crowd);
+    uint32_t inc = on ? 1u : 0u;
+    while (left) {
+        const uint32_t q1 = __shfl_sync(kBFull, q, __ffs(left) - 1);
+        const bool mine = (left >> lane & 1u) && q == q1;
+        const unsigned m = __ballot_sync(kBFull, mine);
+        if (mine) {
+            const unsigned grp = __match_any_sync(m, v);
+            inc = (grp & ((1u << lane) - 1u)) == 0 ? __popc(grp) : 0u;
+        }
+        left &= ~m;
+    }
+    if (inc) count_add(tab, tmask, v, idx, inc, flag, a.n, a.check, pol);
+}
+
+// The count table of query entry e.
+__device__ __forceinline__ void query_table(const BatchArgs &a, uint32_t e, unsigned long long *&tab, uint32_t &mask)
+{
+    tab = a.slots + a.q_tab[e];
+    mask = a.q_mask[e];
+#ifdef PTW_CHECKED
+    const uint64_t tslots = mask == kDenseMask ? ((uint64_t)a.n + 1) / 2 : (uint64_t)mask + 1;
+    if (a.q_tab[e] + tslots > a.n_slots) {  // table outside the slots: count into slot 0
+        atomicOr(a.check, 1ull << kCheckTable);
+        tab = a.slots;
+        mask = 0;
+    }
+#endif
 }
 
 // EXT: moves read the extended column copy and keep the row record of the
-// current vertex in registers (one gather per move instead of two).
-template <bool EXT>
-__global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
+// current vertex in registers; ROWS: they look the row up in the row table in
+// shared memory (one gather per move either way, of 16 or of 4 bytes).
+// ILP: walkers per lane.
+template <bool EXT, bool ROWS, int ILP>
+__device__ __forceinline__ void batch_body(const BatchArgs &a, const uint32_t *s_rows)
 {
+    // the tables of the running queries stay in L2, the columns stream through
+    // it (both at normal priority: 12% slower at R-MAT scales 20 and 22)
+    const uint64_t pol_tab = l2_policy(1), pol_col = l2_policy(2);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
-    uint32_t q[kBatchIlp], v[kBatchIlp], step[kBatchIlp], j[kBatchIlp], qid[kBatchIlp], mask[kBatchIlp];
-    unsigned long long *tab[kBatchIlp];
-    bool act[kBatchIlp], have[kBatchIlp];
-    uint2 rec[kBatchIlp];
+    uint32_t q[ILP], v[ILP], step[ILP], j[ILP], qid[ILP], mask[ILP];
+    unsigned long long *tab[ILP];
+    bool act[ILP], have[ILP];
+    uint2 rec[ILP];
 #pragma unroll
-    for (int k = 0; k < kBatchIlp; ++k) {
+    for (int k = 0; k < ILP; ++k) {
         act[k] = have[k] = false;
         q[k] = v[k] = step[k] = j[k] = qid[k] = mask[k] = 0;
         tab[k] = nullptr;
@@ -139,7 +177,7 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
     unsigned long long moves = 0;
     for (;;) {
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k) {
+        for (int k = 0; k < ILP; ++k) {
             const unsigned need = __ballot_sync(kBFull, !act[k]);
             bool got = false;
             if (need != 0 && !exhausted) {
@@ -170,51 +208,48 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
                     dq = ds.x;
                     dnext = ds.y;
                     dend = ds.y + ds.z;
+                    if (a.app == PTW_APP_VISITS && lane == 0 && dend != dnext) {
+                        // the start visits of all walkers of the descriptor, at once
+                        const uint32_t e = (uint32_t)PTW_IDX(dq, a.nq, a.check, kCheckQuery);
+                        const uint32_t src = a.q_src[e];
+                        unsigned long long *t = nullptr;
+                        uint32_t tm = 0;
+                        query_table(a, e, t, tm);
+                        const uint32_t si =
+                            tm == kDenseMask ? __ldg(&a.int2idx[PTW_IDX(src, a.n, a.check, kCheckCounter)]) : 0u;
+                        count_add(t, tm, src, si, ds.z, &a.q_flag[e], a.n, a.check, pol_tab);
+                    }
                 }
             }
             if (got) {
                 q[k] = (uint32_t)PTW_IDX(q[k], a.nq, a.check, kCheckQuery);
                 qid[k] = a.q_qid[q[k]];
                 v[k] = a.q_src[q[k]];
-                tab[k] = a.slots + a.q_tab[q[k]];
-                mask[k] = a.q_mask[q[k]];
-#ifdef PTW_CHECKED
-                {
-                    const uint64_t tslots = mask[k] == kDenseMask ? ((uint64_t)a.n + 1) / 2 : (uint64_t)mask[k] + 1;
-                    if (a.q_tab[q[k]] + tslots > a.n_slots) {  // table outside the slots: count into slot 0
-                        atomicOr(a.check, 1ull << kCheckTable);
-                        tab[k] = a.slots;
-                        mask[k] = 0;
-                    }
-                }
-#endif
+                query_table(a, q[k], tab[k], mask[k]);
                 step[k] = 0;
                 act[k] = true;
                 have[k] = false;
             }
-            if (a.app == PTW_APP_VISITS) {
-                // Start visits: one table update per (warp, query) group.
-                const uint32_t sidx =
-                    got && mask[k] == kDenseMask ? __ldg(&a.int2idx[PTW_IDX(v[k], a.n, a.check, kCheckCounter)]) : 0u;
-                visit_agg(kBFull, got, q[k], v[k], sidx, tab[k], mask[k], &a.q_flag[q[k]], lane, a);
-            }
         }
         bool any = false;
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k) any |= act[k];
+        for (int k = 0; k < ILP; ++k) any |= act[k];
         if (!__any_sync(kBFull, any)) break;
 
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k)
-            if (act[k] && !(EXT && have[k])) rec[k] = __ldg(&a.adj[PTW_IDX(v[k], a.n, a.check, kCheckRecord)]);
-        uint4 r[kBatchIlp];
+        for (int k = 0; k < ILP; ++k)
+            if (act[k] && !(EXT && have[k])) {
+                const uint32_t x = (uint32_t)PTW_IDX(v[k], a.n, a.check, kCheckRecord);
+                rec[k] = ROWS ? row_of(s_rows, a.row_runs, x) : __ldg(&a.adj[x]);
+            }
+        uint4 r[ILP];
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k)
+        for (int k = 0; k < ILP; ++k)
             if (act[k]) r[k] = philox(make_uint4(j[k], qid[k], step[k], PTW_TAG_WALK), a.key0, a.key1);
-        uint32_t nb[kBatchIlp], nidx[kBatchIlp];
-        uint2 nrec[kBatchIlp];
+        uint32_t nb[ILP], nidx[ILP];
+        uint2 nrec[ILP];
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k) {
+        for (int k = 0; k < ILP; ++k) {
             nidx[k] = 0;
             if (act[k] && rec[k].y != 0) {
                 const uint32_t e = rec[k].x + __umulhi(r[k].x, rec[k].y);
@@ -224,21 +259,24 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
                     nrec[k] = make_uint2(x.y, x.z);
                     nidx[k] = x.w;  // the neighbour's name: its canonical index when a.ext_idx
                 } else {
-                    nb[k] = __ldg(&a.col[PTW_IDX(e, a.m, a.check, kCheckColumn)]);
+                    nb[k] = ld_line_u32(&a.col[PTW_IDX(e, a.m, a.check, kCheckColumn)], pol_col);
                 }
             }
         }
         // Canonical indices of the new vertices for dense tables, every
         // slot's load issued before any table update waits on one (with
-        // a.ext_idx the gathered column entry already holds it).
+        // a.ext_idx the gathered column entry already holds it).  Through L1:
+        // the hubs' indices are asked for by all SMs, and reading them from L2
+        // each time held R-MAT scale 16 at 43 G moves/s (109 with L1).
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k)
+        for (int k = 0; k < ILP; ++k)
             if (act[k] && rec[k].y != 0 && mask[k] == kDenseMask && !(EXT && a.ext_idx))
                 nidx[k] = __ldg(&a.int2idx[PTW_IDX(nb[k], a.n, a.check, kCheckCounter)]);
 #pragma unroll
-        for (int k = 0; k < kBatchIlp; ++k) {
+        for (int k = 0; k < ILP; ++k) {
             // every lane runs the aggregation calls (warp-collective)
             const bool moved = act[k] && rec[k].y != 0;
+            const uint32_t left_deg = rec[k].y;  // of the vertex that the move left
             if (moved) {
                 v[k] = nb[k];
                 if (EXT) {
@@ -249,7 +287,7 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
                 ++moves;
             }
             if (a.app == PTW_APP_VISITS)
-                visit_agg(kBFull, moved, q[k], v[k], nidx[k], tab[k], mask[k], &a.q_flag[q[k]], lane, a);
+                visit_merged(moved, step[k] == 1 || left_deg <= kCrowdDegree, q[k], v[k], nidx[k], tab[k], mask[k], &a.q_flag[q[k]], lane, a, pol_tab);
             const bool done = act[k] && (!moved || (uint64_t)r[k].y < a.thr || (a.max_moves && step[k] >= a.max_moves));
             if (a.app == PTW_APP_ENDPOINT) {
                 // a walker stuck at its start (no out-edge) ends where it began
@@ -257,7 +295,7 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
                     moved ? nidx[k]
                           : done && mask[k] == kDenseMask ? __ldg(&a.int2idx[PTW_IDX(v[k], a.n, a.check, kCheckCounter)])
                                                           : 0u;
-                visit_agg(kBFull, done, q[k], v[k], eidx, tab[k], mask[k], &a.q_flag[q[k]], lane, a);
+                visit_merged(done, step[k] <= 1 || left_deg <= kCrowdDegree, q[k], v[k], eidx, tab[k], mask[k], &a.q_flag[q[k]], lane, a, pol_tab);
             }
             if (done) act[k] = false;
         }
@@ -265,6 +303,76 @@ __global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
 #pragma unroll
     for (int o = 16; o; o >>= 1) moves += __shfl_xor_sync(kBFull, moves, o);
     if (lane == 0 && moves) atomicAdd(&a.ctrl[1], moves);
+}
+
+// Without row table: two walkers per lane, 256 threads.
+template <bool EXT>
+__global__ void __launch_bounds__(256) k_batch(const BatchArgs a)
+{
+    batch_body<EXT, false, 2>(a, nullptr);
+}
+
+// With it (dynamic shared memory): one walker per lane, two blocks per SM share
+// it with few copies.  Against the extended columns and two walkers per lane,
+// 300-512 queries, budgets 10^3 to 10^6, device results: R-MAT scale 16 3.4 ->
+// 1.8 ms, 20 8.1 -> 5.6, 22 10.7 -> 8.7, Chung-Lu 10^6 vertices 5.2 -> 3.8.
+constexpr int kBatchRowsBlock = 768;
+__global__ void __launch_bounds__(kBatchRowsBlock, 2) k_batch_rows(const BatchArgs a)
+{
+    extern __shared__ __align__(16) uint32_t s_rows[];
+    row_table_load(s_rows, a.rows, a.row_words);
+    __syncthreads();
+    batch_body<false, true, 1>(a, s_rows);
+}
+
+// Kernel, block and shared memory of a batched launch, and the column layout's
+// arguments: the extended columns when asked for, else the row table when the
+// graph has one.
+struct BatchLaunch {
+    const void *fn;
+    int block;
+    size_t smem;
+    int per_sm;  // blocks per SM
+};
+
+// Walker ranks per descriptor for a launch of `walkers` walkers: a warp per
+// descriptor on the whole GPU (48 per SM) before a descriptor gets a second
+// round of 32, since a short launch lasts as long as its slowest warp.
+inline uint32_t desc_walkers_for(const ptw_graph *g, uint64_t walkers)
+{
+    const uint64_t per = walkers / ((uint64_t)g->num_sms * 48) + 1;
+    return (uint32_t)std::min<uint64_t>((per + 31) / 32 * 32, kDescWalkers);
+}
+
+// Blocks of a launch over nd descriptors; with few of them the row table kernel
+// also takes smaller blocks, so that they spread over all SMs.
+inline unsigned batch_grid(const ptw_graph *g, BatchLaunch &l, uint64_t nd)
+{
+    if (l.smem) {
+        const uint64_t per_sm = (nd + g->num_sms - 1) / g->num_sms;
+        l.block = (int)std::max<uint64_t>(1, std::min<uint64_t>(per_sm, kBatchRowsBlock / 32)) * 32;
+    }
+    const uint64_t warps = l.block / 32;
+    return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g->num_sms * l.per_sm, (nd + warps - 1) / warps));
+}
+
+inline int batch_launch(const ptw_graph *g, bool ext, BatchArgs &a, BatchLaunch &l)
+{
+    const bool rows = !ext && g->dg.rows;
+    l.fn = ext ? (const void *)k_batch<true> : rows ? (const void *)k_batch_rows : (const void *)k_batch<false>;
+    l.block = rows ? kBatchRowsBlock : 256;  // at most: batch_grid
+    l.smem = 0;
+    a.col_ext = g->dg.col_ext;
+    if (rows) {
+        a.rows = g->dg.rows;
+        a.row_runs = g->dg.row_runs;
+        a.row_words = row_words(g->dg.row_runs, g->dg.n);
+        l.smem = (size_t)a.row_words * 4;
+        PTW_CUDA(cudaFuncSetAttribute(l.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
+    }
+    PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l.per_sm, l.fn, l.block, l.smem));
+    l.per_sm = std::max(l.per_sm, 1);
+    return PTW_OK;
 }
 
 // ---- compaction of count tables into (name, count) lists ------------------

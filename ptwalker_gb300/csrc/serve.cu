@@ -135,7 +135,7 @@ struct ptw_server {
     std::deque<ptw::Done> done;
     ptw::BatchArgs args{};
     unsigned grid = 1;
-    const void *kfn = nullptr;        // k_batch<false> or k_batch<true> (extended columns)
+    ptw::BatchLaunch launch{};
     bool uses_ext = false;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -198,7 +198,7 @@ int build_tick_graph(ptw_server *s)
     PTW_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
     cudaError_t e1 = cudaMemcpyAsync(s->d_plan, s->h_plan, s->plan_bytes, cudaMemcpyHostToDevice, st);
     void *kargs[] = {&s->args};
-    cudaError_t e2 = cudaLaunchKernel(s->kfn, dim3(s->grid), dim3(256), kargs, 0, st);
+    cudaError_t e2 = cudaLaunchKernel(s->launch.fn, dim3(s->grid), dim3(s->launch.block), kargs, s->launch.smem, st);
     cudaError_t e3 = cudaMemcpyAsync((char *)s->h_plan + s->ret_off, (char *)s->d_plan + s->ret_off,
                                      s->ret_bytes, cudaMemcpyDeviceToHost, st);
     cudaError_t e4 = cudaStreamEndCapture(st, &s->graph);
@@ -363,15 +363,11 @@ try {
         a.key1 = (uint32_t)(cfg->seed >> 32);
         a.max_moves = cfg->max_moves;
         a.app = cfg->app;
-        int per_sm = 0;
-        const bool ext = (g->tune.ext_columns & 1) && ensure_ext_columns(g);
-        a.col_ext = g->dg.col_ext;
-        s->kfn = ext ? (const void *)k_batch<true> : (const void *)k_batch<false>;
+        const bool ext = !g->dg.rows && (g->tune.ext_columns & 1) && ensure_ext_columns(g);
+        rc = batch_launch(g, ext, a, s->launch);
         s->uses_ext = ext;
         if (ext) ++g->ext_users;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, s->kfn, 256, 0);
-        if (e != cudaSuccess) rc = cuda_fail(e, "occupancy");
-        s->grid = (unsigned)std::max(1, g->num_sms * std::max(per_sm, 1));
+        s->grid = (unsigned)std::max(1, g->num_sms * s->launch.per_sm);
         if (rc == PTW_OK) {
             e = cudaEventCreate(&s->ev[0]);
             if (e == cudaSuccess) e = cudaEventCreate(&s->ev[1]);
@@ -469,7 +465,13 @@ try {
         std::vector<uint3> desc;
         std::vector<uint64_t> tbytes(na);
         for (uint32_t i = 0; i < na; ++i) tbytes[i] = s->active[i].cap * 8;
-        interleave_descriptors(j0, s->take, tbytes, kGroupBytes, desc);
+        uint64_t walkers = 0;
+        for (uint64_t t : s->take) walkers += t;
+        // (at most D descriptors: na of them may be cut short)
+        const uint64_t room = s->D > na ? s->D - na : 1, least = ((walkers + room - 1) / room + 31) / 32 * 32;
+        interleave_descriptors(j0, s->take, tbytes, kGroupBytes, desc,
+                               (uint32_t)std::min<uint64_t>(
+                                   std::max<uint64_t>(least, desc_walkers_for(s->g, walkers)), kDescWalkers));
         if (desc.size() > s->D) {
             // more active queries than the plan holds descriptors for: keep
             // the first D (whole queries stay consistent: trim their takes)
@@ -481,18 +483,21 @@ try {
         std::memcpy(hv.desc, desc.data(), desc.size() * sizeof(uint3));
         hv.ctrl[0] = hv.ctrl[1] = 0;
         s->args.ndesc = (uint32_t)desc.size();
+        s->grid = batch_grid(s->g, s->launch, desc.size());
         // 3. the tick
         PTW_CUDA(cudaEventRecord(s->ev[0], st));
         if (s->exec) {
             void *kp[] = {&s->args};
             cudaKernelNodeParams p = s->kparams;
             p.kernelParams = kp;
+            p.gridDim = dim3(s->grid);
+            p.blockDim = dim3(s->launch.block);
             PTW_CUDA(cudaGraphExecKernelNodeSetParams(s->exec, s->knode, &p));
             PTW_CUDA(cudaGraphLaunch(s->exec, st));
         } else {
             PTW_CUDA(cudaMemcpyAsync(s->d_plan, s->h_plan, s->plan_bytes, cudaMemcpyHostToDevice, st));
             void *kargs[] = {&s->args};
-            PTW_CUDA(cudaLaunchKernel(s->kfn, dim3(s->grid), dim3(256), kargs, 0, st));
+            PTW_CUDA(cudaLaunchKernel(s->launch.fn, dim3(s->grid), dim3(s->launch.block), kargs, s->launch.smem, st));
             PTW_CUDA(cudaMemcpyAsync((char *)s->h_plan + s->ret_off, (char *)s->d_plan + s->ret_off,
                                      s->ret_bytes, cudaMemcpyDeviceToHost, st));
         }

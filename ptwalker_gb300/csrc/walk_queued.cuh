@@ -46,17 +46,6 @@ namespace {
 
 constexpr int kQueuedBlock = 1024;  // largest block, one per SM: 768 x 2 and 1024 x 2 were 3-10% slower
 
-// A miss reads the whole 128-byte line from DRAM, and the L2::128B qualifier
-// keeps all of it: for arrays of about the L2's size the next reader of the
-// line then hits (random 4-byte loads: 192 MB 82 -> 97 G/s, 512 MB 58 -> 61,
-// 1 GB and more the same).
-__device__ __forceinline__ uint32_t ld_col_line(const uint32_t *p, uint64_t pol)
-{
-    uint32_t r;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::128B.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
-    return r;
-}
-
 // ROWS: row records from the row table in shared memory instead of adj.
 template <bool ENDPOINT, bool HOT, bool BYNAME, bool GROUP, bool ROWS>
 __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs a)
@@ -101,7 +90,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
         return ld_hint_u2(&a.adj[PTW_IDX(x, a.n, &a.ctrl[7], kCheckRecord)], pol_keep);
     };
     auto gather = [&]() -> uint32_t {
-        return ld_col_line(&a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)],
+        return ld_line_u32(&a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)],
                            pol_stream);
     };
     auto name_of = [&](uint32_t x) -> uint32_t {
