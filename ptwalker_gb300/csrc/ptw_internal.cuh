@@ -27,6 +27,8 @@
 
 namespace ptw {
 
+constexpr size_t kMaxSharedBytes = 227 * 1024;  // dynamic shared memory of a block, sm_103a
+
 // Names a host-side span for profilers (NVTX ranges; nothing is recorded
 // unless a profiler is attached).
 struct NvtxRange {
@@ -242,6 +244,20 @@ __device__ __forceinline__ uint32_t ld_line_u32(const uint32_t *p, uint64_t pol)
     uint32_t r;
     asm("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::128B.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
     return r;
+}
+
+// The same through L1 (tables whose hot entries every SM asks for).
+__device__ __forceinline__ uint32_t ld_hot_u32(const uint32_t *p, uint64_t pol)
+{
+    uint32_t r;
+    asm("ld.global.nc.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(r) : "l"(p), "l"(pol));
+    return r;
+}
+
+// A 4-byte store with an L2 eviction-priority policy.
+__device__ __forceinline__ void st_hint_s32(int32_t *p, int32_t v, uint64_t pol)
+{
+    asm volatile("st.global.L2::cache_hint.s32 [%0], %1, %2;" ::"l"(p), "r"(v), "l"(pol) : "memory");
 }
 
 __device__ __forceinline__ void red_add_hint(uint32_t *p, uint32_t v, uint64_t pol)

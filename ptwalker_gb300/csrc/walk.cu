@@ -32,6 +32,7 @@
 // columns DeepWalk runs in the per-lane loop of node2vec.cu.
 #include <algorithm>
 
+#include "path_rows.cuh"
 #include "ptw_internal.cuh"
 
 namespace ptw {
@@ -467,6 +468,8 @@ inline size_t async_smem(int slots, int block, uint32_t hot_k)
 struct PathArgs {
     const uint2 *__restrict__ adj;
     const uint32_t *__restrict__ col;
+    const uint32_t *__restrict__ rows;    // k_paths_rows: row table
+    uint32_t row_runs, row_words;
     const uint2 *__restrict__ col_named;  // {internal id, name} per column entry
     const uint32_t *__restrict__ start_map;
     const uint32_t *__restrict__ sources;
@@ -584,6 +587,98 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
                                                            pol_keep);
                 stage[wib][g][lane][p - c0] = out;
             }
+        }
+    }
+}
+
+constexpr int kPathRowsBlock = 768;   // many waves: 768 threads per SM (1,024: 5-15% slower)
+constexpr int kPathWaveBlock = 1024;  // one wave
+constexpr uint32_t kPathStage = 32;   // positions collected before they are written
+
+// DeepWalk of a graph whose path parameters are the ones it was built with
+// (paths_launch_is_auto): one walker per lane, warps take groups of 32
+// consecutive walkers in turn (all walks have one length), a move is one 4-byte
+// gather from the plain columns; no column copy is built or read.  The
+// neighbour's name is loaded beside the next gather, through L1 (the hubs'
+// names are asked for by all SMs), and the draw of a move is made while the
+// gather before it is on its way.
+// MANY (more walkers than one wave): the row comes from the row table in shared
+// memory, and a warp's paths are collected there and written 32 positions of
+// one row at a time, first to be evicted from L2: in pieces of 16 bytes they
+// leave it half-filled and cost DRAM a line each time (R-MAT scale 22, 80
+// positions: 39 against 47 G moves/s), at normal priority they push out columns
+// and names (scale 20: 54 against 79).  Otherwise the row record from L2 is as
+// quick, the output fits L2, and paths are written from registers.
+// Against k_paths on name-paired columns, one walker per vertex, 80 positions:
+// scale 10 66 -> 41 us, 16 74 -> 51, 18 169 -> 127, 20 859 -> 643, 22 4,563 ->
+// 3,880 us, 24 19.6 -> 18.3 ms.  At scale 22 a move without names and stores
+// takes as long (50 G moves/s): it is one DRAM line.
+template <bool MANY>
+__global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_paths_rows(const PathArgs a)
+{
+    extern __shared__ __align__(16) uint32_t s_rows[];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int32_t(*stage)[kPathStage + 1] =
+        reinterpret_cast<int32_t(*)[kPathStage + 1]>(s_rows + a.row_words) + warp * 32;
+    if (MANY) {
+        row_table_load(s_rows, a.rows, a.row_words);
+        __syncthreads();
+    }
+    const uint64_t pol_keep = l2_policy(1), pol_stream = l2_policy(2);
+    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
+    const uint64_t n_groups = (a.n_walk + 31) / 32;
+    for (uint64_t g = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp; g < n_groups; g += warps) {
+        const uint64_t j = g * 32 + lane;
+        bool alive = j < a.n_walk;
+        const uint64_t wid = a.w_begin + j;
+        PathOut out;
+        uint32_t v = 0, rx = 0;
+        int32_t name = -1;
+        if (alive) {
+            v = walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
+            name = (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep);
+            rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), 0u, PTW_TAG_WALK), a.key0, a.key1).x;
+            if (!MANY) out.start(a.paths + j * a.L);
+        }
+        // Writes positions [c0, p) of the group's rows, consecutive lanes
+        // consecutive positions of one row.
+        auto flush = [&](uint32_t c0, uint32_t p) {
+            __syncwarp();
+            const uint32_t rows = (uint32_t)umin64(32, a.n_walk - g * 32);
+            int32_t *o = a.paths + g * 32 * a.L + c0 + lane;
+            if (c0 + lane < p)
+#pragma unroll 4
+                for (uint32_t r = 0; r < rows; ++r) st_hint_s32(o + (uint64_t)r * a.L, stage[r][lane], pol_stream);
+            __syncwarp();
+        };
+        const bool valid = alive;
+        for (uint32_t p = 1; p < a.L; ++p) {
+            if (alive) {
+                const uint32_t x = (uint32_t)PTW_IDX(v, a.n, a.check, kCheckRecord);
+                const uint2 rec = MANY ? row_of(s_rows, a.row_runs, x) : ld_hint_u2(&a.adj[x], pol_keep);
+                alive = rec.y != 0;  // no out-edge: -1 from here on
+                if (alive)
+                    v = ld_line_u32(
+                        &a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, a.check, kCheckColumn)], pol_stream);
+            }
+            if (MANY) {
+                stage[lane][(p - 1) % kPathStage] = name;
+                if (p % kPathStage == 0) flush(p - kPathStage, p);
+            } else if (valid) {
+                out.put(p - 1, name);
+            }
+            name = -1;
+            if (alive) {
+                rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), p, PTW_TAG_WALK), a.key0, a.key1).x;
+                name = (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep);
+            }
+        }
+        if (MANY) {
+            stage[lane][(a.L - 1) % kPathStage] = name;
+            flush((a.L - 1) / kPathStage * kPathStage, a.L);
+        } else if (valid) {
+            out.put(a.L - 1, name);
+            out.finish(a.L);
         }
     }
 }
@@ -712,6 +807,13 @@ bool walk_launch_is_auto(const ptw_tune &t)
     return t.block == d.block && t.ilp == d.ilp && t.chunk == d.chunk && t.hot_k == d.hot_k &&
            t.blocks_per_sm == d.blocks_per_sm && t.min_blocks == d.min_blocks && t.cache_hints == d.cache_hints &&
            !(t.ext_columns & 1) && t.gather_slots == d.gather_slots && t.warp_agg == d.warp_agg;
+}
+
+static bool paths_launch_is_auto(const ptw_tune &t)
+{
+    const ptw_tune d = default_tune();
+    return t.paths_ilp == d.paths_ilp && t.paths_named == d.paths_named && t.cache_hints == d.cache_hints &&
+           !(t.ext_columns & 2);
 }
 
 bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
@@ -917,7 +1019,7 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
                  int start_mode, uint32_t n_sources, int32_t *paths)
 {
     const DeviceGraph &dg = g->dg;
-    PathArgs a;
+    PathArgs a{};
     a.adj = dg.adj;
     a.col = dg.col;
     a.start_map = dg.idx2int;
@@ -935,6 +1037,25 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
     a.n_sources = n_sources;
     a.start_mode = start_mode;
     a.hints = g->tune.cache_hints;
+    // One wave: as few threads per SM as the walkers take, so that all SMs share
+    // them.  A graph without row table takes the name-paired columns for more.
+    const uint64_t sm_walkers = (a.n_walk + g->num_sms - 1) / g->num_sms;
+    const bool many = sm_walkers > (uint64_t)kPathWaveBlock;
+    const uint32_t words = many && dg.rows ? row_words(dg.row_runs, dg.n) : 0u;
+    const size_t path_smem = many ? (size_t)kPathRowsBlock * (kPathStage + 1) * 4 + words * 4ull : 0;
+    if (paths_launch_is_auto(g->tune) && (!many || (dg.rows && path_smem <= kMaxSharedBytes))) {
+        const int block = many ? kPathRowsBlock : (int)(std::max<uint64_t>(1, (sm_walkers + 31) / 32) * 32);
+        const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms, (a.n_walk + block - 1) / block));
+        const void *fn = many ? (const void *)k_paths_rows<true> : (const void *)k_paths_rows<false>;
+        a.rows = dg.rows;
+        a.row_runs = dg.row_runs;
+        a.row_words = words;
+        if (path_smem > 48 * 1024)
+            PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)path_smem));
+        void *args[] = {&a};
+        PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(block), args, path_smem, g->stream));
+        return PTW_OK;
+    }
     // Extended columns (16 bytes per CSR entry) take precedence; then
     // name-paired columns, built once on the first path walk (8 bytes per
     // CSR entry); without either the kernel looks names up per move.
