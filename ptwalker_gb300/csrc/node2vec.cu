@@ -54,30 +54,44 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kLaneWarps = 4;                // warps per block
+constexpr uint32_t kLaneWaveWalkers = 512;   // per SM: those resident without a register limit
+constexpr uint32_t kFirstDrawNames = 8u << 20;  // p = q = 1: vertices up to which the plain columns are walked
 constexpr uint32_t kN2vMaxTrials = 65536u;  // trials per move before the last is taken
 
-// MurmurHash3 64-bit finaliser (Appleby, public domain).
-__host__ __device__ __forceinline__ uint64_t fmix64(uint64_t k)
+// MurmurHash3 32-bit finaliser (Appleby, public domain).
+__device__ __forceinline__ uint32_t fmix32(uint32_t k)
 {
-    k ^= k >> 33;
-    k *= 0xff51afd7ed558ccdull;
-    k ^= k >> 33;
-    k *= 0xc4ceb9fe1a85ec53ull;
-    k ^= k >> 33;
+    k ^= k >> 16;
+    k *= 0x85ebca6bu;
+    k ^= k >> 13;
+    k *= 0xc2b2ae35u;
+    k ^= k >> 16;
     return k;
 }
 
-// Filter block of the directed edge (u, v) (internal ids) and the bit of
-// each of its 8 words.
+// Filter block of the directed edge (u, v) (internal ids) and the bit of each
+// of its 8 words, from two 32-bit hashes of different mixtures of u and v (a
+// test is 25 instructions that way, 60 with 64-bit hashes).
 struct FilterKey {
     uint64_t block;
-    uint64_t bits;  // 5 bits per word
+    uint32_t a, b;
+    __device__ __forceinline__ uint32_t bit(int j) const { return (j < 6 ? a >> (5 * j) : b >> (5 * (j - 6))) & 31; }
 };
 
 __device__ __forceinline__ FilterKey filter_key(uint32_t u, uint32_t v, uint64_t blocks)
 {
-    const uint64_t key = ((uint64_t)u << 32) | v;
-    return FilterKey{fmix64(key) & (blocks - 1), fmix64(key + 0x9E3779B97F4A7C15ull)};
+    const uint32_t h = fmix32(u * 0xcc9e2d51u + v);
+    const uint32_t a = fmix32(v * 0x1b873593u ^ (u + 0x7f4a7c15u));
+    return FilterKey{h & (blocks - 1), a, (a * 0x9E3779B1u) >> 22};
+}
+
+// The 32 bytes of a filter block in one request: two of 16 bytes to a sector
+// that L2 does not hold read its line from DRAM twice.
+__device__ __forceinline__ void ld_block(uint4 &x, uint4 &y, const uint32_t *p, uint64_t pol)
+{
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;"
+        : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w), "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+        : "l"(p), "l"(pol));
 }
 
 // One warp per vertex: sets the bits of every out-edge.
@@ -90,9 +104,10 @@ __global__ void k_build_edge_filter(const uint2 *__restrict__ adj, const uint32_
         const uint2 r = adj[u];
         for (uint32_t i = lane; i < r.y; i += 32) {
             const FilterKey fk = filter_key((uint32_t)u, col[(uint64_t)r.x + i], blocks);
-            uint32_t *blk = filter + fk.block * 8;
+            unsigned long long *blk = reinterpret_cast<unsigned long long *>(filter + fk.block * 8);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) atomicOr(&blk[j], 1u << ((fk.bits >> (5 * j)) & 31));
+            for (int j = 0; j < 4; ++j)
+                atomicOr(&blk[j], 1ull << fk.bit(2 * j) | 1ull << (32 + fk.bit(2 * j + 1)));
         }
     }
 }
@@ -124,6 +139,14 @@ struct LaneArgs {
 // Walker slot states.
 enum : uint32_t { kIdle = 0, kDraw = 1, kFilter = 2, kSearch = 3 };
 
+// The filter stays in L2, the columns stream through it; node2vec of more walkers
+// than are resident without a limit (WAVE: at most those) is held to 64 registers,
+// for 1,024 walkers per SM (R-MAT scale 22 7,616 -> 7,420 us, 12 385 -> 403).
+// Against 64-bit hashes, two 16-byte reads per block and the filter streaming as
+// well, p = 2, q = 0.5, one walker per vertex: scale 12 401 -> 383 us, 18 895 ->
+// 865, 20 2,296 -> 2,131, 22 7,820 -> 7,478, 24 27.5 -> 27.0 ms.  Slower: candidates and names from the plain or name-paired columns with
+// rows from the row table (scale 20 2,841 and 2,615 us: a pass is bound by its
+// instructions, and the 16-byte entry saves the lookup).
 // ILP walker slots per lane, each an independent state machine: every pass
 // of the loop issues one read per active slot -- a candidate's column entry
 // (kDraw), an edge-filter block (kFilter) or one entry of the previous
@@ -138,8 +161,8 @@ enum : uint32_t { kIdle = 0, kDraw = 1, kFilter = 2, kSearch = 3 };
 // candidate, the neighbour mulhi(x, degree) of
 // Philox(ctr = (wid_lo, wid_hi, s, "WALK")), the draw of the other walk
 // kernels.
-template <int ILP>
-__global__ void __launch_bounds__(kLaneWarps * 32) k_lane_paths(const LaneArgs a)
+template <int ILP, bool WAVE>
+__global__ void __launch_bounds__(kLaneWarps * 32, WAVE ? 1 : 8) k_lane_paths(const LaneArgs a)
 {
     constexpr uint32_t C = 32;
     __shared__ int32_t stage[kLaneWarps][ILP][32][C + 1];
@@ -278,18 +301,16 @@ __global__ void __launch_bounds__(kLaneWarps * 32) k_lane_paths(const LaneArgs a
                 }
                 if (appx[s]) x[s] = make_uint4(t[s], trec[s].x, trec[s].y, tname[s]);
                 else
-                    x[s] = ld_hint_u4(&a.col_ext[PTW_IDX((uint64_t)rec[s].x + idx, a.m, &a.ctrl[7], kCheckColumn)],
+                    x[s] = ld_line_u4(&a.col_ext[PTW_IDX((uint64_t)rec[s].x + idx, a.m, &a.ctrl[7], kCheckColumn)],
                                       pol_stream);
             } else if (st[s] == kFilter) {
                 const FilterKey fk = filter_key(t[s], cx[s].x, a.filter_blocks);
-                fbits[s] = fk.bits;
-                const uint4 *blk = reinterpret_cast<const uint4 *>(
-                    a.filter + PTW_IDX(fk.block, a.filter_blocks, &a.ctrl[7], kCheckFilter) * 8);
-                x[s] = ld_hint_u4(blk, pol_stream);
-                x2[s] = ld_hint_u4(blk + 1, pol_stream);
+                fbits[s] = (uint64_t)fk.b << 30 | (fk.a & 0x3FFFFFFFu);
+                const uint32_t *blk = a.filter + PTW_IDX(fk.block, a.filter_blocks, &a.ctrl[7], kCheckFilter) * 8;
+                ld_block(x[s], x2[s], blk, pol_keep);
             } else if (st[s] == kSearch) {
                 mid[s] = lo[s] + ((hi[s] - lo[s]) >> 1);
-                x[s] = ld_hint_u4(&a.col_ext[PTW_IDX((uint64_t)soff[s] + mid[s], a.m, &a.ctrl[7], kCheckColumn)],
+                x[s] = ld_line_u4(&a.col_ext[PTW_IDX((uint64_t)soff[s] + mid[s], a.m, &a.ctrl[7], kCheckColumn)],
                                   pol_stream);
             }
         }
@@ -456,11 +477,9 @@ bool ensure_edge_filter(ptw_graph *g)
 
 namespace {
 
-// Launches k_lane_paths<ILP>, ILP = 1, 2 or 4.
-int launch_lane_paths(ptw_graph *g, LaneArgs &a, int ilp)
+// Launches fn, a k_lane_paths of ilp slots per lane.
+int launch_lane_paths(ptw_graph *g, LaneArgs &a, const void *fn, int ilp)
 {
-    const void *fn = ilp == 1 ? (const void *)k_lane_paths<1>
-                              : ilp == 4 ? (const void *)k_lane_paths<4> : (const void *)k_lane_paths<2>;
     int per_sm = 0;
     PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, kLaneWarps * 32, 0));
     per_sm = std::max(per_sm, 1);
@@ -506,6 +525,11 @@ int launch_node2vec(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, 
     if (!ensure_ext_columns(g) || !ensure_edge_filter(g))
         return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
                                 "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
+    // Every first draw is accepted: the plain columns, while the names stay in L2
+    // beside them (scale 18 273 -> 160 us, 20 1,086 -> 719, 22 4,119 -> 3,838; 24
+    // 15.3 ms against 18.4).
+    if (p == 1.0 && q == 1.0 && g->dg.n <= kFirstDrawNames && paths_rows_apply(g, w_end - w_begin))
+        return launch_paths(g, w_begin, w_end, L, seed, start_mode, n_sources, paths, PTW_TAG_N2V, g->sc.ctrl + 1);
     LaneArgs a = lane_args(g, w_begin, w_end, L, seed, start_mode, n_sources, paths);
     a.thr_ret = thr[0];
     a.thr_nb = thr[1];
@@ -524,11 +548,14 @@ int launch_node2vec(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, 
             a.fold_fx = (uint64_t)((w[0] - m) / m * 1048576.0);
         }
     }
-    a.tag = PTW_TAG_N2V;
     // One slot per lane: with rejections the slots of a lane wait on each
     // other's reads (R-MAT scale 24, p = 2, q = 0.5: 24.9 / 22.8 / 12.8 G
     // moves/s with 1 / 2 / 4 slots).
-    return launch_lane_paths(g, a, 1);
+    a.tag = PTW_TAG_N2V;
+    const bool wave = a.n_walk <= (uint64_t)g->num_sms * kLaneWaveWalkers;
+    return launch_lane_paths(g, a,
+                             wave ? (const void *)k_lane_paths<1, true> : (const void *)k_lane_paths<1, false>,
+                             1);
 }
 
 int launch_lane_deepwalk(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
@@ -538,7 +565,12 @@ int launch_lane_deepwalk(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_
     LaneArgs a = lane_args(g, w_begin, w_end, L, seed, start_mode, n_sources, paths);
     a.thr_ret = a.thr_nb = a.thr_out = 1ull << 32;  // every first candidate accepted
     a.tag = PTW_TAG_WALK;
-    return launch_lane_paths(g, a, g->tune.paths_ilp == 1 || g->tune.paths_ilp == 4 ? g->tune.paths_ilp : 2);
+    const int ilp = g->tune.paths_ilp == 1 || g->tune.paths_ilp == 4 ? g->tune.paths_ilp : 2;
+    return launch_lane_paths(g, a,
+                             ilp == 1   ? (const void *)k_lane_paths<1, true>
+                             : ilp == 4 ? (const void *)k_lane_paths<4, true>
+                                        : (const void *)k_lane_paths<2, true>,
+                             ilp);
 }
 
 }  // namespace ptw

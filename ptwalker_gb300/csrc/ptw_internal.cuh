@@ -246,7 +246,17 @@ __device__ __forceinline__ uint32_t ld_line_u32(const uint32_t *p, uint64_t pol)
     return r;
 }
 
-// The same through L1 (tables whose hot entries every SM asks for).
+// The 16-byte form.
+__device__ __forceinline__ uint4 ld_line_u4(const uint4 *p, uint64_t pol)
+{
+    uint4 r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.L2::128B.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
+        : "l"(p), "l"(pol));
+    return r;
+}
+
+// The 4-byte gather through L1 (tables whose hot entries every SM asks for).
 __device__ __forceinline__ uint32_t ld_hot_u32(const uint32_t *p, uint64_t pol)
 {
     uint32_t r;
@@ -379,7 +389,11 @@ bool walk_launch_is_auto(const ptw_tune &t);
 bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk);
 int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t);
 int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
-                 int start_mode, uint32_t n_sources, int32_t *paths);
+                 int start_mode, uint32_t n_sources, int32_t *paths,
+                 uint32_t tag = PTW_TAG_WALK, unsigned long long *counters = nullptr);
+// launch_paths takes k_paths_rows for n_walk walkers (which counts moves and draws
+// in counters, if not null).
+bool paths_rows_apply(const ptw_graph *g, uint64_t n_walk);
 // Second-order (node2vec) paths (node2vec.cu): thr = acceptance thresholds
 // {return, neighbour of the previous vertex, other} for the envelope
 // max(1/p, 1, 1/q) (p and q pick the folded form on simple symmetric

@@ -470,6 +470,11 @@ struct PathArgs {
     const uint32_t *__restrict__ col;
     const uint32_t *__restrict__ rows;    // k_paths_rows: row table
     uint32_t row_runs, row_words;
+    unsigned long long *counters;         // k_paths_rows: {moves, draws} of node2vec, or null
+    uint32_t tag;                         // draw tag: "WALK" or "N2"
+    const uint4 *__restrict__ col_ext;    // extended columns: {id, first column, degree, name} per entry
+    const uint4 *__restrict__ vtx_ext;    // and per vertex, by canonical index
+    const uint32_t *__restrict__ int2idx;
     const uint2 *__restrict__ col_named;  // {internal id, name} per column entry
     const uint32_t *__restrict__ start_map;
     const uint32_t *__restrict__ sources;
@@ -593,6 +598,7 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
 
 constexpr int kPathRowsBlock = 768;   // many waves: 768 threads per SM (1,024: 5-15% slower)
 constexpr int kPathWaveBlock = 1024;  // one wave
+constexpr uint64_t kPathExtBytes = 512ull << 20;  // extended columns up to here: k_paths_rows
 constexpr uint32_t kPathStage = 32;   // positions collected before they are written
 
 // DeepWalk of a graph whose path parameters are the ones it was built with
@@ -613,31 +619,46 @@ constexpr uint32_t kPathStage = 32;   // positions collected before they are wri
 // scale 10 66 -> 41 us, 16 74 -> 51, 18 169 -> 127, 20 859 -> 643, 22 4,563 ->
 // 3,880 us, 24 19.6 -> 18.3 ms.  At scale 22 a move without names and stores
 // takes as long (50 G moves/s): it is one DRAM line.
-template <bool MANY>
+// EXT (extended columns asked for): the record and the name come with the 16-byte
+// entry.  Against k_lane_paths, scale 10 to 16 91 - 102 -> 31 - 37 us, 18 311 ->
+// 216, 19 606 -> 475, 20 1,127 -> 1,080 us; of columns that DRAM holds for the most
+// part (kPathExtBytes) k_lane_paths reads more (scale 22 4.1 against 4.7 ms).
+// node2vec with p = q = 1 accepts every first draw: the same walk with its tag.
+template <bool MANY, bool EXT>
 __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_paths_rows(const PathArgs a)
 {
     extern __shared__ __align__(16) uint32_t s_rows[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int32_t(*stage)[kPathStage + 1] =
         reinterpret_cast<int32_t(*)[kPathStage + 1]>(s_rows + a.row_words) + warp * 32;
-    if (MANY) {
+    if (MANY && !EXT) {
         row_table_load(s_rows, a.rows, a.row_words);
         __syncthreads();
     }
     const uint64_t pol_keep = l2_policy(1), pol_stream = l2_policy(2);
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t n_groups = (a.n_walk + 31) / 32;
+    unsigned long long moves = 0;
     for (uint64_t g = (uint64_t)blockIdx.x * (blockDim.x >> 5) + warp; g < n_groups; g += warps) {
         const uint64_t j = g * 32 + lane;
         bool alive = j < a.n_walk;
         const uint64_t wid = a.w_begin + j;
         PathOut out;
         uint32_t v = 0, rx = 0;
+        uint2 rec = make_uint2(0u, 0u);
         int32_t name = -1;
         if (alive) {
-            v = walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
-            name = (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep);
-            rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), 0u, PTW_TAG_WALK), a.key0, a.key1).x;
+            if (EXT) {
+                const uint32_t i =
+                    walker_start_index(a.start_mode, a.int2idx, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
+                const uint4 x = ld_hint_u4(&a.vtx_ext[PTW_IDX(i, a.n, a.check, kCheckRecord)], pol_keep);
+                rec = make_uint2(x.y, x.z);
+                name = (int32_t)x.w;
+            } else {
+                v = walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
+                name = (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep);
+            }
+            rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), 0u, a.tag), a.key0, a.key1).x;
             if (!MANY) out.start(a.paths + j * a.L);
         }
         // Writes positions [c0, p) of the group's rows, consecutive lanes
@@ -653,13 +674,23 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
         };
         const bool valid = alive;
         for (uint32_t p = 1; p < a.L; ++p) {
+            uint32_t next_name = ~0u;  // EXT
             if (alive) {
-                const uint32_t x = (uint32_t)PTW_IDX(v, a.n, a.check, kCheckRecord);
-                const uint2 rec = MANY ? row_of(s_rows, a.row_runs, x) : ld_hint_u2(&a.adj[x], pol_keep);
+                if (!EXT) {
+                    const uint32_t x = (uint32_t)PTW_IDX(v, a.n, a.check, kCheckRecord);
+                    rec = MANY ? row_of(s_rows, a.row_runs, x) : ld_hint_u2(&a.adj[x], pol_keep);
+                }
                 alive = rec.y != 0;  // no out-edge: -1 from here on
-                if (alive)
-                    v = ld_line_u32(
-                        &a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, a.check, kCheckColumn)], pol_stream);
+                if (alive) {
+                    const uint64_t e = PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, a.check, kCheckColumn);
+                    if (EXT) {
+                        const uint4 x = ld_hint_u4(&a.col_ext[e], pol_stream);
+                        rec = make_uint2(x.y, x.z);
+                        next_name = x.w;
+                    } else {
+                        v = ld_line_u32(&a.col[e], pol_stream);
+                    }
+                }
             }
             if (MANY) {
                 stage[lane][(p - 1) % kPathStage] = name;
@@ -667,11 +698,10 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
             } else if (valid) {
                 out.put(p - 1, name);
             }
-            name = -1;
-            if (alive) {
-                rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), p, PTW_TAG_WALK), a.key0, a.key1).x;
-                name = (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep);
-            }
+            if (alive) rx = philox(make_uint4((uint32_t)wid, (uint32_t)(wid >> 32), p, a.tag), a.key0, a.key1).x;
+            if (EXT) name = (int32_t)next_name;
+            else name = alive ? (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v, a.n, a.check, kCheckCounter)], pol_keep) : -1;
+            moves += alive;
         }
         if (MANY) {
             stage[lane][(a.L - 1) % kPathStage] = name;
@@ -679,6 +709,14 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
         } else if (valid) {
             out.put(a.L - 1, name);
             out.finish(a.L);
+        }
+    }
+    if (a.counters) {  // node2vec: every move is its first draw
+#pragma unroll
+        for (int o = 16; o; o >>= 1) moves += __shfl_xor_sync(~0u, moves, o);
+        if (lane == 0 && moves) {
+            atomicAdd(&a.counters[0], moves);
+            atomicAdd(&a.counters[1], moves);
         }
     }
 }
@@ -1015,8 +1053,30 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     return PTW_OK;
 }
 
+namespace {
+
+// k_paths_rows: walkers of one wave, or more of them with a row table whose
+// copy fits beside the collected positions.
+bool path_rows_many(const ptw_graph *g, uint64_t n_walk)
+{
+    return (n_walk + g->num_sms - 1) / g->num_sms > (uint64_t)kPathWaveBlock;
+}
+
+size_t path_rows_smem(uint32_t table_words)
+{
+    return (size_t)kPathRowsBlock * (kPathStage + 1) * 4 + table_words * 4ull;
+}
+
+}  // namespace
+
+bool paths_rows_apply(const ptw_graph *g, uint64_t n_walk)
+{
+    return paths_launch_is_auto(g->tune) &&
+           (!path_rows_many(g, n_walk) || (g->dg.rows && path_rows_smem(row_words(g->dg.row_runs, g->dg.n)) <= kMaxSharedBytes));
+}
+
 int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
-                 int start_mode, uint32_t n_sources, int32_t *paths)
+                 int start_mode, uint32_t n_sources, int32_t *paths, uint32_t tag, unsigned long long *counters)
 {
     const DeviceGraph &dg = g->dg;
     PathArgs a{};
@@ -1037,29 +1097,35 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
     a.n_sources = n_sources;
     a.start_mode = start_mode;
     a.hints = g->tune.cache_hints;
-    // One wave: as few threads per SM as the walkers take, so that all SMs share
-    // them.  A graph without row table takes the name-paired columns for more.
-    const uint64_t sm_walkers = (a.n_walk + g->num_sms - 1) / g->num_sms;
-    const bool many = sm_walkers > (uint64_t)kPathWaveBlock;
-    const uint32_t words = many && dg.rows ? row_words(dg.row_runs, dg.n) : 0u;
-    const size_t path_smem = many ? (size_t)kPathRowsBlock * (kPathStage + 1) * 4 + words * 4ull : 0;
-    if (paths_launch_is_auto(g->tune) && (!many || (dg.rows && path_smem <= kMaxSharedBytes))) {
+    a.tag = tag;
+    a.counters = counters;
+    const bool ext = (g->tune.ext_columns & 2) && ensure_ext_columns(g);
+    const bool many = path_rows_many(g, a.n_walk);
+    if (paths_rows_apply(g, a.n_walk) || (ext && (!many || dg.m * sizeof(uint4) <= kPathExtBytes))) {
+        // One wave: as few threads per SM as the walkers take, so that all SMs
+        // share them.
+        const uint64_t sm_walkers = (a.n_walk + g->num_sms - 1) / g->num_sms;
         const int block = many ? kPathRowsBlock : (int)(std::max<uint64_t>(1, (sm_walkers + 31) / 32) * 32);
         const uint64_t blocks = std::max<uint64_t>(1, std::min<uint64_t>(g->num_sms, (a.n_walk + block - 1) / block));
-        const void *fn = many ? (const void *)k_paths_rows<true> : (const void *)k_paths_rows<false>;
+        const void *fn = ext    ? (many ? (const void *)k_paths_rows<true, true> : (const void *)k_paths_rows<false, true>)
+                         : many ? (const void *)k_paths_rows<true, false>
+                                : (const void *)k_paths_rows<false, false>;
         a.rows = dg.rows;
         a.row_runs = dg.row_runs;
-        a.row_words = words;
-        if (path_smem > 48 * 1024)
-            PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)path_smem));
+        a.row_words = many && !ext ? row_words(dg.row_runs, dg.n) : 0u;
+        const size_t smem = many ? path_rows_smem(a.row_words) : 0;
+        a.col_ext = g->dg.col_ext;
+        a.vtx_ext = g->dg.vtx_ext;
+        a.int2idx = dg.int2idx;
+        if (smem > 48 * 1024)
+            PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         void *args[] = {&a};
-        PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(block), args, path_smem, g->stream));
+        PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(block), args, smem, g->stream));
         return PTW_OK;
     }
     // Extended columns (16 bytes per CSR entry) take precedence; then
     // name-paired columns, built once on the first path walk (8 bytes per
     // CSR entry); without either the kernel looks names up per move.
-    const bool ext = (g->tune.ext_columns & 2) && ensure_ext_columns(g);
     bool named = !ext && g->tune.paths_named != 0;
     if (named && !g->dg.col_named) {
         uint2 *cn = nullptr;
