@@ -106,6 +106,19 @@ void trim_pools()
         if (p) cudaMemPoolTrimTo(p, 0);
 }
 
+void release_pool_above(cudaStream_t st, uint64_t keep)
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    uint64_t held = 0;
+    if (!g_pools[dev] || cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+        held <= keep)
+        return;
+    cudaStreamSynchronize(st);  // frees queued on st have happened
+    cudaMemPoolTrimTo(g_pools[dev], keep);
+}
+
 cudaError_t device_malloc_bytes(void **p, size_t bytes)
 {
     cudaError_t e = cudaMalloc(p, bytes);
@@ -251,8 +264,8 @@ int upload_and_build(const uint32_t *h_src, const uint32_t *h_dst, uint64_t m, b
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
-        cudaError_t e = cudaMallocAsync(&d_src, m * 4, g->stream);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_dst, m * 4, g->stream);
+        cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
+        if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_src, h_src, m * 4, cudaMemcpyHostToDevice, g->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_dst, h_dst, m * 4, cudaMemcpyHostToDevice, g->stream);
         if (e != cudaSuccess) {
@@ -731,8 +744,8 @@ try {
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
-        cudaError_t e = cudaMallocAsync(&d_src, m * 4, g->stream);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_dst, m * 4, g->stream);
+        cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
+        if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e != cudaSuccess) {
             rc = cuda_fail(e, "R-MAT edge buffers");
             if (d_src) cudaFreeAsync(d_src, g->stream);
@@ -770,8 +783,8 @@ try {
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
-        cudaError_t e = cudaMallocAsync(&d_src, m * 4, g->stream);
-        if (e == cudaSuccess) e = cudaMallocAsync(&d_dst, m * 4, g->stream);
+        cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
+        if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e != cudaSuccess) {
             rc = cuda_fail(e, "Chung-Lu edge buffers");
             if (d_src) cudaFreeAsync(d_src, g->stream);

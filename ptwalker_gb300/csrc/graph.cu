@@ -10,12 +10,14 @@
 // array, where the 129 MB L2 keeps them.
 //
 // Pipeline (all on the graph's stream):
-//   edges -> packed u64 keys (src<<b | dst) -> [drop self-loops] -> radix
-//   sort -> [unique] -> names = sorted unique endpoints -> index space ->
-//   degrees -> stable sort by degree (desc) -> internal CSR.
+//   edges -> names = ascending distinct endpoints, index of every name ->
+//   packed u64 keys (src index << b | dst index) [without self-loops] -> radix
+//   sort -> [unique] -> row bounds, degrees -> stable sort by degree (desc) ->
+//   internal CSR.
 #include <cub/cub.cuh>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -25,6 +27,7 @@ namespace ptw {
 namespace {
 
 constexpr int kThreads = 256;
+constexpr uint64_t kBuildPoolKeep = 1ull << 30;
 
 inline unsigned grid_for(uint64_t n, int threads = kThreads)
 {
@@ -32,54 +35,56 @@ inline unsigned grid_for(uint64_t n, int threads = kThreads)
     return (unsigned)std::min<uint64_t>(std::max<uint64_t>(b, 1), 1u << 20);
 }
 
-__global__ void k_max2(const uint32_t *a, const uint32_t *b, uint64_t m, unsigned *out)
+// Largest of 2m names; one atomic per block.
+__global__ void __launch_bounds__(kThreads) k_max2(const uint32_t *a, const uint32_t *b, uint64_t m, unsigned *out)
 {
+    __shared__ unsigned s_mx[kThreads / 32];
     unsigned mx = 0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        mx = max(mx, max(a[i], b[i]));
-    for (int o = 16; o; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(out, mx);
-}
-
-__global__ void k_make_keys(const uint32_t *src, const uint32_t *dst, uint64_t m, int bits,
-                            bool both, bool drop_loops, unsigned long long *keys,
-                            unsigned long long *n_out)
-{
-    // Warp-uniform trip count: blockDim is a multiple of 32, so every lane of
-    // a warp runs the same iterations and the full-mask scan below is legal.
-    const unsigned lane = threadIdx.x & 31;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i0 = blockIdx.x * (uint64_t)blockDim.x + (threadIdx.x & ~31u); i0 < m; i0 += stride) {
-        const uint64_t i = i0 + lane;
-        const bool valid = i < m;
-        const uint64_t u = valid ? src[i] : 0, v = valid ? dst[i] : 0;
-        const bool keep = valid && !(drop_loops && u == v);
-        const unsigned nk = keep ? (both ? 2u : 1u) : 0u;
-        // Warp-aggregated slot reservation keeps the output dense.
-        unsigned incl = nk;
-        for (int o = 1; o < 32; o <<= 1) {
-            unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= (unsigned)o) incl += t;
-        }
-        const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-        unsigned long long base = 0;
-        if (lane == 31 && total) base = atomicAdd(n_out, (unsigned long long)total);
-        base = __shfl_sync(0xffffffffu, base, 31);
-        const uint64_t pos = base + incl - nk;
-        if (nk >= 1) keys[pos] = (u << bits) | v;
-        if (nk == 2) keys[pos + 1] = (v << bits) | u;
+    const uint64_t t = blockIdx.x * (uint64_t)kThreads + threadIdx.x, stride = (uint64_t)gridDim.x * kThreads;
+    const uint4 *a4 = reinterpret_cast<const uint4 *>(a), *b4 = reinterpret_cast<const uint4 *>(b);
+    for (uint64_t i = t; i < m / 4; i += stride) {
+        const uint4 x = a4[i], y = b4[i];
+        mx = max(mx, max(max(max(x.x, x.y), max(x.z, x.w)), max(max(y.x, y.y), max(y.z, y.w))));
+    }
+    for (uint64_t i = (m & ~3ull) + t; i < m; i += stride) mx = max(mx, max(a[i], b[i]));
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) s_mx[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x < kThreads / 32) {
+        mx = __reduce_max_sync((1u << (kThreads / 32)) - 1, s_mx[threadIdx.x]);
+        if (threadIdx.x == 0) atomicMax(out, mx);
     }
 }
 
-__global__ void k_split_keys(const unsigned long long *keys, uint64_t m, int bits, uint32_t *s,
-                             uint32_t *d)
+// seen[x] = 1 for both names of every edge (of every edge that is not a
+// self-loop), *n_out += edges.  A name already seen is only read: hubs stay in L1.
+__global__ void __launch_bounds__(kThreads) k_mark_names(const uint32_t *src, const uint32_t *dst, uint64_t m,
+                                                         bool drop_loops, uint32_t *seen, unsigned long long *n_out)
 {
-    const unsigned long long mask = (1ull << bits) - 1;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        s[i] = (uint32_t)(keys[i] >> bits);
-        d[i] = (uint32_t)(keys[i] & mask);
+    __shared__ unsigned long long s_n;
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    unsigned n = 0;
+    for (uint64_t i = blockIdx.x * (uint64_t)kThreads + threadIdx.x; i < m; i += (uint64_t)gridDim.x * kThreads) {
+        const uint32_t u = src[i], v = dst[i];
+        if (drop_loops && u == v) continue;
+        ++n;
+        if (!seen[u]) seen[u] = 1;
+        if (!seen[v]) seen[v] = 1;
+    }
+    if (n) atomicAdd(&s_n, (unsigned long long)n);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_n) atomicAdd(n_out, s_n);
+}
+
+// names[index_of[x]] = x of every name seen (index_of: exclusive sums of the
+// marks, [bound + 1]); *n_out = their number.
+__global__ void k_collect_names(const uint32_t *index_of, uint64_t bound, uint32_t *names, unsigned long long *n_out)
+{
+    for (uint64_t x = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; x < bound; x += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t i = index_of[x], j = index_of[x + 1];
+        if (i != j) names[i] = (uint32_t)x;
+        if (x + 1 == bound) *n_out = j;
     }
 }
 
@@ -94,32 +99,68 @@ __device__ __forceinline__ uint32_t lower_bound_u32(const uint32_t *a, uint32_t 
     return lo;
 }
 
-// Names -> canonical indices, in place.
-__global__ void k_to_index(uint32_t *x, uint64_t m, const uint32_t *names, uint32_t n)
+// keys[i] = (index of src[i]) << bits | index of dst[i], and the reverse in
+// keys[m + i] (both).  A dropped self-loop becomes the last key of all: no kept
+// edge of a graph without loops equals it.  index_of null: indices by search of
+// the n names.
+__global__ void k_make_keys(const uint32_t *src, const uint32_t *dst, uint64_t m, int bits, bool both, bool drop_loops,
+                            const uint32_t *index_of, const uint32_t *names, uint32_t n, unsigned long long *keys)
 {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        x[i] = lower_bound_u32(names, n, x[i]);
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t u = src[i], v = dst[i];
+        unsigned long long k = ~0ull >> (64 - 2 * bits), r = k;
+        if (!(drop_loops && u == v)) {
+            const unsigned long long a = index_of ? index_of[u] : lower_bound_u32(names, n, u);
+            const unsigned long long b = index_of ? index_of[v] : lower_bound_u32(names, n, v);
+            k = a << bits | b;
+            r = b << bits | a;
+        }
+        keys[i] = k;
+        if (both) keys[m + i] = r;
+    }
 }
 
-// Row bounds from the sorted source indices, without atomics (a hub of
+// Row bounds from the sorted keys, without atomics (a hub of
 // degree d would otherwise serialise d atomics on one counter): the first
 // entry of a run of v records first[v], the last records end[v].
-__global__ void k_row_bounds(const uint32_t *si, uint64_t m, uint32_t *first, uint32_t *end)
+__global__ void k_row_bounds(const unsigned long long *keys, uint64_t m, int bits, uint32_t *first, uint32_t *end)
 {
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < m;
          i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t v = si[i];
-        if (i == 0 || si[i - 1] != v) first[v] = (uint32_t)i;
-        if (i + 1 == m || si[i + 1] != v) end[v] = (uint32_t)(i + 1);
+        const uint32_t v = (uint32_t)(keys[i] >> bits);
+        if (i == 0 || (uint32_t)(keys[i - 1] >> bits) != v) first[v] = (uint32_t)i;
+        if (i + 1 == m || (uint32_t)(keys[i + 1] >> bits) != v) end[v] = (uint32_t)(i + 1);
     }
 }
 
 // deg[v] = end[v] - first[v] in place (both 0 for a vertex without out-edges).
-__global__ void k_degree_from_bounds(uint32_t *end_deg, const uint32_t *first, uint32_t n)
+__global__ void k_degrees(uint32_t *end_deg, const uint32_t *first, uint32_t n, uint32_t *iota)
 {
-    for (uint64_t v = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; v < n; v += (uint64_t)gridDim.x * blockDim.x)
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         end_deg[v] -= first[v];
+        iota[v] = v;
+    }
+}
+
+// Everything of internal vertex i = rank by degree, order[i] its canonical index,
+// off the exclusive sums of deg.  shift[index]: internal minus canonical place of
+// a row.  run: {0: runs of equal degree (also beyond max_runs), largest degree},
+// then {id, first column, degree} of each run's first vertex, unordered.
+__global__ void k_relabel(const uint32_t *order, const uint32_t *deg, const uint32_t *off, const uint32_t *first,
+                          const uint32_t *names, bool compact, uint32_t n, uint32_t *idx2int, uint32_t *int2name,
+                          uint2 *adj, uint32_t *shift, uint32_t max_runs, uint4 *run)
+{
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t idx = order[i], d = deg[i], o = off[i];
+        idx2int[idx] = i;
+        int2name[i] = compact ? idx : names[idx];
+        adj[i] = make_uint2(o, d);
+        shift[idx] = o - first[idx];
+        if (i == 0) run[0].y = d;
+        if (i != 0 && deg[i - 1] == d) continue;
+        const uint32_t p = atomicAdd(&run[0].x, 1u);
+        if (p < max_runs) run[1 + p] = make_uint4(i, o, d, 0u);
+    }
 }
 
 __global__ void k_iota(uint32_t *x, uint32_t n)
@@ -128,66 +169,65 @@ __global__ void k_iota(uint32_t *x, uint32_t n)
         x[i] = i;
 }
 
-// order[i] = canonical index of internal vertex i.
-__global__ void k_relabel(const uint32_t *order, const uint32_t *deg_idx, const uint32_t *names,
-                          uint32_t n, uint32_t *idx2int, uint32_t *int_deg, uint32_t *int2name)
+// Canonical edges into internal rows.
+__global__ void k_fill_col(const unsigned long long *keys, uint64_t m, int bits, const uint32_t *shift,
+                           const uint32_t *idx2int, uint32_t *col)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t idx = order[i];
-        idx2int[idx] = i;
-        int_deg[i] = deg_idx[idx];
-        int2name[i] = names[idx];
+    const uint32_t mask = (uint32_t)((1ull << bits) - 1);
+    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
+        const unsigned long long k = keys[e];
+        col[shift[k >> bits] + (uint32_t)e] = idx2int[(uint32_t)k & mask];
     }
 }
 
-__global__ void k_adj(const uint32_t *int_deg, const uint32_t *int_off, uint32_t n, uint2 *adj)
-{
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        adj[i] = make_uint2(int_off[i], int_deg[i]);
-}
+// Canonical export: kExportTile consecutive columns per warp.  A row per warp left
+// it to one warp to copy a hub and 27 lanes of most others idle (16 M entries, 3 M
+// rows: 695 -> 124 us).  Rows lie in the order of their columns; those of a tile are found
+// from its two ends, by division where all have one degree.
+constexpr uint32_t kExportTile = 256;
 
-// Appends {id, first column, degree} of every vertex that starts a run of
-// equal degree (unordered; run[0].x counts them, also beyond max_runs).
-__global__ void k_row_runs(const uint2 *adj, uint32_t n, uint32_t max_runs, uint4 *run)
+__device__ __forceinline__ uint32_t row_with(const uint2 *adj, uint32_t lo, uint32_t hi, uint32_t e)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint2 r = adj[i];
-        if (i != 0 && adj[i - 1].y == r.y) continue;
-        const uint32_t p = atomicAdd(&run[0].x, 1u);
-        if (p < max_runs) run[1 + p] = make_uint4(i, r.x, r.y, 0u);
+    while (hi - lo > 1) {  // adj[lo].x <= e < adj[hi].x (hi may be n)
+        const uint32_t mid = lo + (hi - lo) / 2;
+        if (adj[mid].x <= e) lo = mid;
+        else hi = mid;
     }
+    return lo;
 }
 
-// Scatter canonical edges into internal rows.  Edge e belongs to canonical
-// row si[e]; its rank inside the row is e - row_ptr[si[e]].
-__global__ void k_fill_col(const uint32_t *si, const uint32_t *di, const uint32_t *row_ptr,
-                           uint64_t m, const uint32_t *idx2int, const uint2 *adj, uint32_t *col)
-{
-    for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m;
-         e += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t s = si[e];
-        const uint32_t r = (uint32_t)(e - row_ptr[s]);
-        col[adj[idx2int[s]].x + r] = idx2int[di[e]];
-    }
-}
-
-// Canonical export: one warp per internal row.
-__global__ void k_export(const uint2 *adj, const uint32_t *col, const uint32_t *int2idx,
-                         const uint32_t *canon_off, uint32_t n, uint32_t *out_col)
+__global__ void k_export(const uint2 *adj, const uint32_t *col, const uint32_t *int2idx, const uint32_t *canon_off,
+                         uint32_t n_rows, uint64_t m, uint32_t *out_col)
 {
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
-    for (uint64_t i = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; i < n; i += warps) {
-        const uint2 a = adj[i];
-        const uint32_t base = canon_off[int2idx[i]];
-        for (uint32_t r = lane; r < a.y; r += 32) out_col[base + r] = int2idx[col[a.x + r]];
+    for (uint64_t t = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; t * kExportTile < m; t += warps) {
+        const uint64_t e0 = t * kExportTile, e1 = e0 + kExportTile < m ? e0 + kExportTile : m;
+        uint32_t row = 0;
+        if (lane < 2) row = row_with(adj, 0, n_rows, (uint32_t)(lane ? e1 - 1 : e0));
+        const uint32_t lo = __shfl_sync(0xffffffffu, row, 0), hi = __shfl_sync(0xffffffffu, row, 1);
+        const uint2 first = adj[lo];
+        const bool even = first.y == adj[hi].y;
+        for (uint64_t e = e0 + lane; e < e1; e += 32) {
+            const uint32_t r = even ? lo + ((uint32_t)e - first.x) / first.y : row_with(adj, lo, hi + 1, (uint32_t)e);
+            const uint32_t start = even ? first.x + (r - lo) * first.y : adj[r].x;
+            out_col[canon_off[int2idx[r]] + ((uint32_t)e - start)] = int2idx[col[e]];
+        }
     }
 }
 
+// Degrees by canonical index, [n + 1] with a 0 at the end.
 __global__ void k_deg_by_index(const uint2 *adj, const uint32_t *idx2int, uint32_t n, uint32_t *deg)
 {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        deg[i] = adj[idx2int[i]].y;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x)
+        deg[i] = i < n ? adj[idx2int[i]].y : 0u;
+}
+
+// Row offsets as the caller takes them.
+__global__ void k_widen(const uint32_t *x, uint64_t n, unsigned long long *y)
+{
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        y[i] = x[i];
 }
 
 __global__ void k_rmat(uint32_t scale, uint64_t m, uint32_t ta, uint32_t tab, uint32_t tabc,
@@ -289,7 +329,7 @@ struct AsyncBufs {
     template <typename T> cudaError_t alloc(T **p, uint64_t count)
     {
         void *q = nullptr;
-        cudaError_t e = cudaMallocAsync(&q, std::max<uint64_t>(count, 1) * sizeof(T), st);
+        cudaError_t e = pooled_alloc_async(&q, std::max<uint64_t>(count, 1) * sizeof(T), st);
         if (e == cudaSuccess) ptrs.push_back(q);
         *p = (T *)q;
         return e;
@@ -315,7 +355,7 @@ template <typename F> cudaError_t cub_call(F f, cudaStream_t st)
     cudaError_t e = f(nullptr, bytes);
     if (e != cudaSuccess) return e;
     void *tmp = nullptr;
-    e = cudaMallocAsync(&tmp, std::max<size_t>(bytes, 16), st);
+    e = pooled_alloc_async(&tmp, std::max<size_t>(bytes, 16), st);
     if (e != cudaSuccess) return e;
     e = f(tmp, bytes);
     cudaFreeAsync(tmp, st);
@@ -346,19 +386,12 @@ void graph_release(ptw_graph *g)
 {
     if (!g) return;
     if (g->stream) cudaStreamSynchronize(g->stream);
-    cudaFree(g->dg.adj);
+    cudaFree(g->vertex_arrays);  // adj, int2name, idx2int, int2idx, names, rows, sc.counts, sc.ctrl
     cudaFree(g->dg.col);
-    cudaFree(g->dg.int2name);
-    cudaFree(g->dg.idx2int);
-    cudaFree(g->dg.int2idx);
-    cudaFree(g->dg.names);
     cudaFree(g->dg.col_named);
     cudaFree(g->dg.col_ext);
     cudaFree(g->dg.vtx_ext);
-    cudaFree(g->dg.rows);
     cudaFree(g->dg.edge_filter);
-    cudaFree(g->sc.counts);
-    cudaFree(g->sc.ctrl);
     cudaFree(g->sc.sources);
     cudaFree(g->sc.by_name);
     cudaFree(g->sc.out_stage);
@@ -431,8 +464,8 @@ int csr_to_device_edges(const uint64_t *h_row_ptr, const uint32_t *h_col, const 
         tmp.release(sorted);
     }
     // The edge arrays are handed to the caller, so they are not in tmp.
-    PTW_CUDA(cudaMallocAsync(&src, std::max<uint64_t>(m, 1) * 4, st));
-    cudaError_t e = cudaMallocAsync(&dst, std::max<uint64_t>(m, 1) * 4, st);
+    PTW_CUDA(pooled_alloc_async((void **)&src, std::max<uint64_t>(m, 1) * 4, st));
+    cudaError_t e = pooled_alloc_async((void **)&dst, std::max<uint64_t>(m, 1) * 4, st);
     if (e != cudaSuccess) {
         cudaFreeAsync(src, st);
         return cuda_fail(e, "CSR edge buffers");
@@ -455,12 +488,12 @@ int csr_to_device_edges(const uint64_t *h_row_ptr, const uint32_t *h_col, const 
 
 namespace {
 
-// Builds the row table from the runs of equal degree (k_row_runs); none when
-// there are more than kMaxRowRuns of them.
-int build_row_table(ptw_graph *g, const std::vector<uint4> &found)
+// Host image of the row table from the runs of equal degree (k_relabel); empty
+// when there are more than kMaxRowRuns of them.
+std::vector<uint32_t> row_table_image(const std::vector<uint4> &found, uint32_t n)
 {
-    const uint32_t runs = found[0].x, n = g->dg.n;
-    if (runs > kMaxRowRuns) return PTW_OK;
+    const uint32_t runs = found[0].x;
+    if (runs > kMaxRowRuns) return {};
     std::vector<uint4> run(found.begin() + 1, found.begin() + 1 + runs);
     std::sort(run.begin(), run.end(), [](const uint4 &x, const uint4 &y) { return x.x < y.x; });
     std::vector<uint32_t> img(row_words(runs, n), 0u);
@@ -480,11 +513,196 @@ int build_row_table(ptw_graph *g, const std::vector<uint4> &found)
         const uint32_t last = row_bucket(end - 1);
         for (; next <= last; ++next) bucket[next] = (uint16_t)k;
     }
-    PTW_CUDA(device_malloc(&g->dg.rows, img.size() * 4));
-    PTW_CUDA(cudaMemcpyAsync(g->dg.rows, img.data(), img.size() * 4, cudaMemcpyHostToDevice, g->stream));
-    PTW_CUDA(cudaStreamSynchronize(g->stream));  // img is read until then
-    g->dg.row_runs = runs;
-    g->device_bytes += img.size() * 4;
+    return img;
+}
+
+// The arrays of a graph whose size is known with its vertices, in one allocation
+// (of a small graph's build, seven of them were a fifth).
+int alloc_vertex_arrays(ptw_graph *g, uint32_t n, uint32_t max_runs)
+{
+    DeviceGraph &dg = g->dg;
+    uint64_t bytes = 0;
+    auto take = [&](uint64_t b) {
+        const uint64_t at = bytes;
+        bytes += (b + 255) & ~255ull;
+        return at;
+    };
+    const uint64_t adj = take((uint64_t)n * sizeof(uint2)), int2name = take(n * 4ull), idx2int = take(n * 4ull),
+                   int2idx = take(n * 4ull), names = take(n * 4ull), counts = take(n * 4ull),
+                   ctrl = take(16 * sizeof(unsigned long long)), rows = take(row_words(max_runs, n) * 4ull);
+    PTW_CUDA(device_malloc(&g->vertex_arrays, bytes));
+    char *p = static_cast<char *>(g->vertex_arrays);
+    dg.adj = reinterpret_cast<uint2 *>(p + adj);
+    dg.int2name = reinterpret_cast<uint32_t *>(p + int2name);
+    dg.idx2int = reinterpret_cast<uint32_t *>(p + idx2int);
+    dg.int2idx = reinterpret_cast<uint32_t *>(p + int2idx);
+    dg.names = reinterpret_cast<uint32_t *>(p + names);
+    g->sc.counts = reinterpret_cast<uint32_t *>(p + counts);
+    g->sc.ctrl = reinterpret_cast<unsigned long long *>(p + ctrl);
+    g->row_space = reinterpret_cast<uint32_t *>(p + rows);
+    return PTW_OK;
+}
+
+// Device time of 8 M edges, both directions, 3 M names below 12 M: names and keys
+// from a table over the name range 0.26 ms (sorting all endpoints for the distinct
+// ones and searching those for every endpoint: 1.6 ms), the sort of the keys 1.0
+// ms (six passes at 1.7 TB/s of reads and writes), rows and columns 0.3 ms.
+// R-MAT scale 20 7.8 -> 3.6 ms, 22 29 -> 16, 24 119 -> 68; 1,087 edges 449 -> 300 us.
+int build_arrays(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, bool as_undirected, bool clean,
+                 bool compact_names)
+{
+    cudaStream_t st = g->stream;
+    AsyncBufs tmp(st);
+    tmp.ptrs = {d_src, d_dst};
+    if (m == 0) return fail(PTW_EINVAL, "edge list is empty");
+    const unsigned wide = (unsigned)g->num_sms * 8;
+
+    // Name range.
+    unsigned *d_max = nullptr;
+    unsigned long long *d_cnt = nullptr;  // {edges kept, vertices, entries after unique}
+    PTW_CUDA(tmp.alloc(&d_cnt, 4));
+    PTW_CUDA(cudaMemsetAsync(d_cnt, 0, 4 * sizeof(unsigned long long), st));
+    d_max = reinterpret_cast<unsigned *>(d_cnt + 3);
+    k_max2<<<std::min(grid_for(m / 4), wide), kThreads, 0, st>>>(d_src, d_dst, m, d_max);
+    unsigned h_max = 0;
+    PTW_CUDA(cudaMemcpyAsync(&h_max, d_max, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+    PTW_CUDA(cudaStreamSynchronize(st));
+    const uint64_t id_bound = (uint64_t)h_max + 1;
+    const uint64_t cap = as_undirected ? 2 * m : m;
+
+    // Names, and the index of each: over the name range while that is not far
+    // above the number of entries (4 bytes of it against the two sorts' 32 per
+    // entry), else by sorting the endpoints (edges of a clean graph come from the
+    // generators, whose vertices are their range).
+    const bool table = clean || id_bound <= 4 * cap;
+    uint32_t *index_of = nullptr, *names = nullptr;
+    unsigned long long h_cnt[2] = {m, 0};
+    if (table) {
+        PTW_CUDA(tmp.alloc(&index_of, id_bound + 1));
+        PTW_CUDA(tmp.alloc(&names, std::min(id_bound, 2 * m)));
+        PTW_CUDA(cudaMemsetAsync(index_of, 0, (id_bound + 1) * 4, st));
+        k_mark_names<<<std::min(grid_for(m), wide), kThreads, 0, st>>>(d_src, d_dst, m, clean, index_of, d_cnt);
+        PTW_CUDA(cub_call([&](void *t, size_t &b) {
+            return cub::DeviceScan::ExclusiveSum(t, b, index_of, index_of, (int64_t)id_bound + 1, st);
+        }, st));
+        k_collect_names<<<grid_for(id_bound), kThreads, 0, st>>>(index_of, id_bound, names, d_cnt + 1);
+        PTW_CUDA(cudaGetLastError());
+        PTW_CUDA(cudaMemcpyAsync(h_cnt, d_cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
+    } else {
+        uint32_t *ends = nullptr;
+        PTW_CUDA(tmp.alloc(&ends, 2 * m));
+        PTW_CUDA(tmp.alloc(&names, 2 * m));
+        PTW_CUDA(cudaMemcpyAsync(ends, d_src, m * 4, cudaMemcpyDeviceToDevice, st));
+        PTW_CUDA(cudaMemcpyAsync(ends + m, d_dst, m * 4, cudaMemcpyDeviceToDevice, st));
+        cub::DoubleBuffer<uint32_t> db(ends, names);
+        PTW_CUDA(cub_call([&](void *t, size_t &b) {
+            return cub::DeviceRadixSort::SortKeys(t, b, db, (int64_t)(2 * m), 0, bits_for(id_bound), st);
+        }, st));
+        if (db.Current() == names) std::swap(ends, names);
+        PTW_CUDA(cub_call([&](void *t, size_t &b) {
+            return cub::DeviceSelect::Unique(t, b, ends, names, d_cnt + 1, (int64_t)(2 * m), st);
+        }, st));
+        tmp.release(ends);
+        PTW_CUDA(cudaMemcpyAsync(h_cnt + 1, d_cnt + 1, sizeof(h_cnt[1]), cudaMemcpyDeviceToHost, st));
+    }
+    PTW_CUDA(cudaStreamSynchronize(st));
+    uint64_t mm = as_undirected ? 2 * h_cnt[0] : h_cnt[0];
+    const uint32_t n = (uint32_t)h_cnt[1];
+    if (mm == 0) return fail(PTW_EINVAL, "graph has no edges after clean-up");
+    if (mm >= (1ull << 32)) return fail(PTW_EINVAL, "graphs with 2^32 or more CSR entries are not supported");
+
+    // Packed keys, sorted.
+    const int bits = bits_for(n);
+    unsigned long long *keys = nullptr, *keys_alt = nullptr;
+    PTW_CUDA(tmp.alloc(&keys, cap));
+    k_make_keys<<<grid_for(m), kThreads, 0, st>>>(d_src, d_dst, m, bits, as_undirected, clean, index_of, names, n, keys);
+    PTW_CUDA(cudaGetLastError());
+    tmp.release(d_src);
+    tmp.release(d_dst);
+    if (index_of) tmp.release(index_of);
+    PTW_CUDA(tmp.alloc(&keys_alt, cap));
+    {
+        cub::DoubleBuffer<unsigned long long> db(keys, keys_alt);
+        PTW_CUDA(cub_call([&](void *t, size_t &b) {
+            return cub::DeviceRadixSort::SortKeys(t, b, db, (int64_t)cap, 0, 2 * bits, st);
+        }, st));
+        if (db.Current() != keys) std::swap(keys, keys_alt);
+    }
+    if (clean) {
+        PTW_CUDA(cub_call([&](void *t, size_t &b) {
+            return cub::DeviceSelect::Unique(t, b, keys, keys_alt, d_cnt + 2, (int64_t)mm, st);
+        }, st));
+        PTW_CUDA(cudaMemcpyAsync(h_cnt, d_cnt + 2, sizeof(h_cnt[0]), cudaMemcpyDeviceToHost, st));
+        PTW_CUDA(cudaStreamSynchronize(st));
+        std::swap(keys, keys_alt);
+        mm = h_cnt[0];
+    }
+    tmp.release(keys_alt);
+
+    // The distinct degrees d of a graph sum up to mm at most.
+    const uint32_t max_runs =
+        (uint32_t)std::min<uint64_t>(std::min<uint64_t>(n, kMaxRowRuns), (uint64_t)std::sqrt(2.0 * (double)mm) + 2);
+    DeviceGraph &dg = g->dg;
+    dg.n = n;
+    dg.m = mm;
+    dg.id_bound = compact_names ? n : (uint32_t)id_bound;
+    int rc = alloc_vertex_arrays(g, n, max_runs);
+    if (rc) return rc;
+    PTW_CUDA(device_malloc(&dg.col, mm * 4));
+
+    // Degrees; internal order: stable sort of canonical indices by descending
+    // degree; rows in that order.
+    uint32_t *first = nullptr, *deg = nullptr, *deg_sorted = nullptr, *iota = nullptr;
+    uint4 *d_run = nullptr;
+    PTW_CUDA(tmp.alloc(&first, 2ull * n));
+    deg = first + n;
+    PTW_CUDA(tmp.alloc(&deg_sorted, n));
+    PTW_CUDA(tmp.alloc(&iota, n));
+    PTW_CUDA(tmp.alloc(&d_run, 1ull + max_runs));
+    PTW_CUDA(cudaMemsetAsync(first, 0, n * 8ull, st));
+    PTW_CUDA(cudaMemsetAsync(d_run, 0, sizeof(uint4), st));
+    PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 16 * sizeof(unsigned long long), st));  // [7]: index checks
+    k_row_bounds<<<grid_for(mm), kThreads, 0, st>>>(keys, mm, bits, first, deg);
+    k_degrees<<<grid_for(n), kThreads, 0, st>>>(deg, first, n, iota);
+    PTW_CUDA(cub_call([&](void *t, size_t &b) {
+        return cub::DeviceRadixSort::SortPairsDescending(t, b, deg, deg_sorted, iota, dg.int2idx, (int64_t)n, 0,
+                                                         bits_for(mm + 1), st);
+    }, st));
+    uint32_t *off = iota, *shift = deg;  // reuse
+    PTW_CUDA(cub_call([&](void *t, size_t &b) {
+        return cub::DeviceScan::ExclusiveSum(t, b, deg_sorted, off, (int64_t)n, st);
+    }, st));
+    k_relabel<<<grid_for(n), kThreads, 0, st>>>(dg.int2idx, deg_sorted, off, first, names, compact_names, n, dg.idx2int,
+                                                dg.int2name, dg.adj, shift, max_runs, d_run);
+    if (compact_names) k_iota<<<grid_for(n), kThreads, 0, st>>>(dg.names, n);
+    else PTW_CUDA(cudaMemcpyAsync(dg.names, names, n * 4ull, cudaMemcpyDeviceToDevice, st));
+    PTW_CUDA(cudaGetLastError());
+    std::vector<uint4> h_run(1 + max_runs);
+    PTW_CUDA(cudaMemcpyAsync(h_run.data(), d_run, h_run.size() * sizeof(uint4), cudaMemcpyDeviceToHost, st));
+    PTW_CUDA(cudaStreamSynchronize(st));
+
+    // The host makes the row table while the columns are filled.
+    k_fill_col<<<grid_for(mm), kThreads, 0, st>>>(keys, mm, bits, shift, dg.idx2int, dg.col);
+    PTW_CUDA(cudaGetLastError());
+    const std::vector<uint32_t> img = row_table_image(h_run, n);
+    if (!img.empty()) {
+        PTW_CUDA(cudaMemcpyAsync(g->row_space, img.data(), img.size() * 4, cudaMemcpyHostToDevice, st));
+        dg.rows = g->row_space;
+        dg.row_runs = h_run[0].x;
+    }
+    // Host copy of the ascending names for source lookups.
+    g->h_names = new (std::nothrow) uint32_t[n];
+    if (!g->h_names) return fail(PTW_ENOMEM, "host allocation of the name table failed");
+    PTW_CUDA(cudaMemcpyAsync(g->h_names, dg.names, (uint64_t)n * 4, cudaMemcpyDeviceToHost, st));
+    g->h_idx2int = new (std::nothrow) uint32_t[n];
+    if (!g->h_idx2int) return fail(PTW_ENOMEM, "host allocation of the index table failed");
+    PTW_CUDA(cudaMemcpyAsync(g->h_idx2int, dg.idx2int, (uint64_t)n * 4, cudaMemcpyDeviceToHost, st));
+    PTW_CUDA(cudaStreamSynchronize(st));
+    dg.max_degree = h_run[0].y;
+    // symmetrised, self-loops dropped and duplicates removed: simple and
+    // symmetric by construction (node2vec then skips its check)
+    dg.simple_symmetric = as_undirected && clean ? 1 : -1;
+    g->device_bytes = (uint64_t)n * (8 + 4 * 4 + 4) + mm * 4 + 64 + img.size() * 4;
     return PTW_OK;
 }
 
@@ -493,169 +711,11 @@ int build_row_table(ptw_graph *g, const std::vector<uint4> &found)
 int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m,
                                   bool as_undirected, bool clean, bool compact_names)
 {
-    cudaStream_t st = g->stream;
-    AsyncBufs tmp(st);
-    if (m == 0) return fail(PTW_EINVAL, "edge list is empty");
-
-    // Name range -> key packing width.
-    unsigned *d_max = nullptr;
-    PTW_CUDA(tmp.alloc(&d_max, 1));
-    PTW_CUDA(cudaMemsetAsync(d_max, 0, sizeof(unsigned), st));
-    k_max2<<<grid_for(m), kThreads, 0, st>>>(d_src, d_dst, m, d_max);
-    unsigned h_max = 0;
-    PTW_CUDA(cudaMemcpyAsync(&h_max, d_max, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
-    PTW_CUDA(cudaStreamSynchronize(st));
-    const uint64_t id_bound = (uint64_t)h_max + 1;
-    const int bits = bits_for(id_bound);
-
-    // Packed keys, optionally symmetrised / without self-loops.
-    const uint64_t cap = as_undirected ? 2 * m : m;
-    unsigned long long *keys = nullptr, *keys_alt = nullptr, *d_cnt = nullptr;
-    PTW_CUDA(tmp.alloc(&keys, cap));
-    PTW_CUDA(tmp.alloc(&d_cnt, 2));
-    PTW_CUDA(cudaMemsetAsync(d_cnt, 0, 2 * sizeof(unsigned long long), st));
-    k_make_keys<<<grid_for(m), kThreads, 0, st>>>(d_src, d_dst, m, bits, as_undirected, clean, keys,
-                                                  d_cnt);
-    PTW_CUDA(cudaGetLastError());
-    unsigned long long h_cnt = 0;
-    PTW_CUDA(cudaMemcpyAsync(&h_cnt, d_cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    PTW_CUDA(cudaStreamSynchronize(st));
-    cudaFreeAsync(d_src, st);
-    cudaFreeAsync(d_dst, st);
-    uint64_t mm = h_cnt;
-    if (mm == 0) return fail(PTW_EINVAL, "graph has no edges after clean-up");
-    if (mm >= (1ull << 32)) return fail(PTW_EINVAL, "graphs with 2^32 or more CSR entries are not supported");
-
-    PTW_CUDA(tmp.alloc(&keys_alt, mm));
-    {
-        cub::DoubleBuffer<unsigned long long> db(keys, keys_alt);
-        PTW_CUDA(cub_call([&](void *t, size_t &b) {
-            return cub::DeviceRadixSort::SortKeys(t, b, db, (int64_t)mm, 0, 2 * bits, st);
-        }, st));
-        if (db.Current() != keys) std::swap(keys, keys_alt);
-    }
-    if (clean) {
-        PTW_CUDA(cub_call([&](void *t, size_t &b) {
-            return cub::DeviceSelect::Unique(t, b, keys, keys_alt, d_cnt + 1, (int64_t)mm, st);
-        }, st));
-        PTW_CUDA(cudaMemcpyAsync(&h_cnt, d_cnt + 1, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-        PTW_CUDA(cudaStreamSynchronize(st));
-        std::swap(keys, keys_alt);
-        mm = h_cnt;
-    }
-    tmp.release(keys_alt);
-
-    // Split into (src, dst) names, then the sorted unique name set.
-    uint32_t *si = nullptr, *di = nullptr, *nm = nullptr, *nm_alt = nullptr;
-    PTW_CUDA(tmp.alloc(&si, mm));
-    PTW_CUDA(tmp.alloc(&di, mm));
-    k_split_keys<<<grid_for(mm), kThreads, 0, st>>>(keys, mm, bits, si, di);
-    tmp.release(keys);
-    PTW_CUDA(tmp.alloc(&nm, 2 * mm));
-    PTW_CUDA(tmp.alloc(&nm_alt, 2 * mm));
-    PTW_CUDA(cudaMemcpyAsync(nm, si, mm * 4, cudaMemcpyDeviceToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(nm + mm, di, mm * 4, cudaMemcpyDeviceToDevice, st));
-    {
-        cub::DoubleBuffer<uint32_t> db(nm, nm_alt);
-        PTW_CUDA(cub_call([&](void *t, size_t &b) {
-            return cub::DeviceRadixSort::SortKeys(t, b, db, (int64_t)(2 * mm), 0, bits, st);
-        }, st));
-        if (db.Current() != nm) std::swap(nm, nm_alt);
-    }
-    PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceSelect::Unique(t, b, nm, nm_alt, d_cnt + 1, (int64_t)(2 * mm), st);
-    }, st));
-    PTW_CUDA(cudaMemcpyAsync(&h_cnt, d_cnt + 1, sizeof(h_cnt), cudaMemcpyDeviceToHost, st));
-    PTW_CUDA(cudaStreamSynchronize(st));
-    const uint32_t n = (uint32_t)h_cnt;
-    uint32_t *names = nm_alt;  // [n] ascending
-    tmp.release(nm);
-
-    k_to_index<<<grid_for(mm), kThreads, 0, st>>>(si, mm, names, n);
-    k_to_index<<<grid_for(mm), kThreads, 0, st>>>(di, mm, names, n);
-    if (compact_names) k_iota<<<grid_for(n), kThreads, 0, st>>>(names, n);
-    PTW_CUDA(cudaGetLastError());
-
-    // Degrees and canonical row offsets (u32: mm < 2^32).
-    uint32_t *deg = nullptr, *row_ptr = nullptr;
-    PTW_CUDA(tmp.alloc(&deg, n + 1));
-    PTW_CUDA(tmp.alloc(&row_ptr, n + 1));
-    PTW_CUDA(cudaMemsetAsync(deg, 0, (n + 1) * 4ull, st));
-    {
-        uint32_t *first = nullptr;
-        PTW_CUDA(tmp.alloc(&first, n));
-        PTW_CUDA(cudaMemsetAsync(first, 0, n * 4ull, st));
-        k_row_bounds<<<grid_for(mm), kThreads, 0, st>>>(si, mm, first, deg);
-        k_degree_from_bounds<<<grid_for(n), kThreads, 0, st>>>(deg, first, n);
-        tmp.release(first);
-    }
-    PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceScan::ExclusiveSum(t, b, deg, row_ptr, (int64_t)n + 1, st);
-    }, st));
-
-    // Internal order: stable sort of canonical indices by descending degree.
-    uint32_t *deg_keys = nullptr, *deg_keys_out = nullptr, *iota = nullptr, *order = nullptr;
-    PTW_CUDA(tmp.alloc(&deg_keys_out, n));
-    PTW_CUDA(tmp.alloc(&iota, n));
-    PTW_CUDA(tmp.alloc(&order, n));
-    deg_keys = deg;
-    k_iota<<<grid_for(n), kThreads, 0, st>>>(iota, n);
-    PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceRadixSort::SortPairsDescending(t, b, deg_keys, deg_keys_out, iota, order,
-                                                         (int64_t)n, 0, 32, st);
-    }, st));
-    uint32_t h_maxdeg = 0;
-    PTW_CUDA(cudaMemcpyAsync(&h_maxdeg, deg_keys_out, 4, cudaMemcpyDeviceToHost, st));
-
-    DeviceGraph &dg = g->dg;
-    dg.n = n;
-    dg.m = mm;
-    dg.id_bound = compact_names ? n : (uint32_t)id_bound;
-    PTW_CUDA(device_malloc(&dg.adj, (uint64_t)n * sizeof(uint2)));
-    PTW_CUDA(device_malloc(&dg.col, mm * 4));
-    PTW_CUDA(device_malloc(&dg.int2name, (uint64_t)n * 4));
-    PTW_CUDA(device_malloc(&dg.idx2int, (uint64_t)n * 4));
-    PTW_CUDA(device_malloc(&dg.int2idx, (uint64_t)n * 4));
-    PTW_CUDA(cudaMemcpyAsync(dg.int2idx, order, (uint64_t)n * 4, cudaMemcpyDeviceToDevice, st));
-    PTW_CUDA(device_malloc(&dg.names, (uint64_t)n * 4));
-    PTW_CUDA(cudaMemcpyAsync(dg.names, names, (uint64_t)n * 4, cudaMemcpyDeviceToDevice, st));
-    uint32_t *int_deg = iota;  // reuse
-    k_relabel<<<grid_for(n), kThreads, 0, st>>>(order, deg, names, n, dg.idx2int, int_deg,
-                                                dg.int2name);
-    uint32_t *int_off = deg_keys_out;  // reuse
-    PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceScan::ExclusiveSum(t, b, int_deg, int_off, (int64_t)n, st);
-    }, st));
-    k_adj<<<grid_for(n), kThreads, 0, st>>>(int_deg, int_off, n, dg.adj);
-    k_fill_col<<<grid_for(mm), kThreads, 0, st>>>(si, di, row_ptr, mm, dg.idx2int, dg.adj, dg.col);
-    PTW_CUDA(cudaGetLastError());
-
-    // Host copy of the ascending names for source lookups.
-    g->h_names = new (std::nothrow) uint32_t[n];
-    if (!g->h_names) return fail(PTW_ENOMEM, "host allocation of the name table failed");
-    PTW_CUDA(cudaMemcpyAsync(g->h_names, names, (uint64_t)n * 4, cudaMemcpyDeviceToHost, st));
-    g->h_idx2int = new (std::nothrow) uint32_t[n];
-    if (!g->h_idx2int) return fail(PTW_ENOMEM, "host allocation of the index table failed");
-    PTW_CUDA(cudaMemcpyAsync(g->h_idx2int, dg.idx2int, (uint64_t)n * 4, cudaMemcpyDeviceToHost, st));
-
-    // Scratch reused by every walk.
-    PTW_CUDA(device_malloc(&g->sc.counts, (uint64_t)n * 4));
-    PTW_CUDA(device_malloc(&g->sc.ctrl, 16 * sizeof(unsigned long long)));
-    PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 16 * sizeof(unsigned long long), st));  // [7]: index checks
-    uint4 *d_run = nullptr;
-    std::vector<uint4> h_run(1 + kMaxRowRuns);
-    PTW_CUDA(tmp.alloc(&d_run, h_run.size()));
-    PTW_CUDA(cudaMemsetAsync(d_run, 0, sizeof(uint4), st));
-    k_row_runs<<<grid_for(n), kThreads, 0, st>>>(dg.adj, n, kMaxRowRuns, d_run);
-    PTW_CUDA(cudaGetLastError());
-    PTW_CUDA(cudaMemcpyAsync(h_run.data(), d_run, h_run.size() * sizeof(uint4), cudaMemcpyDeviceToHost, st));
-    PTW_CUDA(cudaStreamSynchronize(st));
-    dg.max_degree = h_maxdeg;
-    // symmetrised, self-loops dropped and duplicates removed: simple and
-    // symmetric by construction (node2vec then skips its check)
-    dg.simple_symmetric = as_undirected && clean ? 1 : -1;
-    g->device_bytes = (uint64_t)n * (8 + 4 * 4 + 4) + mm * 4 + 64;
-    return build_row_table(g, h_run);
+    const int rc = build_arrays(g, d_src, d_dst, m, as_undirected, clean, compact_names);
+    // The temporaries come from the pool that batches use: mapping fresh memory
+    // takes longer than a small build.  A large one hands back what it added.
+    release_pool_above(g->stream, kBuildPoolKeep);
+    return rc;
 }
 
 }  // namespace ptw
@@ -685,27 +745,27 @@ try {
     PTW_CUDA(cudaSetDevice(g->device));
     AsyncBufs tmp(st);
     uint32_t *deg = nullptr, *off = nullptr;
-    PTW_CUDA(tmp.alloc(&deg, dg.n + 1));
-    PTW_CUDA(tmp.alloc(&off, dg.n + 1));
-    PTW_CUDA(cudaMemsetAsync(deg + dg.n, 0, 4, st));
-    k_deg_by_index<<<grid_for(dg.n), kThreads, 0, st>>>(dg.adj, dg.idx2int, dg.n, deg);
+    PTW_CUDA(tmp.alloc(&deg, dg.n + 1ull));
+    PTW_CUDA(tmp.alloc(&off, dg.n + 1ull));
+    k_deg_by_index<<<grid_for(dg.n + 1ull), kThreads, 0, st>>>(dg.adj, dg.idx2int, dg.n, deg);
     PTW_CUDA(cub_call([&](void *t, size_t &b) {
         return cub::DeviceScan::ExclusiveSum(t, b, deg, off, (int64_t)dg.n + 1, st);
     }, st));
-    if (h_row_ptr) {
-        std::vector<uint32_t> tmp_off(dg.n + 1);
-        PTW_CUDA(cudaMemcpyAsync(tmp_off.data(), off, (dg.n + 1) * 4ull, cudaMemcpyDeviceToHost, st));
-        PTW_CUDA(cudaStreamSynchronize(st));
-        for (uint64_t i = 0; i <= dg.n; ++i) h_row_ptr[i] = tmp_off[i];
-    }
+    uint32_t *c = nullptr;
     if (h_col) {
-        uint32_t *c = nullptr;
         PTW_CUDA(tmp.alloc(&c, dg.m));
-        k_export<<<grid_for((uint64_t)dg.n * 32), kThreads, 0, st>>>(dg.adj, dg.col, dg.int2idx, off,
-                                                                    dg.n, c);
+        const uint64_t tiles = (dg.m + kExportTile - 1) / kExportTile;
+        k_export<<<grid_for(tiles * 32), kThreads, 0, st>>>(dg.adj, dg.col, dg.int2idx, off, dg.n, dg.m, c);
         PTW_CUDA(cudaGetLastError());
-        PTW_CUDA(cudaMemcpyAsync(h_col, c, dg.m * 4, cudaMemcpyDeviceToHost, st));
     }
+    if (h_row_ptr) {
+        unsigned long long *rows = nullptr;
+        PTW_CUDA(tmp.alloc(&rows, dg.n + 1ull));
+        k_widen<<<grid_for(dg.n + 1ull), kThreads, 0, st>>>(off, dg.n + 1ull, rows);
+        PTW_CUDA(cudaGetLastError());
+        PTW_CUDA(cudaMemcpyAsync(h_row_ptr, rows, (dg.n + 1ull) * 8, cudaMemcpyDeviceToHost, st));
+    }
+    if (h_col) PTW_CUDA(cudaMemcpyAsync(h_col, c, dg.m * 4, cudaMemcpyDeviceToHost, st));
     if (h_names) std::memcpy(h_names, g->h_names, (uint64_t)dg.n * 4);
     PTW_CUDA(cudaStreamSynchronize(st));
     return PTW_OK;

@@ -339,6 +339,8 @@ struct ptw_graph {
     int num_sms = 0;
     ptw_tune tune{};
     ptw_batch_tune btune{};  // zero fields: defaults (see ptw_batch_tune)
+    void *vertex_arrays = nullptr;  // one allocation: dg.adj .. dg.names, dg.rows, sc.counts, sc.ctrl
+    uint32_t *row_space = nullptr;  // room of the row table in it
     uint64_t device_bytes = 0;
     int ext_users = 0;  // open servers reading the extended columns (kept while > 0)
     ptw::AsyncSlot async[2];             // pipelined count walks in flight
@@ -412,6 +414,8 @@ int launch_lane_deepwalk(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_
 // pool hands memory back at each one), for count tables and the short-lived
 // buffers of every result compaction.  Freed with cudaFreeAsync.
 cudaError_t pooled_alloc_async(void **p, size_t bytes, cudaStream_t st);
+// Waits for st and unmaps what the pool holds unused above keep bytes.
+void release_pool_above(cudaStream_t st, uint64_t keep);
 // Hands the pools' cached memory back to the CUDA driver.
 void trim_pools();
 // cudaMalloc that, when the device is out of memory, trims the pools and
