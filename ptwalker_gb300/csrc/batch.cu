@@ -687,43 +687,51 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
     const uint64_t nch = tch[nt];
     if (nch >= (1ull << 31)) return fail(PTW_EINVAL, "count tables too large to compact in one call");
     DevBuf db(st);
-    unsigned long long *d_base, *d_cnt, *d_seg, *d_fill, *d_tch, *d_cc, *d_hc, *d_pos = nullptr, *d_hpos = nullptr;
-    uint32_t *d_cap, *d_hist = nullptr;
-    uint8_t *d_dense;
-    PTW_CUDA(db.alloc(&d_base, nt));
-    PTW_CUDA(db.alloc(&d_cap, nt));
-    PTW_CUDA(db.alloc(&d_dense, nt));
-    PTW_CUDA(db.alloc(&d_cnt, nt));
-    PTW_CUDA(db.alloc(&d_seg, nt + 1));
-    PTW_CUDA(db.alloc(&d_fill, nt));
-    PTW_CUDA(db.alloc(&d_tch, nt + 1));
+    // What the kernels read of the tables, in one upload: base, chunk starts,
+    // lengths, kinds; and what they add to, in one clear: cnt, fill, histograms.
+    unsigned long long *d_in, *d_zero, *d_sums, *d_cc, *d_hc, *d_pos = nullptr, *d_hpos = nullptr;
+    const uint64_t in_words = 2ull * nt + 1 + (4ull * nt + nt + 7) / 8;
+    std::vector<unsigned long long> in(in_words);
+    std::memcpy(in.data(), h_base, nt * 8ull);
+    std::memcpy(in.data() + nt, tch.data(), (nt + 1) * 8ull);
+    uint32_t *const in_cap = reinterpret_cast<uint32_t *>(in.data() + 2ull * nt + 1);
+    std::memcpy(in_cap, h_cap, nt * 4ull);
+    std::memcpy(in_cap + nt, dense_flags.data(), nt);
+    const uint64_t hist_words = k ? (uint64_t)nt * kCountBins / 2 : 0;
+    PTW_CUDA(db.alloc(&d_in, in_words));
+    PTW_CUDA(db.alloc(&d_zero, 2ull * nt + hist_words));
+    PTW_CUDA(db.alloc(&d_sums, (k ? 3ull : 1ull) * (nt + 1)));
+    unsigned long long *const d_base = d_in, *const d_tch = d_in + nt;
+    uint32_t *const d_cap = reinterpret_cast<uint32_t *>(d_in + 2ull * nt + 1);
+    uint8_t *const d_dense = reinterpret_cast<uint8_t *>(d_cap + nt);
+    unsigned long long *const d_cnt = d_zero, *const d_fill = d_zero + nt;
+    uint32_t *const d_hist = reinterpret_cast<uint32_t *>(d_zero + 2ull * nt);
+    unsigned long long *const d_seg = d_sums, *const d_sseg = d_sums + (nt + 1), *const d_kseg = d_sums + 2ull * (nt + 1);
+    uint32_t *d_thr = nullptr;
+    unsigned long long *d_sel = nullptr;
     const uint64_t npc = nch * 8;  // warp pieces: 8 per chunk
     PTW_CUDA(db.alloc(&d_cc, std::max<uint64_t>(npc, 1)));
     PTW_CUDA(db.alloc(&d_hc, std::max<uint64_t>(npc, 1)));
     const int sp_count = ph->begin(PhaseTimer::kCount, st);
-    PTW_CUDA(cudaMemcpyAsync(d_base, h_base, nt * 8ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_cap, h_cap, nt * 4ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_dense, dense_flags.data(), nt, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_tch, tch.data(), (nt + 1) * 8ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemsetAsync(d_cnt, 0, nt * 8ull, st));
-    PTW_CUDA(cudaMemsetAsync(d_fill, 0, nt * 8ull, st));
-    PTW_CUDA(cudaMemsetAsync(d_seg, 0, 8, st));
-    // Pass 1: occupied entries per chunk and per table (+ histograms for top-k).
+    PTW_CUDA(cudaMemcpyAsync(d_in, in.data(), in_words * 8, cudaMemcpyHostToDevice, st));
+    PTW_CUDA(cudaMemsetAsync(d_zero, 0, (2ull * nt + hist_words) * 8, st));
+    // Pass 1: occupied entries per chunk and per table (+ histograms for top-k,
+    // and from those the lowest bin that top-k keeps of each table).
     if (k) {
-        PTW_CUDA(db.alloc(&d_hist, (uint64_t)nt * kCountBins));
-        PTW_CUDA(cudaMemsetAsync(d_hist, 0, (uint64_t)nt * kCountBins * 4, st));
         if (nch)
             k_tabs_count<true><<<(unsigned)nch, 256, 0, st>>>(d_slots, d_base, d_cap, d_dense, d_tch, nt, d_cnt, d_cc,
                                                              d_hc, d_hist);
+        PTW_CUDA(db.alloc(&d_thr, nt));
+        PTW_CUDA(db.alloc(&d_sel, nt));
+        k_tabs_thresh<<<(nt + 7) / 8, 256, 0, st>>>(d_cnt, d_hist, nt, k, d_thr, d_sel);
     } else if (nch) {
         k_tabs_count<false><<<(unsigned)nch, 256, 0, st>>>(d_slots, d_base, d_cap, d_dense, d_tch, nt, d_cnt, d_cc,
                                                           d_hc, nullptr);
     }
+    k_table_sums<<<1, 1024, 0, st>>>(d_cnt, d_sel, nt, k, d_sums);
     PTW_CUDA(cudaGetLastError());
-    PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceScan::InclusiveSum(t, b, d_cnt, d_seg + 1, (int64_t)nt, st);
-    }, st));
-    PTW_CUDA(cudaMemcpyAsync(out->seg.data(), d_seg, (nt + 1) * 8ull, cudaMemcpyDeviceToHost, st));
+    std::vector<unsigned long long> sums((k ? 3ull : 1ull) * (nt + 1));
+    PTW_CUDA(cudaMemcpyAsync(sums.data(), d_sums, sums.size() * 8, cudaMemcpyDeviceToHost, st));
     if (!k && nch) {
         // output position of every dense piece, sort-input position of every hash piece
         PTW_CUDA(db.alloc(&d_pos, npc));
@@ -737,15 +745,17 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
     }
     ph->end(sp_count, st);
     PTW_CUDA(cudaStreamSynchronize(st));
+    std::copy(sums.begin(), sums.begin() + nt + 1, out->seg.begin());
     const uint64_t n_ent = out->seg[nt];
     // top-k: every table keeps its min(k, entries) largest counts
     std::vector<uint64_t> kseg;
-    uint64_t n_out = n_ent;
+    uint64_t n_out = n_ent, n_sel = 0, max_sel = 0;
     if (k && n_ent) {
-        kseg.assign(nt + 1, 0);
-        for (uint32_t i = 0; i < nt; ++i)
-            kseg[i + 1] = kseg[i] + std::min<uint64_t>(k, out->seg[i + 1] - out->seg[i]);
+        const unsigned long long *sseg = sums.data() + nt + 1;
+        kseg.assign(sums.begin() + 2ull * (nt + 1), sums.end());
         n_out = kseg[nt];
+        n_sel = sseg[nt];
+        for (uint32_t i = 0; i < nt; ++i) max_sel = std::max<uint64_t>(max_sel, sseg[i + 1] - sseg[i]);
     }
     out->n = n_out;
     if (n_ent) {
@@ -818,40 +828,28 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
             // as keys, so the radix sort sees about k entries per table
             // instead of all of them.  The sort orders each table by count
             // (ties by name) and the first k are kept.
-            uint32_t *d_thr;
-            unsigned long long *d_sel, *d_sseg;
             const int sp_place = ph->begin(PhaseTimer::kPlace, st);
-            PTW_CUDA(db.alloc(&d_thr, nt));
-            PTW_CUDA(db.alloc(&d_sel, nt));
-            PTW_CUDA(db.alloc(&d_sseg, nt + 1));
-            PTW_CUDA(cudaMemsetAsync(d_sseg, 0, 8, st));
-            k_tabs_thresh<<<(nt + 7) / 8, 256, 0, st>>>(d_cnt, d_hist, nt, k, d_thr, d_sel);
-            PTW_CUDA(cudaGetLastError());
-            PTW_CUDA(cub_call([&](void *t, size_t &b) {
-                return cub::DeviceScan::InclusiveSum(t, b, d_sel, d_sseg + 1, (int64_t)nt, st);
-            }, st));
-            unsigned long long n_sel = 0;
-            PTW_CUDA(cudaMemcpyAsync(&n_sel, d_sseg + nt, 8, cudaMemcpyDeviceToHost, st));
-            PTW_CUDA(cudaStreamSynchronize(st));
-            unsigned long long *e_key, *s_key;
-            uint32_t *e_cnt, *s_cnt;
-            PTW_CUDA(db.alloc(&e_key, n_sel));
-            PTW_CUDA(db.alloc(&s_key, n_sel));
-            PTW_CUDA(db.alloc(&e_cnt, n_sel));
-            PTW_CUDA(db.alloc(&s_cnt, n_sel));
+            unsigned long long *e_key, *s_key = nullptr;
+            uint32_t *e_cnt, *s_cnt = nullptr;
             // (table, ~count, name) in 64 bits: one sort, keys only
             const bool packed = q_bits + 32 + name_bits <= 64;
+            const bool by_table = packed && max_sel <= kTopkSort;
+            PTW_CUDA(db.alloc(&e_key, n_sel));
+            PTW_CUDA(db.alloc(&e_cnt, n_sel));
+            if (!by_table) {
+                PTW_CUDA(db.alloc(&s_key, n_sel));
+                PTW_CUDA(db.alloc(&s_cnt, n_sel));
+            }
             k_tabs_place<true><<<(unsigned)nch, 256, 0, st>>>(d_slots, d_base, d_cap, d_dense, d_tch, nt, 0ull,
                                                              nullptr, nullptr, d_thr, d_sseg, d_fill, g->dg.int2name,
                                                              g->dg.names, name_bits, packed, nullptr, nullptr,
                                                              nullptr, nullptr, e_key, e_cnt);
             PTW_CUDA(cudaGetLastError());
-            unsigned long long *d_kseg;
-            PTW_CUDA(db.alloc(&d_kseg, nt + 1));
             PTW_CUDA(alloc_out(&o_name, &o_cnt, n_out));
-            PTW_CUDA(cudaMemcpyAsync(d_kseg, kseg.data(), (nt + 1) * 8ull, cudaMemcpyHostToDevice, st));
             const unsigned sg = (unsigned)std::min<uint64_t>((n_sel + 255) / 256, (uint64_t)g->num_sms * 32);
-            if (packed) {
+            if (by_table) {
+                k_topk_sort<<<nt, kTopkBlock, 0, st>>>(e_key, name_bits, d_sseg, d_kseg, o_name, o_cnt);
+            } else if (packed) {
                 PTW_CUDA(cub_call([&](void *t, size_t &b) {
                     return cub::DeviceRadixSort::SortKeys(t, b, e_key, s_key, (int64_t)n_sel, 0,
                                                           q_bits + 32 + name_bits, st);

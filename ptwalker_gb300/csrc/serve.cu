@@ -221,6 +221,47 @@ int build_tick_graph(ptw_server *s)
     return PTW_OK;
 }
 
+constexpr uint32_t kClearSlots = 8192;  // slots per block: 64 KB
+
+__global__ void __launch_bounds__(256) k_clear_tables(ulonglong2 *arena, const ulonglong2 *pieces)
+{
+    const ulonglong2 p = pieces[blockIdx.x];  // {first slot, slots}, both even
+    for (uint32_t i = threadIdx.x; i < p.y / 2; i += 256) arena[p.x / 2 + i] = make_ulonglong2(0, 0);
+}
+
+// Zeroes the tables of newly admitted queries ({arena offset, slots}, even: the
+// arena hands out multiples of 256 slots): neighbours in one piece, several pieces in one
+// launch (300 queries at once: 300 clears of 2 us, or 30 us).
+int clear_tables(ptw_server *s, std::vector<std::pair<uint64_t, uint64_t>> &fresh)
+{
+    cudaStream_t st = s->g->stream;
+    std::sort(fresh.begin(), fresh.end());
+    size_t n = 0;
+    for (const auto &f : fresh) {
+        if (n && fresh[n - 1].first + fresh[n - 1].second == f.first) fresh[n - 1].second += f.second;
+        else fresh[n++] = f;
+    }
+    fresh.resize(n);
+    if (n <= 2) {
+        for (const auto &f : fresh) PTW_CUDA(cudaMemsetAsync(s->arena + f.first, 0, f.second * 8, st));
+        return PTW_OK;
+    }
+    std::vector<ulonglong2> pieces;
+    for (const auto &f : fresh)
+        for (uint64_t o = 0; o < f.second; o += kClearSlots)
+            pieces.push_back(make_ulonglong2(f.first + o, std::min<uint64_t>(kClearSlots, f.second - o)));
+    ulonglong2 *d = nullptr;
+    PTW_CUDA(pooled_alloc_async((void **)&d, pieces.size() * sizeof(ulonglong2), st));
+    cudaError_t e = cudaMemcpyAsync(d, pieces.data(), pieces.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice, st);
+    if (e == cudaSuccess) {
+        k_clear_tables<<<(unsigned)pieces.size(), 256, 0, st>>>(reinterpret_cast<ulonglong2 *>(s->arena), d);
+        e = cudaGetLastError();
+    }
+    cudaFreeAsync(d, st);
+    PTW_CUDA(e);
+    return PTW_OK;
+}
+
 // A free pinned block of at least `words` words: reuses one that no pending
 // result refers to, else allocates (blocks grow geometrically).
 std::shared_ptr<PinnedBlock> pinned_block(ptw_server *s, uint64_t words)
@@ -417,7 +458,9 @@ try {
     cudaStream_t st = s->g->stream;
     const uint32_t n = s->g->dg.n;
     const size_t done_before = s->done.size();
-    // 1. admission: FIFO while a slot and a table fit
+    // 1. admission: FIFO while a slot and a table fit.  Their tables are cleared
+    // together, neighbours in one piece (300 queries at once: 300 clears of 2 us).
+    std::vector<std::pair<uint64_t, uint64_t>> fresh;  // {arena offset, slots}
     while (!s->pending.empty() && s->active.size() < s->S) {
         Pending &pd = s->pending.front();
         const TableSize ts = pd.full ? dense_table(n)
@@ -430,7 +473,7 @@ try {
                 return fail(PTW_ENOMEM, "a query's count table is larger than the whole table arena");
             break;
         }
-        PTW_CUDA(cudaMemsetAsync(s->arena + off, 0, cap * 8, st));
+        fresh.emplace_back(off, (cap + 1) & ~1ull);  // (a dense table's n counters may end in half a slot pair)
         Active a;
         a.p = pd;
         a.cap = cap;
@@ -441,6 +484,7 @@ try {
         s->active.push_back(a);
         s->pending.pop_front();
     }
+    if (const int rc0 = clear_tables(s, fresh)) return rc0;
     uint32_t nd = 0;
     if (!s->active.empty()) {
         // 2. plan: a fair share of the tick's walkers per active query
