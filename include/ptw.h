@@ -462,6 +462,10 @@ int ptw_serve_take(ptw_server *s, uint32_t *h_names, uint32_t *h_counts);
  * device wrote them to, valid until that result is taken or the server is
  * closed. */
 int ptw_serve_view(const ptw_server *s, const uint32_t **names, const uint32_t **counts);
+/* Takes up to max completed results, oldest first: r, names and counts [max], *n
+ * how many.  The entries are views as above, valid until the next step. */
+int ptw_serve_take_many(ptw_server *s, uint32_t max, ptw_serve_result *r, const uint32_t **names,
+                        const uint32_t **counts, uint32_t *n);
 
 typedef struct ptw_serve_stats {
     uint64_t ticks;         /* steps that ran a tick */

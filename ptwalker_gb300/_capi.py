@@ -184,6 +184,7 @@ SIGNATURES = [
     ("ptw_serve_poll", ctypes.c_int, [_G, ctypes.POINTER(ServeResult)]),
     ("ptw_serve_take", ctypes.c_int, [_G, _u32p, _u32p]),
     ("ptw_serve_view", ctypes.c_int, [_G, ctypes.POINTER(_u32p), ctypes.POINTER(_u32p)]),
+    ("ptw_serve_take_many", ctypes.c_int, [_G, ctypes.c_uint32, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, _u32p]),
     ("ptw_serve_get_stats", ctypes.c_int, [_G, ctypes.POINTER(ServeStats)]),
     ("ptw_serve_clock", ctypes.c_double, [_G]),
     ("ptw_serve_close", None, [_G]),

@@ -631,6 +631,24 @@ try {
     return host_exception();
 }
 
+extern "C" int ptw_serve_take_many(ptw_server *s, uint32_t max, ptw_serve_result *r, const uint32_t **names,
+                                   const uint32_t **counts, uint32_t *n)
+try {
+    if (!s || !n || (max && (!r || !names || !counts))) return fail(PTW_EINVAL, "null argument");
+    uint32_t k = 0;
+    for (; k < max && !s->done.empty(); ++k) {
+        const Done &d = s->done.front();
+        r[k] = d.r;
+        names[k] = d.names;
+        counts[k] = d.counts;
+        s->done.pop_front();
+    }
+    *n = k;
+    return PTW_OK;
+} catch (...) {
+    return host_exception();
+}
+
 extern "C" int ptw_serve_get_stats(const ptw_server *s, ptw_serve_stats *out)
 try {
     if (!s || !out) return fail(PTW_EINVAL, "null argument");

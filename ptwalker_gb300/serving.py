@@ -15,6 +15,20 @@ from . import _capi as C
 from .batch import APPS
 
 
+# ptw_serve_result
+_RESULT = np.dtype([("query_id", np.uint32), ("source", np.uint32), ("budget", np.uint64), ("n_entries", np.uint64),
+                    ("submit_s", np.float64), ("admit_s", np.float64), ("done_s", np.float64)])
+
+
+def _words(address, n):
+    """n 32-bit words at address, read-only."""
+    if n == 0:
+        return np.empty(0, dtype=np.uint32)
+    a = np.frombuffer((ctypes.c_uint32 * n).from_address(address), dtype=np.uint32)
+    a.flags.writeable = False
+    return a
+
+
 class Server:
     def __init__(self, graph, sp=0.2, seed=0, app="visits", max_moves=0, table_bytes=0,
                  tick_walkers=0, max_active=0, use_graph=True, table_factor=0.0, top_k=0, staging_mb=0):
@@ -68,28 +82,33 @@ class Server:
         names and counts as read-only views of the server's page-locked
         staging (no copy), valid until the next step()."""
         out = []
-        r = C.ServeResult()
-        pn, pc = ctypes.POINTER(ctypes.c_uint32)(), ctypes.POINTER(ctypes.c_uint32)()
-        while self._lib.ptw_serve_poll(self._h, ctypes.byref(r)) == 1:
-            ne = int(r.n_entries)
-            if ne:
-                # the entries sit in the page-locked block the device wrote them to
-                C.check(self._lib.ptw_serve_view(self._h, ctypes.byref(pn), ctypes.byref(pc)))
-                names = np.ctypeslib.as_array(pn, shape=(ne,))
-                counts = np.ctypeslib.as_array(pc, shape=(ne,))
-                if copy:
-                    names, counts = names.copy(), counts.copy()
-                else:
-                    names.flags.writeable = False
-                    counts.flags.writeable = False
-            else:
-                names = np.empty(0, dtype=np.uint32)
-                counts = np.empty(0, dtype=np.uint32)
-            C.check(self._lib.ptw_serve_take(self._h, None, None))
-            out.append(dict(query_id=int(r.query_id), source=int(r.source), budget=int(r.budget),
-                            names=names, counts=counts, submit_s=float(r.submit_s),
-                            admit_s=float(r.admit_s), done_s=float(r.done_s)))
-        return out
+        cap, n = 512, ctypes.c_uint32()
+        rows = np.empty(cap, dtype=_RESULT)
+        ptrs = np.empty((2, cap), dtype=np.uint64)
+        while True:
+            C.check(self._lib.ptw_serve_take_many(self._h, cap, rows.ctypes.data, ptrs[0].ctypes.data,
+                                                  ptrs[1].ctypes.data, ctypes.byref(n)))
+            k = int(n.value)
+            res, pn, pc = rows[:k].tolist(), ptrs[0, :k].tolist(), ptrs[1, :k].tolist()
+            i = 0
+            while i < k:
+                # results of one step lie one after the other in the page-locked
+                # block that the device wrote them to
+                j, total = i, 0
+                while j < k and pn[j] - pn[i] == pc[j] - pc[i] == 4 * total:
+                    total += res[j][3]
+                    j += 1
+                names, counts = _words(pn[i], total), _words(pc[i], total)
+                a = 0
+                for q, source, budget, ne, t_submit, t_admit, t_done in res[i:j]:
+                    nm, ct = names[a:a + ne], counts[a:a + ne]
+                    out.append(dict(query_id=q, source=source, budget=budget, names=nm.copy() if copy else nm,
+                                    counts=ct.copy() if copy else ct, submit_s=t_submit, admit_s=t_admit,
+                                    done_s=t_done))
+                    a += ne
+                i = j
+            if k < cap:
+                return out
 
     def stats(self):
         """Counters since open (ptw_serve_stats) as a dict."""
