@@ -14,16 +14,22 @@
 // A training step is 3.6 MFLOP at batch 256: its time is latency.  As five
 // launches per step with one thread per sample or parameter, each waiting on
 // its own loads, and a copy of the loss per step, a step took 155 us.  Now one
-// cluster of 16 CTAs runs all steps of an epoch in one launch (k_mlp_steps):
+// cluster of 16 CTAs runs the steps of several epochs in one launch (k_mlp_steps):
 // samples are spread over the CTAs in tiles of 16 (a thread makes four of the 64
 // sums of a layer for two samples, weights in shared memory), then every
 // CTA sums the gradients of a sixteenth of the parameters over the whole
 // batch, with the optimiser's state of a parameter in its thread's registers.
 // The two exchanges per step (per-sample terms, updated parameters) go through
 // L2 between cluster barriers, copied to shared memory asynchronously; the
-// next step's samples are read ahead.  A step takes 7 us at batch 16 and 11 us
-// at 256; training 2,000 samples for 30 epochs of batch 256 went from 37.4 to
-// 3.3 ms, model creation and prediction included.
+// next step's samples are read ahead.  Through distributed shared memory both
+// were slower: its stores move 14 bytes per cycle and SM (terms 3,900 cycles
+// against 2,500, parameters 3,000 against 900).
+// Of the 17,800 cycles of a step at batch 256 the exchanges take 7,500, the layers
+// 4,400 and the sums over the samples 3,600 -- both bound by their shared memory
+// reads, 4 cycles per 16-byte read of a warp however many of its threads read the
+// same --, the update 460.  A step takes 6 us at batch 16 and 9 us at 256;
+// training 2,000 samples for 30 epochs of batch 256 went from 37.4 to 2.5 ms,
+// model creation and prediction included.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -53,10 +59,11 @@ struct Norm {
 constexpr int kTile = 16;        // samples per tile
 constexpr int kCluster = 16;     // CTAs of k_mlp_steps
 constexpr int kTileThreads = 128;  // per tile: two samples and four units each
-constexpr int kW2Threads = 256;    // one per W2 gradient of a CTA
-constexpr int kStepThreads = kW2Threads + 64;  // and two warps for its other gradients
+constexpr int kW2 = 256;           // W2 parameters of a CTA, and its others:
+constexpr int kOthers = 4 * IN + 13;
+constexpr int kStepThreads = kW2 + 64;  // one per parameter
 constexpr int kRow = H + 4;      // row stride of the tile's per-sample arrays (16-byte rows, no bank conflicts)
-constexpr int kChunk = 256;      // samples whose terms are staged at a time
+constexpr int kChunk = kCluster * kTile;  // samples that the cluster takes at a time
 constexpr int kChunkRow = kChunk + 4;
 
 // One tile of samples.
@@ -69,10 +76,11 @@ struct Tile {
     float y[kTile];
 };
 
-// Terms of the batch's samples in device memory, exchanged between the CTAs:
-// rows of n_pad values (the batch rounded up to whole tiles), one per unit.
+// Terms of a tile's samples, one row per unit: what the gradients add up.
 constexpr int TA1 = 0, TD2 = H, TD1 = 2 * H, TA2 = 3 * H, TX = 4 * H, TE = TX + IN, kTermRows = TE + 1;
-// Rows that a CTA stages: 16 of a1 and of d2 for its W2 block; 4 of d1, d2 and
+constexpr int kTermRow = kTile + 1;  // (odd: a tile's threads write columns)
+constexpr int kTermsWords = (kTermRows * kTermRow + 3) & ~3;
+// Rows that a CTA needs of every tile: 16 of a1 and of d2 for its W2 block; 4 of d1, d2 and
 // a2, all of x, and e for its other parameters.
 constexpr int kStageRows = 16 + 16 + 4 + 4 + 4 + IN + 1;
 
@@ -89,7 +97,7 @@ constexpr int kParamsPadded = (PTW_MLP_NPARAMS + 3) & ~3;  // 16-byte copies
 template <int N>
 __device__ __forceinline__ void dot24(float (&acc)[2][4], const float *v0, const float *v1, const float *m, int col)
 {
-#pragma unroll 4
+#pragma unroll
     for (int k = 0; k < N; k += 4) {
         const float4 x0 = ld4(v0 + k), x1 = ld4(v1 + k);
         const float xs[2][4] = {{x0.x, x0.y, x0.z, x0.w}, {x1.x, x1.y, x1.z, x1.w}};
@@ -107,6 +115,23 @@ __device__ __forceinline__ void dot24(float (&acc)[2][4], const float *v0, const
     }
 }
 
+__device__ __forceinline__ void st4(float *p, const float (&v)[4])
+{
+    *reinterpret_cast<float4 *>(p) = make_float4(v[0], v[1], v[2], v[3]);
+}
+
+__device__ __forceinline__ void load_bias(float (&z)[2][4], const float *b, int col)
+{
+    const float4 x = ld4(b + 4 * col);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        z[q][0] = x.x;
+        z[q][1] = x.y;
+        z[q][2] = x.z;
+        z[q][3] = x.w;
+    }
+}
+
 // Forward pass of a tile whose inputs are in t.x: a1, z2 and y, with the
 // parameters w.  Called by the whole block (threads past kTileThreads only
 // synchronise).
@@ -116,19 +141,19 @@ __device__ __forceinline__ void tile_forward(Tile &t, const float *w)
     const bool on = threadIdx.x < kTileThreads;
     float z[2][4];
     if (on) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) z[q / 4][q % 4] = w[OB1 + 4 * c + q % 4];
+        load_bias(z, w + OB1, c);
         dot24<IN>(z, t.x[s], t.x[s + 1], w + OW1, c);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) t.a1[s + q / 4][4 * c + q % 4] = z[q / 4][q % 4] > 0.f ? z[q / 4][q % 4] : 0.f;
+        for (int q = 0; q < 8; ++q) z[q / 4][q % 4] = z[q / 4][q % 4] > 0.f ? z[q / 4][q % 4] : 0.f;
+        st4(t.a1[s] + 4 * c, z[0]);
+        st4(t.a1[s + 1] + 4 * c, z[1]);
     }
     __syncthreads();
     if (on) {
-#pragma unroll
-        for (int q = 0; q < 8; ++q) z[q / 4][q % 4] = w[OB2 + 4 * c + q % 4];
+        load_bias(z, w + OB2, c);
         dot24<H>(z, t.a1[s], t.a1[s + 1], w + OW2, c);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) t.z2[s + q / 4][4 * c + q % 4] = z[q / 4][q % 4];
+        st4(t.z2[s] + 4 * c, z[0]);
+        st4(t.z2[s + 1] + 4 * c, z[1]);
     }
     __syncthreads();
     if (threadIdx.x < kTile) {
@@ -177,47 +202,37 @@ __device__ __forceinline__ void adam(float &P, float &M, float &V, float g, floa
     P -= lr * (m / c1) / (sqrtf(v / c2) + eps);
 }
 
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_arrive()
+{
+    __syncwarp();
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
 struct StepArgs {
     const float *x, *t;        // all samples
-    const uint32_t *idx;       // sample of every position (null: the position itself)
+    const uint32_t *idx;       // sample of every position of every epoch (null: the position itself)
     const float *corr;         // Adam's bias corrections {c1, c2} per step
     float *P, *PT, *M, *V, *G; // parameters, W2 transposed, Adam's state, gradient
+    float *terms;              // of a chunk's tiles, [2][kCluster][kTermRows][kTile]
     float *loss_terms;         // squared error of every position
-    float *terms;              // [kTermRows][n_pad]
-    uint32_t n_pad;
-    uint32_t n, batch;         // positions, positions per step
+    uint32_t n, batch, epochs; // positions of an epoch, positions per step
     float lr, b1, b2, eps;
 };
 
-// A thread's share of the gradient.  The CTA of rank r has W2 rows
-// 16 (r / 4) .. + 15, columns 16 (r % 4) .. + 15 (one per thread), and, by two
-// warps of their own, columns 4 r .. 4 r + 3 of W1, b1, b2 and w3, and b3 (rank 0).
-struct Share {
-    int p;    // parameter of this thread, -1 = none
-    int u, v; // staged rows: its gradient is the sum over the samples of u[b] * v[b], v < 0: of u[b]
-    bool gate; // only of the samples with v[b] > 0 (v is an activation)
-};
-
-__device__ __forceinline__ Share share_of(int rank, int tid)
+// Parameter of a thread, -1 = none.  The CTA of rank r has W2 rows
+// 16 (r / 4) .. + 15, columns 16 (r % 4) .. + 15, and columns 4 r .. 4 r + 3 of W1,
+// b1, b2 and w3, and b3 (rank 0).
+__device__ __forceinline__ int param_of(int rank, int tid)
 {
-    constexpr int SA1 = 0, SD2 = 16, SD1 = 32, SE2 = 36, SA2 = 40, SX = 44, SE = SX + IN;
-    if (tid < kW2Threads) {
-        const int i = tid / 16, j = tid % 16;
-        return Share{OW2 + (16 * (rank / 4) + i) * H + 16 * (rank % 4) + j, SD2 + j, SA1 + i, true};
-    }
-    const int q = tid - kW2Threads, c = q % 4, col = 4 * rank + c;
-    if (q < 4 * IN) return Share{OW1 + (q / 4) * H + col, SD1 + c, SX + q / 4, false};
-    if (q < 4 * IN + 4) return Share{OB1 + col, SD1 + c, -1, false};
-    if (q < 4 * IN + 8) return Share{OB2 + col, SE2 + c, -1, false};
-    if (q < 4 * IN + 12) return Share{OW3 + col, SE, SA2 + c, true};
-    if (q == 4 * IN + 12 && rank == 0) return Share{OB3, SE, -1, false};
-    return Share{-1, 0, -1, false};
+    if (tid < kW2) return OW2 + (16 * (rank / 4) + tid / 16) * H + 16 * (rank % 4) + tid % 16;
+    const int q = tid - kW2, col = 4 * rank + q % 4;
+    if (q < 4 * IN) return OW1 + (q / 4) * H + col;
+    if (q < 4 * IN + 12) return (q < 4 * IN + 4 ? OB1 : q < 4 * IN + 8 ? OB2 : OW3) + col;
+    return q == 4 * IN + 12 && rank == 0 ? OB3 : -1;
 }
 
-// The terms row that staged row r holds.
+// The terms row that row r of the CTA of rank `rank` holds.
 __device__ __forceinline__ int staged_row(int rank, int r)
 {
     if (r < 16) return TA1 + 16 * (rank / 4) + r;
@@ -228,170 +243,311 @@ __device__ __forceinline__ int staged_row(int rank, int r)
     return TX + r - 44;  // x, then e
 }
 
+// acc = v * u + acc where v > 0, as a predicated instruction (a branch per sample
+// took 26 cycles of it).
+__device__ __forceinline__ void fma_if_positive(float &acc, float v, float u)
+{
+    asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, 0f00000000;\n\t@p fma.rn.f32 %0, %1, %2, %0;\n\t}"
+        : "+f"(acc)
+        : "f"(v), "f"(u));
+}
+
+// acc[i][j] += the sums over n samples (a multiple of 16) of v[i] * u[j], in order;
+// GATE: of those with v[i] > 0.  Two rows of each: four chains of additions keep a
+// scheduler busy, with one read per addition.  The next samples are read while
+// these are added.
+template <bool GATE>
+__device__ __forceinline__ void sum_quad(float (&acc)[2][2], const float *u, const float *v, uint32_t n)
+{
+    constexpr int kFar = 8 * kChunkRow;  // the second row of each
+    __align__(16) float x[4][8], y[4][8];
+    auto load = [&](float (&f)[4][8], uint32_t k) {
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            *reinterpret_cast<float4 *>(f[0] + h) = ld4(u + k + h);
+            *reinterpret_cast<float4 *>(f[1] + h) = ld4(u + kFar + k + h);
+            *reinterpret_cast<float4 *>(f[2] + h) = ld4(v + k + h);
+            *reinterpret_cast<float4 *>(f[3] + h) = ld4(v + kFar + k + h);
+        }
+    };
+    auto add = [&](const float (&f)[4][8]) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (GATE) fma_if_positive(acc[i][j], f[2 + i][c], f[j][c]);
+                    else acc[i][j] = fmaf(f[2 + i][c], f[j][c], acc[i][j]);
+                }
+    };
+    load(x, 0);
+    for (uint32_t k = 0; k < n; k += 16) {
+        load(y, k + 8);
+        add(x);
+        if (k + 16 < n) load(x, k + 16);
+        add(y);
+    }
+}
+
+// The same for one pair of rows.
+template <bool GATE>
+__device__ __forceinline__ void sum_one(float &acc, const float *u, const float *v, uint32_t n)
+{
+    __align__(16) float x[2][8], y[2][8];
+    auto load = [&](float (&f)[2][8], uint32_t k) {
+#pragma unroll
+        for (int h = 0; h < 8; h += 4) {
+            *reinterpret_cast<float4 *>(f[0] + h) = ld4(u + k + h);
+            *reinterpret_cast<float4 *>(f[1] + h) = ld4(v + k + h);
+        }
+    };
+    auto add = [&](const float (&f)[2][8]) {
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+            if (GATE) fma_if_positive(acc, f[1][c], f[0][c]);
+            else acc = fmaf(f[1][c], f[0][c], acc);
+        }
+    };
+    load(x, 0);
+    for (uint32_t k = 0; k < n; k += 16) {
+        load(y, k + 8);
+        add(x);
+        if (k + 16 < n) load(x, k + 16);
+        add(y);
+    }
+}
+
 // TRAIN: one Adam step per batch of positions; otherwise the gradient of the
 // first batch, into G.
 template <bool TRAIN>
-__global__ void __launch_bounds__(kStepThreads) k_mlp_steps(const StepArgs a, const __grid_constant__ Norm nm)
+__global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a, const __grid_constant__ Norm nm)
 {
     extern __shared__ __align__(16) float smem[];
     float *w = smem;                     // parameters
     float *w2t = w + kParamsPadded;      // W2 transposed
-    Tile &t = *reinterpret_cast<Tile *>(w2t + H * H);
-    float *stage = w2t + H * H + sizeof(Tile) / 4;
+    float *terms = w2t + H * H;          // of this CTA's tile, [kTermRows][kTermRow]
+    float *stage = terms + kTermsWords;  // of the cluster's tiles, what this CTA adds up
+    float *ones = stage + kStageRows * kChunkRow;  // a row of ones
+    float *grad = ones + kChunkRow;      // sums, one per thread
+    Tile &t = *reinterpret_cast<Tile *>(grad + kStepThreads);
     const int rank = blockIdx.x;  // one cluster
     const int tid = threadIdx.x;
     const uint64_t pol = l2_policy(0);
+    for (int i = tid; i < kChunkRow; i += kStepThreads) ones[i] = 1.f;
 
-    const Share sh = share_of(rank, tid);
+    // This thread's parameter, with its optimiser state.
+    const int param = param_of(rank, tid);
     float pP = 0.f, pM = 0.f, pV = 0.f;
-    if (TRAIN && sh.p >= 0) {
-        pP = a.P[sh.p];
-        pM = a.M[sh.p];
-        pV = a.V[sh.p];
+    if (TRAIN && param >= 0) {
+        pP = a.P[param];
+        pM = a.M[param];
+        pV = a.V[param];
     }
-    const float *us = stage + sh.u * kChunkRow, *vs = stage + (sh.v < 0 ? 0 : sh.v) * kChunkRow;
 
-    // Inputs and target of this thread in the CTA's first tile of a step
-    // (sample tid / IN, input tid % IN; sample tid), read ahead of the step.
+    // What it copies of a tile's terms: 16 bytes of row r for r = tid / 64, + 5, ...
+    // of tile tid % 64 / 4.
+    constexpr int kRowStep = kStepThreads / (4 * kCluster), kRowRounds = (kStageRows + kRowStep - 1) / kRowStep;
+    const int c_row = tid / (4 * kCluster), c_tile = tid / 4 % kCluster, c_part = 4 * (tid % 4);
+    uint16_t c_from[kRowRounds];
+#pragma unroll
+    for (int i = 0; i < kRowRounds; ++i) {
+        const int r = c_row + i * kRowStep;
+        c_from[i] = (uint16_t)(r < kStageRows ? staged_row(rank, r) : 0);
+    }
+
+    // What this thread adds up: threads 0 .. 63 W2 rows i, i + 8 and columns j, j + 8,
+    // threads 64 .. 95 W1, threads 96 .. 108 b1, b2, w3 and b3 (sums of d1, d2, a2 e
+    // and e; products with 1 where there is one factor).
+    constexpr int SA1 = 0, SD2 = 16, SD1 = 32, SE2 = 36, SA2 = 40, SX = 44, SE = SX + IN;
+    int ru = 0, rv = -1;  // staged rows (-1: ones)
+    if (tid < 64) {
+        ru = SD2 + tid % 8;
+        rv = SA1 + tid / 8;
+    } else if (tid < 96) {
+        ru = SD1 + tid % 4;
+        rv = SX + (tid - 64) / 4;
+    } else if (tid < 96 + 13) {
+        const int q = (tid - 96) / 4, c = tid % 4;
+        ru = q == 0 ? SD1 + c : q == 1 ? SE2 + c : SE;
+        rv = q == 2 ? SA2 + c : -1;
+    }
+
+    // Input and target of this thread in the CTA's tile of a chunk (sample
+    // tid / IN, input tid % IN; sample tid), read a chunk ahead.
     const int xs = tid / IN, xk = tid % IN;
+    const float mu = nm.mu[xk], sd = nm.sd[xk];
     uint32_t ix = 0, it = 0;  // their samples
     float xv = 0.f, tv = 0.f;
-    auto ahead_index = [&](uint32_t b0) {
-        const uint32_t bx = b0 + rank * kTile + xs, bt = b0 + rank * kTile + tid;
-        if (tid < kTileThreads && bx < a.n) ix = a.idx ? a.idx[bx] : bx;
-        if (tid < kTile && bt < a.n) it = a.idx ? a.idx[bt] : bt;
+    // position b of epoch ep (the first of the next epoch behind the last)
+    auto ahead_index = [&](uint32_t ep, uint32_t b) {
+        if (b >= a.n) {
+            if (!TRAIN || ++ep >= a.epochs) return;
+            b = 0;
+        }
+        const uint64_t e0 = (uint64_t)ep * a.n;
+        const uint32_t bx = b + rank * kTile + xs, bt = b + rank * kTile + tid;
+        if (tid < kTileThreads && bx < a.n) ix = a.idx ? a.idx[e0 + bx] : bx;
+        if (tid < kTile && bt < a.n) it = a.idx ? a.idx[e0 + bt] : bt;
     };
     auto ahead_values = [&] {
         if (tid < kTileThreads) xv = a.x[(uint64_t)ix * IN + xk];
         if (tid < kTile) tv = a.t[it];
     };
-    ahead_index(0);
+    ahead_index(0, 0);
     ahead_values();
 
-    const uint32_t np = a.n_pad;
-    for (uint32_t b0 = 0, step = 0; b0 < a.n; b0 += a.batch, ++step) {
+    uint32_t flip = 0;
+    for (uint32_t ep = 0, step = 0; ep < a.epochs; ++ep)
+    for (uint32_t b0 = 0; b0 < a.n; b0 += a.batch, ++step) {
         const uint32_t B = a.n - b0 < a.batch ? a.n - b0 : a.batch;
-        const uint32_t tiles = (B + kTile - 1) / kTile;
-        // W2 transposed is not needed before the backward pass
-        copy_async(w, a.P, kParamsPadded, pol);
-        asm volatile("cp.async.commit_group;" ::: "memory");
-        copy_async(w2t, a.PT, H * H, pol);
-        asm volatile("cp.async.commit_group;" ::: "memory");
         float c1 = 0.f, c2 = 0.f;
         if (TRAIN) {
             c1 = a.corr[2 * step];
             c2 = a.corr[2 * step + 1];
         }
+        // W2 transposed is not needed before the backward pass
+        copy_async(w, a.P, kParamsPadded, pol);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        copy_async(w2t, a.PT, H * H, pol);
+        asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
-        // ---- forward and backward of this CTA's tiles ----------------------------
-        for (uint32_t tl = rank; tl < tiles; tl += kCluster) {
-            const uint32_t t0 = tl * kTile;  // first sample within the batch
-            if (tl != (uint32_t)rank) {
-                const uint32_t bx = b0 + t0 + xs, bt = b0 + t0 + tid;
-                if (tid < kTileThreads && bx < a.n) xv = a.x[(uint64_t)(a.idx ? a.idx[bx] : bx) * IN + xk];
-                if (tid < kTile && bt < a.n) tv = a.t[a.idx ? a.idx[bt] : bt];
-                __syncthreads();  // the tile before is done with t
-            }
-            if (tid < kTileThreads) t.x[xs][xk] = t0 + xs < B ? (xv - nm.mu[xk]) / nm.sd[xk] : 0.f;
-            __syncthreads();
-            tile_forward(t, w);
-            if (tid < kTile) {
-                const uint32_t b = t0 + tid;
-                float eb = 0.f;
-                if (b < B) {
-                    const float tn = (tv - nm.tmu) / nm.tsd;
-                    const float d = t.y[tid] - tn;
-                    if (a.loss_terms) a.loss_terms[b0 + b] = d * d;
-                    eb = 2.f * d / (float)B;
+        float acc[2][2] = {};
+        for (uint32_t k0 = 0; k0 < B; k0 += kChunk, flip ^= 1) {
+            float *const all = a.terms + (uint64_t)flip * (kCluster * kTermRows * kTile);
+            const uint32_t n = B - k0 < kChunk ? (B - k0 + kTile - 1) / kTile * kTile : kChunk;
+            const uint32_t t0 = k0 + rank * kTile;  // first sample of this CTA's tile within the batch
+            // ---- forward and backward of this CTA's tile ------------------------------
+            if (t0 < B) {
+                if (tid < kTileThreads) t.x[xs][xk] = t0 + xs < B ? (xv - mu) / sd : 0.f;
+                __syncthreads();
+                tile_forward(t, w);
+                if (tid < kTile) {
+                    const uint32_t b = t0 + tid;
+                    float eb = 0.f;
+                    if (b < B) {
+                        const float tn = (tv - nm.tmu) / nm.tsd;
+                        const float d = t.y[tid] - tn;
+                        if (a.loss_terms) a.loss_terms[(uint64_t)ep * a.n + b0 + b] = d * d;
+                        eb = 2.f * d / (float)B;
+                    }
+                    t.e[tid] = eb;
+                    terms[TE * kTermRow + tid] = eb;
                 }
-                t.e[tid] = eb;
-                __stcg(a.terms + (uint64_t)TE * np + t0 + tid, eb);
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+                __syncthreads();
+                const int s = tid / 16 * 2, c = tid % 16;
+                if (tid < kTileThreads) {
+                    const float4 w3 = ld4(w + OW3 + 4 * c);
+#pragma unroll
+                    for (int r = s; r < s + 2; ++r) {
+                        const float4 z2 = ld4(t.z2[r] + 4 * c);
+                        const float e = t.e[r];
+                        const float g[4] = {z2.x > 0.f ? e * w3.x : 0.f, z2.y > 0.f ? e * w3.y : 0.f,
+                                            z2.z > 0.f ? e * w3.z : 0.f, z2.w > 0.f ? e * w3.w : 0.f};
+                        st4(t.g2[r] + 4 * c, g);
+                    }
+                }
+                __syncthreads();
+                if (tid < kTileThreads) {
+                    float g[2][4] = {};
+                    dot24<H>(g, t.g2[s], t.g2[s + 1], w2t, c);
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        const int r = s + h;
+                        const bool live = t0 + r < B;  // all terms of the samples past the batch are 0
+                        const float4 a1 = ld4(t.a1[r] + 4 * c), z2 = ld4(t.z2[r] + 4 * c), g2 = ld4(t.g2[r] + 4 * c);
+                        const float va[4] = {a1.x, a1.y, a1.z, a1.w}, vz[4] = {z2.x, z2.y, z2.z, z2.w},
+                                    vg[4] = {g2.x, g2.y, g2.z, g2.w};
+                        float *o = terms + 4 * c * kTermRow + r;
+#pragma unroll
+                        for (int q = 0; q < 4; ++q, o += kTermRow) {
+                            o[TA1 * kTermRow] = live ? va[q] : 0.f;
+                            o[TD1 * kTermRow] = live && va[q] > 0.f ? g[h][q] : 0.f;
+                            o[TD2 * kTermRow] = live ? vg[q] : 0.f;
+                            o[TA2 * kTermRow] = live && vz[q] > 0.f ? vz[q] : 0.f;
+                        }
+                    }
+                    terms[(TX + xk) * kTermRow + xs] = t.x[xs][xk];
+                }
+                __syncthreads();
+                for (int i = tid; i < kTermRows * kTile / 4; i += kStepThreads) {
+                    const float *f = terms + i / 4 * kTermRow + 4 * (i % 4);
+                    __stcg(reinterpret_cast<float4 *>(all + (uint64_t)rank * (kTermRows * kTile)) + i,
+                           make_float4(f[0], f[1], f[2], f[3]));
+                }
             }
             asm volatile("cp.async.wait_group 0;" ::: "memory");
-            __syncthreads();
-            const int s = tid / 16 * 2, c = tid % 16;
-            if (tid < kTileThreads) {
+            cluster_arrive();
+            ahead_index(ep, k0 + kChunk < B ? b0 + k0 + kChunk : b0 + a.batch);
+            cluster_wait();
+            ahead_values();
+            // ---- gradient of this CTA's share, samples in order -----------------------
+            // (the next chunk's terms go to the other half of a.terms; whoever writes to
+            // this one again has passed the barrier after this copy in every CTA)
+            if (c_tile * kTile < n) {
+                const float *from = all + c_tile * (kTermRows * kTile) + c_part;
+                float *to = stage + c_row * kChunkRow + c_tile * kTile + c_part;
 #pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int r = s + q / 4, j = 4 * c + q % 4;
-                    t.g2[r][j] = t.z2[r][j] > 0.f ? t.e[r] * w[OW3 + j] : 0.f;
-                }
+                for (int i = 0; i < kRowRounds; ++i)
+                    if (c_row + i * kRowStep < kStageRows)
+                        cp_async16(to + i * (kRowStep * kChunkRow), from + c_from[i] * kTile, pol);
             }
-            __syncthreads();
-            if (tid < kTileThreads) {
-                float g[2][4] = {};
-                dot24<H>(g, t.g2[s], t.g2[s + 1], w2t, c);
-#pragma unroll
-                for (int q = 0; q < 8; ++q) {
-                    const int r = s + q / 4, i = 4 * c + q % 4;
-                    const bool live = t0 + r < B;  // all terms of the samples past the batch are 0
-                    const float a1 = t.a1[r][i], z2 = t.z2[r][i];
-                    float *o = a.terms + (uint64_t)i * np + t0 + r;
-                    __stcg(o + (uint64_t)TA1 * np, live ? a1 : 0.f);
-                    __stcg(o + (uint64_t)TD1 * np, live && a1 > 0.f ? g[q / 4][q % 4] : 0.f);
-                    __stcg(o + (uint64_t)TD2 * np, live ? t.g2[r][i] : 0.f);
-                    __stcg(o + (uint64_t)TA2 * np, live && z2 > 0.f ? z2 : 0.f);
-                }
-                __stcg(a.terms + (uint64_t)(TX + xk) * np + t0 + xs, t.x[xs][xk]);
-            }
-        }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        cluster_arrive();
-        if (TRAIN) ahead_index(b0 + a.batch);
-        cluster_wait();
-        // ---- gradient of this CTA's share, samples in order -----------------------
-        float acc = 0.f;
-        for (uint32_t k0 = 0; k0 < tiles * kTile; k0 += kChunk) {
-            const uint32_t left = tiles * kTile - k0, n = left < kChunk ? left : kChunk;
-            if (k0) __syncthreads();  // the chunk before is summed
-            for (uint32_t v = tid; v < kStageRows * (n / 4); v += blockDim.x) {
-                const uint32_t r = v / (n / 4), q = 4 * (v - r * (n / 4));
-                cp_async16(stage + r * kChunkRow + q, a.terms + (uint64_t)staged_row(rank, r) * np + k0 + q, pol);
-            }
-            if (TRAIN && !k0) ahead_values();
             cp_async_wait_all();
             __syncthreads();
-            if (sh.p >= 0) {
-                if (sh.v >= 0) {
-#pragma unroll 4
-                    for (uint32_t k = 0; k < n; k += 4) {
-                        const float4 u = ld4(us + k), v = ld4(vs + k);
-                        if (!sh.gate || v.x > 0.f) acc = fmaf(v.x, u.x, acc);
-                        if (!sh.gate || v.y > 0.f) acc = fmaf(v.y, u.y, acc);
-                        if (!sh.gate || v.z > 0.f) acc = fmaf(v.z, u.z, acc);
-                        if (!sh.gate || v.w > 0.f) acc = fmaf(v.w, u.w, acc);
-                    }
-                } else {
-#pragma unroll 4
-                    for (uint32_t k = 0; k < n; k += 4) {
-                        const float4 u = ld4(us + k);
-                        acc += u.x;
-                        acc += u.y;
-                        acc += u.z;
-                        acc += u.w;
-                    }
+            const float *u = stage + ru * kChunkRow, *v = rv < 0 ? ones : stage + rv * kChunkRow;
+            if (tid < 64) {
+                // A sample whose a1 is 0 adds 0 times d2, which only differs from
+                // leaving it out where d2 is not finite: then the sum is NaN and is
+                // made again with the others only (a test per sample doubles it).
+                float q[2][2] = {{acc[0][0], acc[0][1]}, {acc[1][0], acc[1][1]}};
+                sum_quad<false>(q, u, v, n);
+                if (isnan(q[0][0]) || isnan(q[0][1]) || isnan(q[1][0]) || isnan(q[1][1])) sum_quad<true>(acc, u, v, n);
+                else {
+                    acc[0][0] = q[0][0];
+                    acc[0][1] = q[0][1];
+                    acc[1][0] = q[1][0];
+                    acc[1][1] = q[1][1];
                 }
+            } else if (tid < 96) {
+                sum_one<false>(acc[0][0], u, v, n);
+            } else if (tid < 96 + 13) {
+                float q = acc[0][0];
+                sum_one<false>(q, u, v, n);
+                if (isnan(q)) sum_one<true>(acc[0][0], u, v, n);
+                else acc[0][0] = q;
             }
         }
-        if (!TRAIN) {
-            if (sh.p >= 0) a.G[sh.p] = acc;
-            break;
+        if (tid < 64) {
+            float *g = grad + tid / 8 * 16 + tid % 8;
+            g[0] = acc[0][0];
+            g[8] = acc[0][1];
+            g[8 * 16] = acc[1][0];
+            g[8 * 16 + 8] = acc[1][1];
+        } else if (tid < 96 + 13) {
+            grad[kW2 + tid - 64] = acc[0][0];
         }
-        if (sh.p >= 0) {
-            adam(pP, pM, pV, acc, a.lr, a.b1, a.b2, a.eps, c1, c2);
-            __stcg(a.P + sh.p, pP);
-            if (sh.p >= OW2 && sh.p < OB2) __stcg(a.PT + ((sh.p - OW2) % H) * H + (sh.p - OW2) / H, pP);
+        __syncthreads();
+        if (!TRAIN) {
+            if (param >= 0) a.G[param] = grad[tid];
+            return;
+        }
+        if (param >= 0) {
+            adam(pP, pM, pV, grad[tid], a.lr, a.b1, a.b2, a.eps, c1, c2);
+            __stcg(a.P + param, pP);
+            if (tid < kW2) __stcg(a.PT + (param - OW2) % H * H + (param - OW2) / H, pP);
         }
         cluster_arrive();
         cluster_wait();
     }
-    if (TRAIN && sh.p >= 0) {
-        a.M[sh.p] = pM;
-        a.V[sh.p] = pV;
+    if (TRAIN && param >= 0) {
+        a.M[param] = pM;
+        a.V[param] = pV;
     }
 }
 
-constexpr size_t kStepSmem = (kParamsPadded + H * H + kStageRows * kChunkRow) * 4 + sizeof(Tile);
+constexpr size_t kStepSmem =
+    (kParamsPadded + H * H + kTermsWords + (kStageRows + 1) * kChunkRow + kStepThreads) * 4 + sizeof(Tile);
 
 // PT = W2 transposed.
 __global__ void k_mlp_transpose(const float *P, float *PT)
@@ -462,29 +618,26 @@ Norm host_norm(const ptw_mlp *m)
 
 // Device buffers of a training or gradient call, from one allocation.
 struct MlpScratch {
-    float *base = nullptr, *x = nullptr, *t = nullptr, *pt = nullptr, *lt = nullptr, *terms = nullptr;
-    uint32_t n_pad = 0;
+    float *base = nullptr, *x = nullptr, *t = nullptr, *pt = nullptr, *terms = nullptr, *lt = nullptr;
     cudaStream_t st;
     explicit MlpScratch(cudaStream_t s) : st(s) {}
-    // N samples, batches of at most B, `loss` squared errors.
-    cudaError_t alloc(uint64_t N, uint32_t B, uint64_t loss)
+    // N samples, `loss` squared errors.
+    cudaError_t alloc(uint64_t N, uint64_t loss)
     {
-        const uint64_t np = ((uint64_t)B + kTile - 1) / kTile * kTile;
         uint64_t at = 0;
         auto take = [&](uint64_t n) {
             const uint64_t o = at;
             at += (n + 3) & ~3ull;  // 16-byte rows
             return o;
         };
-        const uint64_t ox = take(N * IN), ot = take(N), opt = take(H * H), olt = take(loss), otr = take(kTermRows * np);
+        const uint64_t ox = take(N * IN), ot = take(N), opt = take(H * H), otr = take(2 * kCluster * kTermRows * kTile), olt = take(loss);
         const cudaError_t e = cudaMallocAsync((void **)&base, at * 4, st);
         if (e != cudaSuccess) return e;
         x = base + ox;
         t = base + ot;
         pt = base + opt;
-        lt = base + olt;
         terms = base + otr;
-        n_pad = (uint32_t)np;
+        lt = base + olt;
         return cudaSuccess;
     }
     ~MlpScratch()
@@ -666,7 +819,7 @@ try {
     PTW_CUDA(cudaSetDevice(m->device));
     cudaStream_t st = m->stream;
     MlpScratch s(st);
-    PTW_CUDA(s.alloc(B, B, B));
+    PTW_CUDA(s.alloc(B, B));
     PTW_CUDA(cudaMemcpyAsync(s.x, h_x, (uint64_t)B * IN * 4, cudaMemcpyHostToDevice, st));
     PTW_CUDA(cudaMemcpyAsync(s.t, h_t, B * 4ull, cudaMemcpyHostToDevice, st));
     k_mlp_transpose<<<(H * H + 255) / 256, 256, 0, st>>>(m->params, s.pt);
@@ -675,11 +828,11 @@ try {
     a.t = s.t;
     a.P = m->params;
     a.PT = s.pt;
+    a.terms = s.terms;
     a.G = m->grad;
     a.loss_terms = s.lt;
-    a.terms = s.terms;
-    a.n_pad = s.n_pad;
     a.n = a.batch = B;
+    a.epochs = 1;
     const int rc = launch_steps<false>(a, host_norm(m), st);
     if (rc) return rc;
     std::vector<float> lt(h_loss ? B : 0);
@@ -726,11 +879,14 @@ try {
     // copied (64 MB at most at a time).
     const uint32_t run = h_loss_curve ? (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(epochs, (16ull << 20) / N)) : 0;
     MlpScratch s(st);
-    PTW_CUDA(s.alloc(N, batch, (uint64_t)run * N));
-    // Per epoch: the order of the samples and the steps' bias corrections.
-    const uint64_t words = (uint64_t)N + 2ull * nb;
+    PTW_CUDA(s.alloc(N, (uint64_t)run * N));
+    // A launch runs `group` epochs, from their order of the samples and bias
+    // corrections: first one, then twice as many each time (the host makes the next
+    // ones meanwhile), 64 MB at most.
+    const uint64_t words = (uint64_t)N + 2ull * nb;  // per epoch
+    const uint32_t most = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>((epochs + 1) / 2, (16ull << 20) / words));
     uint32_t *d_plan = nullptr;
-    PTW_CUDA(cudaMallocAsync((void **)&d_plan, words * 4, st));
+    PTW_CUDA(cudaMallocAsync((void **)&d_plan, most * words * 4, st));
     struct Free {
         void *p;
         cudaStream_t st;
@@ -743,13 +899,11 @@ try {
     a.x = s.x;
     a.t = s.t;
     a.idx = d_plan;
-    a.corr = reinterpret_cast<const float *>(d_plan + N);
     a.P = m->params;
     a.PT = s.pt;
+    a.terms = s.terms;
     a.M = m->m;
     a.V = m->v;
-    a.terms = s.terms;
-    a.n_pad = s.n_pad;
     a.n = N;
     a.batch = batch;
     a.lr = lr;
@@ -757,37 +911,46 @@ try {
     a.b2 = 0.999f;
     a.eps = 1e-8f;
     const Norm nm = host_norm(m);
-    std::vector<uint32_t> plan(words);
+    std::vector<uint32_t> plan(most * words), order(N);
     std::vector<float> lt((uint64_t)run * N);
-    for (uint32_t i = 0; i < N; ++i) plan[i] = i;
+    for (uint32_t i = 0; i < N; ++i) order[i] = i;
     uint64_t rs = seed * 0x9E3779B97F4A7C15ull + 1;
     uint32_t ep0 = 0;  // first epoch whose squared errors are not copied yet
-    for (uint32_t ep = 0; ep < epochs; ++ep) {
-        for (uint32_t i = N - 1; i > 0; --i) {  // Fisher-Yates with an LCG
-            rs = rs * 6364136223846793005ull + 1442695040888963407ull;
-            std::swap(plan[i], plan[(rs >> 33) % (i + 1)]);
-        }
-        float *corr = reinterpret_cast<float *>(plan.data() + N);
-        for (uint32_t k = 0; k < nb; ++k) {
-            ++m->step;
-            corr[2 * k] = 1.f - std::pow(a.b1, (float)m->step);
-            corr[2 * k + 1] = 1.f - std::pow(a.b2, (float)m->step);
+    uint32_t group = 1;
+    for (uint32_t ep = 0; ep < epochs; group = std::min(2 * group, most)) {
+        uint32_t E = std::min(group, epochs - ep);
+        if (run) E = std::min(E, run - (ep - ep0));
+        float *corr = reinterpret_cast<float *>(plan.data() + (uint64_t)E * N);
+        for (uint32_t e = 0; e < E; ++e) {
+            for (uint32_t i = N - 1; i > 0; --i) {  // Fisher-Yates with an LCG
+                rs = rs * 6364136223846793005ull + 1442695040888963407ull;
+                std::swap(order[i], order[(rs >> 33) % (i + 1)]);
+            }
+            std::copy(order.begin(), order.end(), plan.begin() + (uint64_t)e * N);
+            for (uint32_t k = 0; k < nb; ++k) {
+                ++m->step;
+                *corr++ = 1.f - std::pow(a.b1, (float)m->step);
+                *corr++ = 1.f - std::pow(a.b2, (float)m->step);
+            }
         }
         // (the copy has left `plan` when the call returns: pageable memory)
-        PTW_CUDA(cudaMemcpyAsync(d_plan, plan.data(), words * 4, cudaMemcpyHostToDevice, st));
+        PTW_CUDA(cudaMemcpyAsync(d_plan, plan.data(), E * words * 4, cudaMemcpyHostToDevice, st));
+        a.corr = reinterpret_cast<const float *>(d_plan + (uint64_t)E * N);
         a.loss_terms = run ? s.lt + (uint64_t)(ep - ep0) * N : nullptr;
+        a.epochs = E;
         const int rc = launch_steps<true>(a, nm, st);
         if (rc) return rc;
-        if (run && (ep + 1 == epochs || ep + 1 - ep0 == run)) {
-            PTW_CUDA(cudaMemcpyAsync(lt.data(), s.lt, (uint64_t)(ep + 1 - ep0) * N * 4, cudaMemcpyDeviceToHost, st));
+        ep += E;
+        if (run && (ep == epochs || ep - ep0 == run)) {
+            PTW_CUDA(cudaMemcpyAsync(lt.data(), s.lt, (uint64_t)(ep - ep0) * N * 4, cudaMemcpyDeviceToHost, st));
             PTW_CUDA(cudaStreamSynchronize(st));
-            for (uint32_t e = ep0; e <= ep; ++e) {
+            for (uint32_t e = ep0; e < ep; ++e) {
                 double loss = 0;
                 for (uint32_t b0 = 0; b0 < N; b0 += batch)
                     loss += mean_loss(lt.data() + (uint64_t)(e - ep0) * N + b0, std::min(batch, N - b0));
                 h_loss_curve[e] = (float)(loss / nb);
             }
-            ep0 = ep + 1;
+            ep0 = ep;
         }
     }
     PTW_CUDA(cudaStreamSynchronize(st));
