@@ -431,20 +431,19 @@ int run_endpoint(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_pairs, bool 
     return PTW_OK;
 }
 
-int run_paths(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t L, int32_t *d_paths)
+int run_paths(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t L, int32_t *d_paths, bool timed)
 {
     int rc = upload_sources(g, cfg);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[3], g->stream));
-    PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 2 * sizeof(unsigned long long), g->stream));
-    PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
+    PTW_CUDA(mark(g, 3, timed));
+    PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers && L) {
         const uint64_t w0 = cfg->first_walker;
         rc = launch_paths(g, w0, w0 + cfg->n_walkers, L, cfg->seed, cfg->start_mode,
                           cfg->start_mode == PTW_START_SOURCES ? cfg->n_sources : 0, d_paths);
         if (rc) return rc;
     }
-    PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
+    PTW_CUDA(mark(g, 1, timed));
     return PTW_OK;
 }
 
@@ -518,23 +517,23 @@ int n2v_thresholds(double p, double q, uint64_t thr[3])
 }
 
 int run_node2vec(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t L, double p, double q, const uint64_t thr[3],
-                 int32_t *d_paths)
+                 int32_t *d_paths, bool timed)
 {
     int rc = upload_sources(g, cfg);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[3], g->stream));
+    PTW_CUDA(mark(g, 3, timed));
     PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 5 * sizeof(unsigned long long), g->stream));
     if (cfg->n_walkers && L && !(ensure_ext_columns(g) && ensure_edge_filter(g)))
         return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
                                 "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
-    PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
+    PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers && L) {
         const uint64_t w0 = cfg->first_walker;
         rc = launch_node2vec(g, w0, w0 + cfg->n_walkers, L, cfg->seed, cfg->start_mode,
                              cfg->start_mode == PTW_START_SOURCES ? cfg->n_sources : 0, p, q, thr, d_paths);
         if (rc) return rc;
     }
-    PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
+    PTW_CUDA(mark(g, 1, timed));
     return PTW_OK;
 }
 
@@ -992,9 +991,9 @@ try {
     if (!d_paths && cfg->n_walkers && L) return fail(PTW_EINVAL, "null paths buffer");
     if (g->dg.id_bound > 0x80000000u) return fail(PTW_EINVAL, "names above 2^31-1 do not fit int32 paths");
     PTW_CUDA(cudaSetDevice(g->device));
-    rc = run_paths(g, cfg, L, d_paths);
+    rc = run_paths(g, cfg, L, d_paths, stats != nullptr);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     if ((rc = check_word_status(g))) return rc;
     if (stats) {
         PTW_CUDA(cudaStreamSynchronize(g->stream));
@@ -1062,9 +1061,9 @@ try {
     if (!d_paths && cfg->n_walkers && L) return fail(PTW_EINVAL, "null paths buffer");
     if (g->dg.id_bound > 0x80000000u) return fail(PTW_EINVAL, "names above 2^31-1 do not fit int32 paths");
     PTW_CUDA(cudaSetDevice(g->device));
-    rc = run_node2vec(g, cfg, L, p, q, thr, d_paths);
+    rc = run_node2vec(g, cfg, L, p, q, thr, d_paths, stats != nullptr);
     if (rc) return rc;
-    PTW_CUDA(cudaEventRecord(g->ev[2], g->stream));
+    PTW_CUDA(mark(g, 2, stats != nullptr));
     if ((rc = check_word_status(g))) return rc;
     return stats ? node2vec_stats(g, cfg, stats) : PTW_OK;
 } catch (...) {
