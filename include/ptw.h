@@ -93,7 +93,9 @@ typedef struct ptw_walk_stats {
  * built with block 256, ilp 2, chunk 256, paths_ilp 2, cache_hints 1,
  * paths_named 1 and zeros; while the fields that count and endpoint walks
  * read have these values, the library picks kernel, column layout and launch
- * of those walks by their number of walkers. */
+ * of those walks by their number of walkers.  Count and endpoint walks of at most
+ * 1,024 walkers per SM do not depend on block, ilp, chunk, hot_k, min_blocks and
+ * ext_columns. */
 typedef struct ptw_tune {
     int32_t block;         /* threads per block (multiple of 32) */
     int32_t ilp;           /* walkers held per thread: 1, 2 or 4 */

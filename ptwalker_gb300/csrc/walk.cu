@@ -854,9 +854,22 @@ static bool paths_launch_is_auto(const ptw_tune &t)
            !(t.ext_columns & 2);
 }
 
+// k_walk_queued takes the walks of a graph whose launch parameters are untouched,
+// and of others those of one wave, where block, chunk and layout only decide how
+// few SMs share them: the launch that is best at scale 24 (768 threads, chunk 64,
+// 8,192 hot counters, extended columns) took 16 to 100% longer for 300 to 155,000
+// walkers on R-MAT scales 10 to 22 (30,000 at scale 16 77 us against 54, 100,000 at
+// scale 20 94 against 73; of 300,000 on either may win).  Merged visits, walkers in
+// shared memory and a limit on blocks stay what they say.
+static bool walk_is_queued(const ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
+{
+    return walk_launch_is_auto(t) ||
+           (n_walk <= queued_lanes(g) && !t.warp_agg && !t.gather_slots && !t.blocks_per_sm && t.cache_hints);
+}
+
 bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
 {
-    if (walk_launch_is_auto(t)) return n_walk <= queued_lanes(g);
+    if (walk_is_queued(g, t, n_walk)) return n_walk <= queued_lanes(g);
     return !t.gather_slots && !t.warp_agg && (t.ext_columns & 1) && ensure_ext_columns(g);
 }
 
@@ -1010,7 +1023,10 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
 {
     int rc = check_tune(t);
     if (rc) return rc;
-    if (walk_launch_is_auto(t)) return launch_walk_queued(g, wl);
+    if (walk_is_queued(g, t, wl.w_end - wl.w_begin)) {
+        if (t.ext_columns & 1) ensure_ext_columns(g);  // for the launches that read them
+        return launch_walk_queued(g, wl);
+    }
     const DeviceGraph &dg = g->dg;
     WalkArgs a = walk_args(g, wl);
     a.chunk = (uint32_t)t.chunk;

@@ -1,6 +1,7 @@
 // k_walk_queued: the count / endpoint walk of a graph whose walk launch
-// parameters are the ones it was built with (walk_launch_is_auto): kernel,
-// layout and launch follow the number of walkers.  Included by walk.cu.
+// parameters are the ones it was built with (walk_launch_is_auto), and of any
+// graph the walks of one wave (walk_is_queued): kernel, layout and launch follow
+// the number of walkers.  Included by walk.cu.
 //
 // What bounds such a walk is either the latency of a move (walkers for one
 // wave at most: the longest walk, 75 moves for 10^5 walkers at sp 0.15, is
