@@ -409,8 +409,13 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     auto clk = [] { return std::chrono::duration<double>(std::chrono::steady_clock::now().time_since_epoch()).count(); };
     const double t_enter = clk();
     double t_plan = 0, t_setup = 0;
-    std::vector<unsigned long long> h_tab(nq + 1);
-    std::vector<uint32_t> h_src(nq), h_qid(nq), h_mask(nq), h_cap(nq);
+    // The queries' tables as the walk reads them, in one upload: first slots
+    // [nq + 1], then sources, ids and masks [nq] each.
+    const uint64_t tab_words = nq + 1 + (3ull * nq + 1) / 2;
+    std::vector<unsigned long long> h_tab(tab_words);
+    uint32_t *const h_src = reinterpret_cast<uint32_t *>(h_tab.data() + nq + 1), *const h_qid = h_src + nq,
+                    *const h_mask = h_qid + nq;
+    std::vector<uint32_t> h_cap(nq);
     std::vector<uint8_t> h_dense(nq);
     std::vector<uint64_t> j0(nq, 0), cnt(nq);
     for (uint32_t i = 0; i < nq; ++i) {
@@ -435,24 +440,18 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     const uint64_t n_slots = h_tab[nq];
     const int sp_up = ph->begin(PhaseTimer::kUpload, st);
     DevBuf db(st);
-    unsigned long long *d_tab, *d_slots, *d_ctrl;
-    uint32_t *d_src, *d_qid, *d_mask, *d_flag;
+    unsigned long long *d_tab, *d_slots, *d_ctrl;  // d_ctrl: cursor, moves, then the queries' flags
     uint3 *d_desc;
-    PTW_CUDA(db.alloc(&d_tab, nq + 1));
-    PTW_CUDA(db.alloc(&d_src, nq));
-    PTW_CUDA(db.alloc(&d_qid, nq));
-    PTW_CUDA(db.alloc(&d_mask, nq));
-    PTW_CUDA(db.alloc(&d_flag, nq));
-    PTW_CUDA(db.alloc(&d_ctrl, 2));
+    const uint64_t ctrl_words = 2 + (nq + 1ull) / 2;
+    PTW_CUDA(db.alloc(&d_tab, tab_words));
+    PTW_CUDA(db.alloc(&d_ctrl, ctrl_words));
     PTW_CUDA(db.alloc(&d_desc, nd));
     PTW_CUDA(db.alloc(&d_slots, n_slots));
-    PTW_CUDA(cudaMemcpyAsync(d_tab, h_tab.data(), (nq + 1) * 8ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_src, h_src.data(), nq * 4ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_qid, h_qid.data(), nq * 4ull, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemcpyAsync(d_mask, h_mask.data(), nq * 4ull, cudaMemcpyHostToDevice, st));
+    uint32_t *const d_src = reinterpret_cast<uint32_t *>(d_tab + nq + 1), *const d_qid = d_src + nq,
+                    *const d_mask = d_qid + nq, *const d_flag = reinterpret_cast<uint32_t *>(d_ctrl + 2);
+    PTW_CUDA(cudaMemcpyAsync(d_tab, h_tab.data(), tab_words * 8, cudaMemcpyHostToDevice, st));
     PTW_CUDA(cudaMemcpyAsync(d_desc, h_desc.get(), nd * sizeof(uint3), cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemsetAsync(d_flag, 0, nq * 4ull, st));
-    PTW_CUDA(cudaMemsetAsync(d_ctrl, 0, 16, st));
+    PTW_CUDA(cudaMemsetAsync(d_ctrl, 0, ctrl_words * 8, st));
     PTW_CUDA(cudaMemsetAsync(d_slots, 0, n_slots * 8, st));
     ph->end(sp_up, st);
     if (timing) {
@@ -535,21 +534,25 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     ph->end(sp_walk, st);
     PTW_CUDA(cudaEventRecord(g->ev[1], st));
     PTW_CUDA(cudaGetLastError());
-    std::vector<uint32_t> h_flag(nq);
-    unsigned long long h_moves = 0;
-    PTW_CUDA(cudaMemcpyAsync(h_flag.data(), d_flag, nq * 4ull, cudaMemcpyDeviceToHost, st));
-    PTW_CUDA(cudaMemcpyAsync(&h_moves, d_ctrl + 1, 8, cudaMemcpyDeviceToHost, st));
     int rc = compact_tables(g, d_slots, h_tab.data(), h_cap.data(), h_dense.data(), nq, &wr.c);
-    if (!rc) rc = check_word_status(g);
+    // (read behind the compaction: a copy into pageable memory waits for the walk,
+    // and the compaction's launches would wait with it)
+    std::vector<unsigned long long> h_ctrl(ctrl_words);
+    if (!rc) {
+        const cudaError_t e = cudaMemcpyAsync(h_ctrl.data(), d_ctrl, ctrl_words * 8, cudaMemcpyDeviceToHost, st);
+        rc = e == cudaSuccess ? check_word_status(g) : cuda_fail(e, "batch flags");
+    }
+    const uint32_t *const h_flag = reinterpret_cast<const uint32_t *>(h_ctrl.data() + 2);
     early.join();
     wr.c.pre_join = nullptr;
     wr.c.pre_names.reset();
     wr.c.pre_counts.reset();
     if (rc) return rc;
+    PTW_CUDA(cudaStreamSynchronize(st));
     float ms = 0;
     PTW_CUDA(cudaEventElapsedTime(&ms, g->ev[0], g->ev[1]));
     *walk_ms += ms;
-    *moves_out += h_moves;
+    *moves_out += h_ctrl[1];
     if (timing)
         std::fprintf(stderr,
                      "[ptw] wave of %u queries, %llu descriptors, %llu slots: plan %.1f ms, setup %.1f ms, "
@@ -689,7 +692,8 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
     DevBuf db(st);
     // What the kernels read of the tables, in one upload: base, chunk starts,
     // lengths, kinds; and what they add to, in one clear: cnt, fill, histograms.
-    unsigned long long *d_in, *d_zero, *d_sums, *d_cc, *d_hc, *d_pos = nullptr, *d_hpos = nullptr;
+    // Its scratch is one allocation.
+    unsigned long long *d_in;
     const uint64_t in_words = 2ull * nt + 1 + (4ull * nt + nt + 7) / 8;
     std::vector<unsigned long long> in(in_words);
     std::memcpy(in.data(), h_base, nt * 8ull);
@@ -698,31 +702,29 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
     std::memcpy(in_cap, h_cap, nt * 4ull);
     std::memcpy(in_cap + nt, dense_flags.data(), nt);
     const uint64_t hist_words = k ? (uint64_t)nt * kCountBins / 2 : 0;
-    PTW_CUDA(db.alloc(&d_in, in_words));
-    PTW_CUDA(db.alloc(&d_zero, 2ull * nt + hist_words));
-    PTW_CUDA(db.alloc(&d_sums, (k ? 3ull : 1ull) * (nt + 1)));
+    const uint64_t zero_words = 2ull * nt + hist_words, sums_words = (k ? 3ull : 1ull) * (nt + 1);
+    const uint64_t npc = nch * 8;  // warp pieces: 8 per chunk
+    PTW_CUDA(db.alloc(&d_in, in_words + zero_words + sums_words + (k ? nt + (nt + 1ull) / 2 : 0) + (k ? 2 : 4) * npc));
+    unsigned long long *const d_zero = d_in + in_words, *const d_sums = d_zero + zero_words;
+    unsigned long long *const d_sel = k ? d_sums + sums_words : nullptr;
+    uint32_t *const d_thr = k ? reinterpret_cast<uint32_t *>(d_sel + nt) : nullptr;
+    unsigned long long *const d_cc = d_sums + sums_words + (k ? nt + (nt + 1ull) / 2 : 0), *const d_hc = d_cc + npc;
+    unsigned long long *const d_pos = d_hc + npc, *const d_hpos = d_pos + npc;  // (!k only)
     unsigned long long *const d_base = d_in, *const d_tch = d_in + nt;
     uint32_t *const d_cap = reinterpret_cast<uint32_t *>(d_in + 2ull * nt + 1);
     uint8_t *const d_dense = reinterpret_cast<uint8_t *>(d_cap + nt);
     unsigned long long *const d_cnt = d_zero, *const d_fill = d_zero + nt;
     uint32_t *const d_hist = reinterpret_cast<uint32_t *>(d_zero + 2ull * nt);
     unsigned long long *const d_seg = d_sums, *const d_sseg = d_sums + (nt + 1), *const d_kseg = d_sums + 2ull * (nt + 1);
-    uint32_t *d_thr = nullptr;
-    unsigned long long *d_sel = nullptr;
-    const uint64_t npc = nch * 8;  // warp pieces: 8 per chunk
-    PTW_CUDA(db.alloc(&d_cc, std::max<uint64_t>(npc, 1)));
-    PTW_CUDA(db.alloc(&d_hc, std::max<uint64_t>(npc, 1)));
     const int sp_count = ph->begin(PhaseTimer::kCount, st);
     PTW_CUDA(cudaMemcpyAsync(d_in, in.data(), in_words * 8, cudaMemcpyHostToDevice, st));
-    PTW_CUDA(cudaMemsetAsync(d_zero, 0, (2ull * nt + hist_words) * 8, st));
+    PTW_CUDA(cudaMemsetAsync(d_zero, 0, zero_words * 8, st));
     // Pass 1: occupied entries per chunk and per table (+ histograms for top-k,
     // and from those the lowest bin that top-k keeps of each table).
     if (k) {
         if (nch)
             k_tabs_count<true><<<(unsigned)nch, 256, 0, st>>>(d_slots, d_base, d_cap, d_dense, d_tch, nt, d_cnt, d_cc,
                                                              d_hc, d_hist);
-        PTW_CUDA(db.alloc(&d_thr, nt));
-        PTW_CUDA(db.alloc(&d_sel, nt));
         k_tabs_thresh<<<(nt + 7) / 8, 256, 0, st>>>(d_cnt, d_hist, nt, k, d_thr, d_sel);
     } else if (nch) {
         k_tabs_count<false><<<(unsigned)nch, 256, 0, st>>>(d_slots, d_base, d_cap, d_dense, d_tch, nt, d_cnt, d_cc,
@@ -730,19 +732,22 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
     }
     k_table_sums<<<1, 1024, 0, st>>>(d_cnt, d_sel, nt, k, d_sums);
     PTW_CUDA(cudaGetLastError());
-    std::vector<unsigned long long> sums((k ? 3ull : 1ull) * (nt + 1));
-    PTW_CUDA(cudaMemcpyAsync(sums.data(), d_sums, sums.size() * 8, cudaMemcpyDeviceToHost, st));
     if (!k && nch) {
         // output position of every dense piece, sort-input position of every hash piece
-        PTW_CUDA(db.alloc(&d_pos, npc));
-        PTW_CUDA(db.alloc(&d_hpos, npc));
-        PTW_CUDA(cub_call([&](void *t, size_t &b) {
-            return cub::DeviceScan::ExclusiveSum(t, b, d_cc, d_pos, (int64_t)npc, st);
-        }, st));
-        PTW_CUDA(cub_call([&](void *t, size_t &b) {
-            return cub::DeviceScan::ExclusiveSum(t, b, d_hc, d_hpos, (int64_t)npc, st);
-        }, st));
+        if (npc <= kPieceSums) {
+            k_piece_sums<<<2, 1024, 0, st>>>(d_cc, npc, d_pos);
+            PTW_CUDA(cudaGetLastError());
+        } else {
+            PTW_CUDA(cub_call([&](void *t, size_t &b) {
+                return cub::DeviceScan::ExclusiveSum(t, b, d_cc, d_pos, (int64_t)npc, st);
+            }, st));
+            PTW_CUDA(cub_call([&](void *t, size_t &b) {
+                return cub::DeviceScan::ExclusiveSum(t, b, d_hc, d_hpos, (int64_t)npc, st);
+            }, st));
+        }
     }
+    std::vector<unsigned long long> sums(sums_words);
+    PTW_CUDA(cudaMemcpyAsync(sums.data(), d_sums, sums.size() * 8, cudaMemcpyDeviceToHost, st));
     ph->end(sp_count, st);
     PTW_CUDA(cudaStreamSynchronize(st));
     std::copy(sums.begin(), sums.begin() + nt + 1, out->seg.begin());
@@ -889,11 +894,11 @@ int compact_tables(ptw_graph *g, unsigned long long *d_slots, const unsigned lon
             unsigned long long *d_hseg = nullptr;
             uint32_t *h_name = nullptr, *h_cnt = nullptr, *s_name = nullptr, *s_cnt = nullptr;
             if (n_hash) {
-                PTW_CUDA(db.alloc(&h_name, n_hash));
-                PTW_CUDA(db.alloc(&h_cnt, n_hash));
-                PTW_CUDA(db.alloc(&s_name, n_hash));
-                PTW_CUDA(db.alloc(&s_cnt, n_hash));
-                PTW_CUDA(db.alloc(&d_hseg, nt + 1));
+                PTW_CUDA(db.alloc(&d_hseg, nt + 1 + 2 * n_hash));
+                h_name = reinterpret_cast<uint32_t *>(d_hseg + nt + 1);
+                h_cnt = h_name + n_hash;
+                s_name = h_cnt + n_hash;
+                s_cnt = s_name + n_hash;
                 PTW_CUDA(cudaMemcpyAsync(d_hseg, hseg.data(), (nt + 1) * 8ull, cudaMemcpyHostToDevice, st));
             }
             // Pass 2 and the hash sorts run over R ranges of consecutive tables

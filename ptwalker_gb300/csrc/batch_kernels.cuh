@@ -792,6 +792,46 @@ __global__ void __launch_bounds__(1024) k_table_sums(const unsigned long long *c
     }
 }
 
+// pos[b * n + i] = exclusive sums of cc[b * n ..] over n pieces, one block each of
+// the two; up to kPieceSums of them (beyond, many blocks are quicker than two
+// library scans of two launches each are long).
+constexpr uint64_t kPieceSums = 32768;
+__global__ void __launch_bounds__(1024) k_piece_sums(const unsigned long long *cc, uint64_t n, unsigned long long *pos)
+{
+    constexpr uint32_t kEach = 4;
+    __shared__ unsigned long long s_w[2][32];
+    cc += blockIdx.x * n;
+    pos += blockIdx.x * n;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    auto scan = [&](unsigned long long x) {
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kBFull, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        return x;
+    };
+    unsigned long long before = 0;
+    uint32_t flip = 0;
+    for (uint64_t i0 = 0; i0 < n; i0 += 1024 * kEach, flip ^= 1) {
+        const uint64_t i = i0 + threadIdx.x * kEach;
+        unsigned long long x[kEach], sum = 0;
+#pragma unroll
+        for (uint32_t e = 0; e < kEach; ++e) sum += x[e] = i + e < n ? cc[i + e] : 0;
+        const unsigned long long inc = scan(sum);
+        if (lane == 31) s_w[flip][warp] = inc;
+        __syncthreads();
+        const unsigned long long w = scan(s_w[flip][lane]);  // of the warps
+        const unsigned long long up = __shfl_sync(kBFull, w, (warp + 31) & 31);
+        unsigned long long at = before + inc - sum + (warp ? up : 0);
+        before += __shfl_sync(kBFull, w, 31);
+#pragma unroll
+        for (uint32_t e = 0; e < kEach; ++e) {
+            if (i + e < n) pos[i + e] = at;
+            at += x[e];
+        }
+    }
+}
+
 // Hash entries j in [j0, j1), sorted by name within their table t's range
 // [hseg[t], hseg[t + 1]), go to position seg[t] + (j - hseg[t]) of the
 // output.
