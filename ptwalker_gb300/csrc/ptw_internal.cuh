@@ -339,8 +339,8 @@ struct ptw_graph {
     int num_sms = 0;
     ptw_tune tune{};
     ptw_batch_tune btune{};  // zero fields: defaults (see ptw_batch_tune)
-    void *vertex_arrays = nullptr;  // one allocation: dg.adj .. dg.names, dg.rows, sc.counts, sc.ctrl
-    uint32_t *row_space = nullptr;  // room of the row table in it
+    std::vector<void *> arrays;     // allocations of dg.adj, col .. names, rows, sc.counts, sc.ctrl
+    uint32_t *row_space = nullptr;  // room of the row table among them
     uint64_t device_bytes = 0;
     int ext_users = 0;  // open servers reading the extended columns (kept while > 0)
     ptw::AsyncSlot async[2];             // pipelined count walks in flight
