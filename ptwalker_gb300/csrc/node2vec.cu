@@ -139,7 +139,9 @@ struct LaneArgs {
 // Walker slot states.
 enum : uint32_t { kIdle = 0, kDraw = 1, kFilter = 2, kSearch = 3 };
 
-// The filter stays in L2, the columns stream through it; node2vec of more walkers
+// The filter stays in L2, the columns pass through it at normal priority (p = 2,
+// q = 0.5, 40 positions, scale 16 244 -> 216 us, behind a kernel that filled L2 271 ->
+// 226, 22 3,734 -> 3,713); node2vec of more walkers
 // than are resident without a limit (WAVE: at most those) is held to 64 registers,
 // for 1,024 walkers per SM (R-MAT scale 22 7,616 -> 7,420 us, 12 385 -> 403).
 // Against 64-bit hashes, two 16-byte reads per block and the filter streaming as
@@ -170,7 +172,8 @@ __global__ void __launch_bounds__(kLaneWarps * 32, WAVE ? 1 : 8) k_lane_paths(co
     const uint32_t wib = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
     const uint64_t pol_keep = l2_policy(a.hints ? 1 : 0);
-    const uint64_t pol_stream = l2_policy(a.hints ? 2 : 0);
+    // (first to be evicted, the columns do not replace what other kernels left in L2)
+    const uint64_t pol_col = l2_policy(0);
     const uint64_t thr_lo = a.thr_nb < a.thr_out ? a.thr_nb : a.thr_out;
     const uint64_t thr_hi = a.thr_nb < a.thr_out ? a.thr_out : a.thr_nb;
     const uint32_t chunk = 32 * ILP;
@@ -302,7 +305,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, WAVE ? 1 : 8) k_lane_paths(co
                 if (appx[s]) x[s] = make_uint4(t[s], trec[s].x, trec[s].y, tname[s]);
                 else
                     x[s] = ld_line_u4(&a.col_ext[PTW_IDX((uint64_t)rec[s].x + idx, a.m, &a.ctrl[7], kCheckColumn)],
-                                      pol_stream);
+                                      pol_col);
             } else if (st[s] == kFilter) {
                 const FilterKey fk = filter_key(t[s], cx[s].x, a.filter_blocks);
                 fbits[s] = (uint64_t)fk.b << 30 | (fk.a & 0x3FFFFFFFu);
@@ -311,7 +314,7 @@ __global__ void __launch_bounds__(kLaneWarps * 32, WAVE ? 1 : 8) k_lane_paths(co
             } else if (st[s] == kSearch) {
                 mid[s] = lo[s] + ((hi[s] - lo[s]) >> 1);
                 x[s] = ld_line_u4(&a.col_ext[PTW_IDX((uint64_t)soff[s] + mid[s], a.m, &a.ctrl[7], kCheckColumn)],
-                                  pol_stream);
+                                  pol_col);
             }
         }
 

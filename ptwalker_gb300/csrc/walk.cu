@@ -635,7 +635,11 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
         row_table_load(s_rows, a.rows, a.row_words);
         __syncthreads();
     }
-    const uint64_t pol_keep = l2_policy(1), pol_stream = l2_policy(2);
+    // the columns at normal priority: first to be evicted, they do not replace what
+    // other kernels left in L2 (scale 20 after a build, whose temporaries stay mapped,
+    // 810 -> 620 us; in a row of calls 40 positions 397 -> 302, scale 21 811 -> 741,
+    // 22 and 23 the same)
+    const uint64_t pol_keep = l2_policy(1), pol_col = l2_policy(0), pol_out = l2_policy(2);
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t n_groups = (a.n_walk + 31) / 32;
     unsigned long long moves = 0;
@@ -669,7 +673,7 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
             int32_t *o = a.paths + g * 32 * a.L + c0 + lane;
             if (c0 + lane < p)
 #pragma unroll 4
-                for (uint32_t r = 0; r < rows; ++r) st_hint_s32(o + (uint64_t)r * a.L, stage[r][lane], pol_stream);
+                for (uint32_t r = 0; r < rows; ++r) st_hint_s32(o + (uint64_t)r * a.L, stage[r][lane], pol_out);
             __syncwarp();
         };
         const bool valid = alive;
@@ -684,11 +688,11 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
                 if (alive) {
                     const uint64_t e = PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, a.check, kCheckColumn);
                     if (EXT) {
-                        const uint4 x = ld_hint_u4(&a.col_ext[e], pol_stream);
+                        const uint4 x = ld_hint_u4(&a.col_ext[e], pol_col);
                         rec = make_uint2(x.y, x.z);
                         next_name = x.w;
                     } else {
-                        v = ld_line_u32(&a.col[e], pol_stream);
+                        v = ld_line_u32(&a.col[e], pol_col);
                     }
                 }
             }
@@ -825,6 +829,7 @@ void *pick_walk(bool endpoint, int ilp, bool hot, int min_blocks, int block, boo
 namespace ptw {
 
 // Walkers of one wave of k_walk_queued.
+constexpr uint64_t kColumnsStay = 192ull << 20;
 static uint64_t queued_lanes(const ptw_graph *g) { return (uint64_t)g->num_sms * kQueuedBlock; }
 
 ptw_tune default_tune()
@@ -1002,6 +1007,11 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
     // scale 16 (45,000) with 1,024, from one wave on 8,192 and 4,096 are alike.
     if (!wl.endpoint)
         a.hot_k = std::min<uint32_t>(!one_wave ? 8192u : a.n_walk >= 24576 ? 1024u : 0u, g->dg.n);
+    // Columns that L2 holds for the most part stay at normal priority, to replace what
+    // other kernels left there (scale 18 66 -> 64 us, 19 91 -> 81, 20 126 -> 116; behind
+    // a kernel that filled L2 81 -> 64, 100 -> 87, 134 -> 128); larger ones are first to
+    // be evicted (RWR, scale 21 94 us against 97, 23 347 against 470).
+    a.hints = g->dg.m * sizeof(uint32_t) > kColumnsStay;
     const bool rows = !one_wave && g->dg.rows;
     if (rows) {
         a.rows = g->dg.rows;

@@ -61,7 +61,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
         for (uint32_t i = threadIdx.x; i < a.hot_k; i += blockDim.x) s_hot[i] = 0;
     __syncthreads();
     const uint64_t pol_keep = l2_policy(1);    // row records, counters, names
-    const uint64_t pol_stream = l2_policy(2);  // column array
+    const uint64_t pol_stream = l2_policy(a.hints ? 2 : 0);  // column array
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
 
