@@ -106,16 +106,23 @@ void trim_pools()
         if (p) cudaMemPoolTrimTo(p, 0);
 }
 
+uint64_t pool_held()
+{
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    uint64_t held = 0;
+    if (!g_pools[dev] || cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess)
+        return 0;
+    return held;
+}
+
 void release_pool_above(cudaStream_t st, uint64_t keep)
 {
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return;
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    uint64_t held = 0;
-    if (!g_pools[dev] || cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
-        held <= keep)
-        return;
+    if (pool_held() <= keep || cudaGetDevice(&dev) != cudaSuccess) return;
     cudaStreamSynchronize(st);  // frees queued on st have happened
+    std::lock_guard<std::mutex> lk(g_pool_mu);
     cudaMemPoolTrimTo(g_pools[dev], keep);
 }
 

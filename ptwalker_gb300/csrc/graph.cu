@@ -717,10 +717,11 @@ int build_arrays(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, boo
 int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m,
                                   bool as_undirected, bool clean, bool compact_names)
 {
-    const int rc = build_arrays(g, d_src, d_dst, m, as_undirected, clean, compact_names);
     // The temporaries come from the pool that batches use: mapping fresh memory
     // takes longer than a small build.  A large one hands back what it added.
-    release_pool_above(g->stream, kBuildPoolKeep);
+    const uint64_t before = pool_held();
+    const int rc = build_arrays(g, d_src, d_dst, m, as_undirected, clean, compact_names);
+    release_pool_above(g->stream, std::max(before, kBuildPoolKeep));
     return rc;
 }
 

@@ -414,6 +414,8 @@ int launch_lane_deepwalk(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_
 // pool hands memory back at each one), for count tables and the short-lived
 // buffers of every result compaction.  Freed with cudaFreeAsync.
 cudaError_t pooled_alloc_async(void **p, size_t bytes, cudaStream_t st);
+// Bytes that the current device's pool holds mapped.
+uint64_t pool_held();
 // Waits for st and unmaps what the pool holds unused above keep bytes.
 void release_pool_above(cudaStream_t st, uint64_t keep);
 // Hands the pools' cached memory back to the CUDA driver.
