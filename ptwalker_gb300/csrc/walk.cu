@@ -830,6 +830,7 @@ namespace ptw {
 
 // Walkers of one wave of k_walk_queued.
 constexpr uint64_t kColumnsStay = 192ull << 20;
+constexpr uint64_t kLocalBytes = 160 * 1024;
 static uint64_t queued_lanes(const ptw_graph *g) { return (uint64_t)g->num_sms * kQueuedBlock; }
 
 ptw_tune default_tune()
@@ -999,9 +1000,15 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
     if (wl.by_name) a.counts = wl.by_name;
     const bool one_wave = a.n_walk <= queued_lanes(g);
     const uint64_t per_sm = (a.n_walk + g->num_sms - 1) / g->num_sms;
-    const int block = (int)std::min<uint64_t>(kQueuedBlock, (per_sm + 31) / 32 * 32);
-    const uint64_t grid = std::min<uint64_t>(g->num_sms, (a.n_walk + block - 1) / block);
     const bool group = wl.start_mode == PTW_START_SOURCES && !wl.endpoint;
+    // A small graph is copied to shared memory by every block (of 256 threads at
+    // least), and a move then waits on L2 for neither of its two accesses (8 KB, 5,000
+    // walkers 54 -> 48 us a call, 150,000 90 -> 55; 153 KB 56 -> 51, 70 -> 63; of 210 KB
+    // the copy takes as long).  Merging visits (group), 256 threads per block are slower
+    // than the spread over all SMs (62 against 60 us).
+    const bool local = one_wave && !group && local_words(g->dg.n, g->dg.m) * 4 <= kLocalBytes;
+    const int block = std::max(local ? 256 : 32, (int)std::min<uint64_t>(kQueuedBlock, (per_sm + 31) / 32 * 32));
+    const uint64_t grid = std::min<uint64_t>(g->num_sms, (a.n_walk + block - 1) / block);
     // Hot counters pay once their flush (hot_k words per block) is small
     // beside the visits: scale 14 (12,557 walkers) is quicker without any,
     // scale 16 (45,000) with 1,024, from one wave on 8,192 and 4,096 are alike.
@@ -1018,8 +1025,8 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
         a.row_runs = g->dg.row_runs;
         a.row_words = row_words(g->dg.row_runs, g->dg.n);
     }
-    void *fn = pick_walk_queued(wl.endpoint, a.hot_k > 0, one_wave, group, rows);
-    const size_t smem = ((size_t)a.hot_k + a.row_words) * 4;
+    void *fn = pick_walk_queued(wl.endpoint, a.hot_k > 0, one_wave, group, rows, local);
+    const size_t smem = ((size_t)a.hot_k + a.row_words + (local ? local_words(g->dg.n, g->dg.m) : 0)) * 4;
     if (smem > 48 * 1024)
         PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     void *args[] = {&a};

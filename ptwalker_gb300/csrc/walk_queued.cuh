@@ -21,6 +21,8 @@
 //    table in shared memory (row_table.cuh), which leaves one gather per move;
 //    a 4-byte one, from the plain columns.  In one wave the L2 load of
 //    adj[v] is as quick as the lookup and the table need not be copied;
+//  - LOCAL: in one wave on a small graph, row records and columns are copied to
+//    shared memory, and the chain of a move is its draw and two reads there;
 //  - BYNAME: in one wave the visits are counted by name (an extra load off the
 //    chain) and there is no second kernel after the walk;
 //  - visits of the hottest ids are counted in shared memory: without it the
@@ -47,16 +49,36 @@ namespace {
 
 constexpr int kQueuedBlock = 1024;  // largest block, one per SM: 768 x 2 and 1024 x 2 were 3-10% slower
 
-// ROWS: row records from the row table in shared memory instead of adj.
-template <bool ENDPOINT, bool HOT, bool BYNAME, bool GROUP, bool ROWS>
+// Row records and columns of a graph that is copied to shared memory whole, in
+// words, each 16-byte aligned.
+__host__ __device__ __forceinline__ uint32_t local_adj_words(uint32_t n) { return (2 * n + 3) & ~3u; }
+__host__ __device__ __forceinline__ uint64_t local_words(uint32_t n, uint64_t m)
+{
+    return local_adj_words(n) + ((m + 3) & ~3ull);
+}
+
+// ROWS: row records from the row table in shared memory instead of adj; LOCAL: row
+// records and columns from shared memory.
+template <bool ENDPOINT, bool HOT, bool BYNAME, bool GROUP, bool ROWS, bool LOCAL = false>
 __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs a)
 {
     extern __shared__ __align__(16) uint32_t s_mem[];
     const uint32_t *s_rows = s_mem;
-    uint32_t *s_hot = s_mem + (ROWS ? a.row_words : 0u);
+    uint32_t *s_hot = s_mem + (ROWS ? a.row_words : LOCAL ? (uint32_t)local_words(a.n, a.m) : 0u);
+    const uint2 *s_adj = reinterpret_cast<const uint2 *>(s_mem);
+    const uint32_t *s_col = s_mem + local_adj_words(a.n);
     __shared__ unsigned long long s_moves;
     if (threadIdx.x == 0) s_moves = 0;
     if (ROWS) row_table_load(s_mem, a.rows, a.row_words);
+    if (LOCAL) {
+        // (the arrays' allocations end on 256-byte boundaries)
+        const uint64_t pol = l2_policy(0);
+        const uint32_t w = local_adj_words(a.n), all = (uint32_t)local_words(a.n, a.m);
+        for (uint32_t i = 4 * threadIdx.x; i < w; i += 4 * blockDim.x)
+            cp_async16(s_mem + i, reinterpret_cast<const uint32_t *>(a.adj) + i, pol);
+        for (uint32_t i = w + 4 * threadIdx.x; i < all; i += 4 * blockDim.x) cp_async16(s_mem + i, a.col + (i - w), pol);
+        cp_async_wait_all();
+    }
     if (HOT)
         for (uint32_t i = threadIdx.x; i < a.hot_k; i += blockDim.x) s_hot[i] = 0;
     __syncthreads();
@@ -88,9 +110,11 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
     };
     auto row = [&](uint32_t x) -> uint2 {
         if (ROWS) return row_of(s_rows, a.row_runs, (uint32_t)PTW_IDX(x, a.n, &a.ctrl[7], kCheckRecord));
+        if (LOCAL) return s_adj[PTW_IDX(x, a.n, &a.ctrl[7], kCheckRecord)];
         return ld_hint_u2(&a.adj[PTW_IDX(x, a.n, &a.ctrl[7], kCheckRecord)], pol_keep);
     };
     auto gather = [&]() -> uint32_t {
+        if (LOCAL) return s_col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)];
         return ld_line_u32(&a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)],
                            pol_stream);
     };
@@ -314,8 +338,13 @@ template <bool H, bool N, bool R> void *queued_fn(bool group)
 
 // The count walks that launch_walk_queued asks for: by name without row table
 // (one wave), or by internal id with hot counters (more).
-void *pick_walk_queued(bool endpoint, bool hot, bool by_name, bool group, bool rows)
+void *pick_walk_queued(bool endpoint, bool hot, bool by_name, bool group, bool rows, bool local)
 {
+    if (local) {  // (one wave, not grouped)
+        if (endpoint) return (void *)k_walk_queued<true, false, false, false, false, true>;
+        return hot ? (void *)k_walk_queued<false, true, true, false, false, true>
+                   : (void *)k_walk_queued<false, false, true, false, false, true>;
+    }
     if (endpoint)
         return rows ? (void *)k_walk_queued<true, false, false, false, true>
                     : (void *)k_walk_queued<true, false, false, false, false>;
