@@ -128,7 +128,7 @@ typedef struct ptw_tune {
 const char *ptw_last_error(void);
 const char *ptw_version(void);
 
-/* Device memory that batched queries and serving free goes back to a pool
+/* Device memory that batched queries, serving and graph builds free goes back to a pool
  * that keeps up to a quarter of the device memory mapped between calls, so
  * the next call reuses it instead of mapping tens of GB again.  This hands
  * that cached memory back to the CUDA driver (after waiting for the device).  An
