@@ -616,8 +616,8 @@ constexpr uint32_t kPathStage = 32;   // positions collected before they are wri
 // and names (scale 20: 54 against 79).  Otherwise the row record from L2 is as
 // quick, the output fits L2, and paths are written from registers.
 // Against k_paths on name-paired columns, one walker per vertex, 80 positions:
-// scale 10 66 -> 41 us, 16 74 -> 51, 18 169 -> 127, 20 859 -> 643, 22 4,563 ->
-// 3,880 us, 24 19.6 -> 18.3 ms.  At scale 22 a move without names and stores
+// scale 10 66 -> 41 us, 16 74 -> 51, 18 169 -> 138, 20 859 -> 588, 22 4,563 ->
+// 3,800 us, 24 19.6 -> 18.5 ms.  At scale 22 a move without names and stores
 // takes as long (50 G moves/s): it is one DRAM line.
 // EXT (extended columns asked for): the record and the name come with the 16-byte
 // entry.  Against k_lane_paths, scale 10 to 16 91 - 102 -> 31 - 37 us, 18 311 ->
