@@ -368,7 +368,7 @@ inline int batch_launch(const ptw_graph *g, bool ext, BatchArgs &a, BatchLaunch 
         a.row_runs = g->dg.row_runs;
         a.row_words = row_words(g->dg.row_runs, g->dg.n);
         l.smem = (size_t)a.row_words * 4;
-        PTW_CUDA(cudaFuncSetAttribute(l.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem));
+        PTW_CUDA(allow_shared(l.fn));
     }
     PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&l.per_sm, l.fn, l.block, l.smem));
     l.per_sm = std::max(l.per_sm, 1);

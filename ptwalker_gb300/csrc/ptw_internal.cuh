@@ -29,6 +29,16 @@ namespace ptw {
 
 constexpr size_t kMaxSharedBytes = 227 * 1024;  // dynamic shared memory of a block, sm_103a
 
+// Lets kernel fn be launched with all the dynamic shared memory that a block has
+// beside fixed_bytes of its own.  The limit belongs to the function, on each
+// device, not to a launch: graphs of other sizes, other threads and a server's
+// later ticks launch the same function, so it is always the same one and is never
+// set to what a launch needs.
+inline cudaError_t allow_shared(const void *fn, size_t fixed_bytes = 0)
+{
+    return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxSharedBytes - fixed_bytes));
+}
+
 // Names a host-side span for profilers (NVTX ranges; nothing is recorded
 // unless a profiler is attached).
 struct NvtxRange {

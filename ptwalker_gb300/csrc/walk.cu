@@ -1027,8 +1027,7 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
     }
     void *fn = pick_walk_queued(wl.endpoint, a.hot_k > 0, one_wave, group, rows, local);
     const size_t smem = ((size_t)a.hot_k + a.row_words + (local ? local_words(g->dg.n, g->dg.m) : 0)) * 4;
-    if (smem > 48 * 1024)
-        PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > 48 * 1024) PTW_CUDA(allow_shared(fn, kQueuedFixedBytes));
     void *args[] = {&a};
     PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)std::max<uint64_t>(grid, 1)), dim3(block), args, smem, g->stream));
     return PTW_OK;
@@ -1067,9 +1066,8 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
                : (t.warp_agg && !wl.endpoint) ? pick_walk_agg(t.ilp, hot, ext)
                                               : pick_walk(wl.endpoint, t.ilp, hot, t.min_blocks, t.block, ext);
     const size_t smem = slots ? async_smem(t.gather_slots, t.block, a.hot_k) : hot ? (size_t)a.hot_k * 4 : 0;
-    if (smem > 227 * 1024) return fail(PTW_EINVAL, "tune.gather_slots x tune.block x hot_k need too much shared memory");
-    if (smem > 48 * 1024)
-        PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (smem > kMaxSharedBytes) return fail(PTW_EINVAL, "tune.gather_slots x tune.block x hot_k need too much shared memory");
+    if (smem > 48 * 1024) PTW_CUDA(allow_shared(fn));
     int per_sm = 0;
     PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, t.block, smem));
     if (per_sm < 1) return fail(PTW_EINVAL, "walk kernel does not fit on an SM with this tune");
@@ -1150,8 +1148,7 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
         a.col_ext = g->dg.col_ext;
         a.vtx_ext = g->dg.vtx_ext;
         a.int2idx = dg.int2idx;
-        if (smem > 48 * 1024)
-            PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        if (smem > 48 * 1024) PTW_CUDA(allow_shared(fn));
         void *args[] = {&a};
         PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(block), args, smem, g->stream));
         return PTW_OK;

@@ -47,6 +47,7 @@
 namespace ptw {
 namespace {
 
+constexpr size_t kQueuedFixedBytes = 16;  // shared memory of the kernel's own (s_moves), at most
 constexpr int kQueuedBlock = 1024;  // largest block, one per SM: 768 x 2 and 1024 x 2 were 3-10% slower
 
 // Row records and columns of a graph that is copied to shared memory whole, in
