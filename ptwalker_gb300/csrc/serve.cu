@@ -96,6 +96,7 @@ struct Active {
     bool dense;         // dense array of n counters instead of a hash table
     uint64_t started;   // ranks run so far
     double admit_s;
+    bool cleared;       // its table holds nothing of an earlier query
 };
 
 // Pinned host memory that completed results are copied into by the device;
@@ -132,6 +133,7 @@ struct ptw_server {
     size_t plan_bytes = 0, ret_off = 0, ret_bytes = 0;
     std::deque<ptw::Pending> pending;
     std::vector<ptw::Active> active;
+    std::vector<ulonglong2> pieces;  // what the last step cleared (a copy in flight may read it)
     std::deque<ptw::Done> done;
     ptw::BatchArgs args{};
     unsigned grid = 1;
@@ -229,12 +231,17 @@ __global__ void __launch_bounds__(256) k_clear_tables(ulonglong2 *arena, const u
     for (uint32_t i = threadIdx.x; i < p.y / 2; i += 256) arena[p.x / 2 + i] = make_ulonglong2(0, 0);
 }
 
-// Zeroes the tables of newly admitted queries ({arena offset, slots}, even: the
-// arena hands out multiples of 256 slots): neighbours in one piece, several pieces in one
-// launch (300 queries at once: 300 clears of 2 us, or 30 us).
-int clear_tables(ptw_server *s, std::vector<std::pair<uint64_t, uint64_t>> &fresh)
+// Zeroes the tables of newly admitted queries (in multiples of two slots: the arena
+// hands out multiples of 256): neighbours in one piece, several pieces in one
+// launch (300 queries at once: 300 clears of 2 us, or 30 us), or one by one where
+// there is no memory for their list.  A query is marked once its clear is
+// queued, so that the next step clears what a failed one left.
+int clear_tables(ptw_server *s)
 {
     cudaStream_t st = s->g->stream;
+    std::vector<std::pair<uint64_t, uint64_t>> fresh;  // {arena offset, slots}
+    for (const Active &a : s->active)
+        if (!a.cleared) fresh.emplace_back(a.off, (a.cap + 1) & ~1ull);
     std::sort(fresh.begin(), fresh.end());
     size_t n = 0;
     for (const auto &f : fresh) {
@@ -242,23 +249,30 @@ int clear_tables(ptw_server *s, std::vector<std::pair<uint64_t, uint64_t>> &fres
         else fresh[n++] = f;
     }
     fresh.resize(n);
-    if (n <= 2) {
-        for (const auto &f : fresh) PTW_CUDA(cudaMemsetAsync(s->arena + f.first, 0, f.second * 8, st));
-        return PTW_OK;
-    }
-    std::vector<ulonglong2> pieces;
-    for (const auto &f : fresh)
-        for (uint64_t o = 0; o < f.second; o += kClearSlots)
-            pieces.push_back(make_ulonglong2(f.first + o, std::min<uint64_t>(kClearSlots, f.second - o)));
     ulonglong2 *d = nullptr;
-    PTW_CUDA(pooled_alloc_async((void **)&d, pieces.size() * sizeof(ulonglong2), st));
-    cudaError_t e = cudaMemcpyAsync(d, pieces.data(), pieces.size() * sizeof(ulonglong2), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) {
-        k_clear_tables<<<(unsigned)pieces.size(), 256, 0, st>>>(reinterpret_cast<ulonglong2 *>(s->arena), d);
-        e = cudaGetLastError();
+    if (n > 2) {
+        s->pieces.clear();
+        for (const auto &f : fresh)
+            for (uint64_t o = 0; o < f.second; o += kClearSlots)
+                s->pieces.push_back(make_ulonglong2(f.first + o, std::min<uint64_t>(kClearSlots, f.second - o)));
+        if (pooled_alloc_async((void **)&d, s->pieces.size() * sizeof(ulonglong2), st) != cudaSuccess) {
+            d = nullptr;
+            cudaGetLastError();
+        }
     }
-    cudaFreeAsync(d, st);
-    PTW_CUDA(e);
+    if (d) {
+        cudaError_t e = cudaMemcpyAsync(d, s->pieces.data(), s->pieces.size() * sizeof(ulonglong2),
+                                        cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) {
+            k_clear_tables<<<(unsigned)s->pieces.size(), 256, 0, st>>>(reinterpret_cast<ulonglong2 *>(s->arena), d);
+            e = cudaGetLastError();
+        }
+        cudaFreeAsync(d, st);
+        PTW_CUDA(e);
+    } else {
+        for (const auto &f : fresh) PTW_CUDA(cudaMemsetAsync(s->arena + f.first, 0, f.second * 8, st));
+    }
+    for (Active &a : s->active) a.cleared = true;
     return PTW_OK;
 }
 
@@ -458,9 +472,7 @@ try {
     cudaStream_t st = s->g->stream;
     const uint32_t n = s->g->dg.n;
     const size_t done_before = s->done.size();
-    // 1. admission: FIFO while a slot and a table fit.  Their tables are cleared
-    // together, neighbours in one piece (300 queries at once: 300 clears of 2 us).
-    std::vector<std::pair<uint64_t, uint64_t>> fresh;  // {arena offset, slots}
+    // 1. admission: FIFO while a slot and a table fit; their tables are cleared together
     while (!s->pending.empty() && s->active.size() < s->S) {
         Pending &pd = s->pending.front();
         const TableSize ts = pd.full ? dense_table(n)
@@ -473,7 +485,6 @@ try {
                 return fail(PTW_ENOMEM, "a query's count table is larger than the whole table arena");
             break;
         }
-        fresh.emplace_back(off, (cap + 1) & ~1ull);  // (a dense table's n counters may end in half a slot pair)
         Active a;
         a.p = pd;
         a.cap = cap;
@@ -481,10 +492,11 @@ try {
         a.off = off;
         a.started = 0;
         a.admit_s = now_s(s);
+        a.cleared = false;
         s->active.push_back(a);
         s->pending.pop_front();
     }
-    if (const int rc0 = clear_tables(s, fresh)) return rc0;
+    if (const int rc0 = clear_tables(s)) return rc0;
     uint32_t nd = 0;
     if (!s->active.empty()) {
         // 2. plan: a fair share of the tick's walkers per active query
@@ -769,7 +781,8 @@ try {
         out.put(&dense);
         out.put(&a.cap);
         tab.resize(a.cap);
-        PTW_CUDA(cudaMemcpy(tab.data(), s->arena + a.off, a.cap * 8, cudaMemcpyDeviceToHost));
+        if (a.cleared) PTW_CUDA(cudaMemcpy(tab.data(), s->arena + a.off, a.cap * 8, cudaMemcpyDeviceToHost));
+        else std::fill(tab.begin(), tab.end(), 0ull);
         out.put(tab.data(), tab.size());
     }
     for (const Done &d : s->done) {
@@ -864,6 +877,7 @@ try {
             return bail(fail(PTW_ENOMEM, "the restored server's table arena cannot hold the saved active queries"));
         cudaError_t e = cudaMemcpy(s->arena + a.off, tab.data(), a.cap * 8, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return bail(cuda_fail(e, "restoring a count table"));
+        a.cleared = true;
         s->active.push_back(a);
     }
     // finished results: read, then staged together in one pinned block
