@@ -271,6 +271,7 @@ int upload_and_build(const uint32_t *h_src, const uint32_t *h_dst, uint64_t m, b
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
+        PoolKeep pool(g->stream);
         cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
         if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e == cudaSuccess) e = cudaMemcpyAsync(d_src, h_src, m * 4, cudaMemcpyHostToDevice, g->stream);
@@ -716,8 +717,11 @@ try {
     if (!g) return fail(PTW_ENOMEM, "host allocation failed");
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
-    if (rc == PTW_OK) rc = csr_to_device_edges(h_row_ptr, h_col, h_names, n, &d_src, &d_dst, g->stream);
-    if (rc == PTW_OK) rc = build_graph_from_device_edges(g, d_src, d_dst, m, false, false, false);
+    if (rc == PTW_OK) {
+        PoolKeep pool(g->stream);
+        rc = csr_to_device_edges(h_row_ptr, h_col, h_names, n, &d_src, &d_dst, g->stream);
+        if (rc == PTW_OK) rc = build_graph_from_device_edges(g, d_src, d_dst, m, false, false, false);
+    }
     if (rc != PTW_OK) {
         graph_release(g);
         delete g;
@@ -750,6 +754,7 @@ try {
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
+        PoolKeep pool(g->stream);
         cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
         if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e != cudaSuccess) {
@@ -789,6 +794,7 @@ try {
     int rc = graph_init_handle(g);
     uint32_t *d_src = nullptr, *d_dst = nullptr;
     if (rc == PTW_OK) {
+        PoolKeep pool(g->stream);
         cudaError_t e = pooled_alloc_async((void **)&d_src, m * 4, g->stream);
         if (e == cudaSuccess) e = pooled_alloc_async((void **)&d_dst, m * 4, g->stream);
         if (e != cudaSuccess) {

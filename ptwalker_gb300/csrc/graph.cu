@@ -27,7 +27,6 @@ namespace ptw {
 namespace {
 
 constexpr int kThreads = 256;
-constexpr uint64_t kBuildPoolKeep = 1ull << 30;
 
 inline unsigned grid_for(uint64_t n, int threads = kThreads)
 {
@@ -551,13 +550,15 @@ int alloc_arrays(ptw_graph *g, uint32_t n, uint64_t m, uint32_t max_runs)
     return PTW_OK;
 }
 
+}  // namespace
+
 // Device time of 8 M edges, both directions, 3 M names below 12 M: names and keys
 // from a table over the name range 0.26 ms (sorting all endpoints for the distinct
 // ones and searching those for every endpoint: 1.6 ms), the sort of the keys 1.0
 // ms (six passes at 1.7 TB/s of reads and writes), rows and columns 0.3 ms.
 // R-MAT scale 20 7.8 -> 3.6 ms, 22 29 -> 16, 24 119 -> 68; 1,087 edges 449 -> 300 us.
-int build_arrays(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, bool as_undirected, bool clean,
-                 bool compact_names)
+int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, bool as_undirected,
+                                  bool clean, bool compact_names)
 {
     cudaStream_t st = g->stream;
     AsyncBufs tmp(st);
@@ -712,19 +713,6 @@ int build_arrays(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, boo
     return PTW_OK;
 }
 
-}  // namespace
-
-int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m,
-                                  bool as_undirected, bool clean, bool compact_names)
-{
-    // The temporaries come from the pool that batches use: mapping fresh memory
-    // takes longer than a small build.  A large one hands back what it added.
-    const uint64_t before = pool_held();
-    const int rc = build_arrays(g, d_src, d_dst, m, as_undirected, clean, compact_names);
-    release_pool_above(g->stream, std::max(before, kBuildPoolKeep));
-    return rc;
-}
-
 }  // namespace ptw
 
 using namespace ptw;
@@ -750,6 +738,7 @@ try {
     const DeviceGraph &dg = g->dg;
     cudaStream_t st = g->stream;
     PTW_CUDA(cudaSetDevice(g->device));
+    PoolKeep pool(st);
     AsyncBufs tmp(st);
     uint32_t *deg = nullptr, *off = nullptr;
     PTW_CUDA(tmp.alloc(&deg, dg.n + 1ull));

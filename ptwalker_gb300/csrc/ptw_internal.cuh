@@ -428,6 +428,17 @@ cudaError_t pooled_alloc_async(void **p, size_t bytes, cudaStream_t st);
 uint64_t pool_held();
 // Waits for st and unmaps what the pool holds unused above keep bytes.
 void release_pool_above(cudaStream_t st, uint64_t keep);
+// Around a graph's construction or export on st: their buffers come from the pool too
+// (mapping fresh memory takes longer than a small build), and what a large one
+// added to it is handed back at the end, down to 1 GB or what it held before.
+// Declared before the first such allocation, destroyed after the last free.
+struct PoolKeep {
+    cudaStream_t st;
+    uint64_t keep;
+    explicit PoolKeep(cudaStream_t s) : st(s), keep(std::max<uint64_t>(pool_held(), 1ull << 30)) {}
+    PoolKeep(const PoolKeep &) = delete;
+    ~PoolKeep() { release_pool_above(st, keep); }
+};
 // Hands the pools' cached memory back to the CUDA driver.
 void trim_pools();
 // cudaMalloc that, when the device is out of memory, trims the pools and
