@@ -8,6 +8,7 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -1140,7 +1141,10 @@ try {
     const int minbs[] = {0, 2};
     const int hintss[] = {0, 1};
     const int exts[] = {0, 1};
-    WalkLaunch wl = make_launch(&cfg);
+    // Walks of one wave hardly depend on the launch, later ones of more do: for a
+    // request of one wave four waves are timed as well, and both times count.
+    std::vector<uint64_t> sizes{cfg.n_walkers};
+    if (cfg.n_walkers <= one_wave_walkers(g)) sizes.push_back(4 * one_wave_walkers(g));
     // Median time per launch of `reps` timings after one warm-up (the warm-up
     // also builds a column copy the candidate asks for); each timing runs
     // three walks back to back, as a caller's loop of walks does, so the
@@ -1150,37 +1154,40 @@ try {
     // marks a candidate that does not launch.
     if (!g->sc.by_name) PTW_CUDA(device_malloc(&g->sc.by_name, std::max<uint64_t>((uint64_t)g->dg.id_bound * 4, 4)));
     auto time_walk = [&](const ptw_tune &t, int reps, float *med) -> int {
-        std::vector<float> ms(reps);
-        const bool by_name = count_walk_by_name(g, t, cfg.n_walkers);
-        WalkLaunch twl = wl;
-        if (by_name) twl.by_name = g->sc.by_name;
-        for (int rep = -1; rep < reps; ++rep) {
-            PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
-            for (int l = 0; l < 3; ++l) {
-                if (by_name) PTW_CUDA(cudaMemsetAsync(g->sc.by_name, 0, (uint64_t)g->dg.id_bound * 4, g->stream));
-                else PTW_CUDA(cudaMemsetAsync(g->sc.counts, 0, (uint64_t)g->dg.n * 4, g->stream));
-                if (launch_walk(g, twl, t) != PTW_OK) {
-                    *med = -1.f;
-                    return PTW_OK;
+        *med = 0.f;
+        for (uint64_t walkers : sizes) {
+            std::vector<float> ms(reps);
+            const bool by_name = count_walk_by_name(g, t, walkers);
+            cfg.n_walkers = walkers;
+            WalkLaunch twl = make_launch(&cfg);
+            if (by_name) twl.by_name = g->sc.by_name;
+            for (int rep = -1; rep < reps; ++rep) {
+                PTW_CUDA(cudaEventRecord(g->ev[0], g->stream));
+                for (int l = 0; l < 3; ++l) {
+                    if (by_name) PTW_CUDA(cudaMemsetAsync(g->sc.by_name, 0, (uint64_t)g->dg.id_bound * 4, g->stream));
+                    else PTW_CUDA(cudaMemsetAsync(g->sc.counts, 0, (uint64_t)g->dg.n * 4, g->stream));
+                    if (launch_walk(g, twl, t) != PTW_OK ||
+                        (!by_name && launch_counts_by_name(g, g->sc.by_name) != PTW_OK)) {
+                        *med = -1.f;
+                        return PTW_OK;
+                    }
                 }
-                if (!by_name && launch_counts_by_name(g, g->sc.by_name) != PTW_OK) {
-                    *med = -1.f;
-                    return PTW_OK;
-                }
+                PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
+                PTW_CUDA(cudaEventSynchronize(g->ev[1]));
+                float x = 0;
+                PTW_CUDA(cudaEventElapsedTime(&x, g->ev[0], g->ev[1]));
+                if (rep >= 0) ms[rep] = x / 3.f;
             }
-            PTW_CUDA(cudaEventRecord(g->ev[1], g->stream));
-            PTW_CUDA(cudaEventSynchronize(g->ev[1]));
-            float x = 0;
-            PTW_CUDA(cudaEventElapsedTime(&x, g->ev[0], g->ev[1]));
-            if (rep >= 0) ms[rep] = x / 3.f;
+            std::sort(ms.begin(), ms.end());
+            *med += reps % 2 ? ms[reps / 2] : 0.5f * (ms[reps / 2 - 1] + ms[reps / 2]);
         }
-        std::sort(ms.begin(), ms.end());
-        *med = reps % 2 ? ms[reps / 2] : 0.5f * (ms[reps / 2 - 1] + ms[reps / 2]);
         return PTW_OK;
     };
     // Stage 1: every candidate, median of 3.  The candidates differ by a few
     // percent, about the launch-to-launch noise, so stage 2 re-times the six
-    // fastest in three interleaved rounds of 5 and keeps the lowest median.
+    // fastest in three interleaved rounds of 5 and keeps the lowest median.  The
+    // library's own choice of launch (walk_launch_is_auto) is timed with them, and
+    // stays unless the other is faster in every round than it in any.
     std::vector<std::pair<float, ptw_tune>> cand;
     for (int ex : exts)
     for (int hn : hintss)
@@ -1239,16 +1246,24 @@ try {
         }
         std::sort(cand.begin(), cand.end(), [](const auto &x, const auto &y) { return x.first < y.first; });
     }
-    cand.resize(std::min<size_t>(cand.size(), 6));
-    std::vector<float> sum(cand.size(), 0.f);
+    size_t own = 0, finals = 6;
+    while (own < cand.size() && !walk_launch_is_auto(cand[own].second)) ++own;
+    if (own >= finals && own < cand.size()) std::swap(cand[finals++], cand[own]);
+    cand.resize(std::min(cand.size(), finals));
+    std::vector<std::array<float, 3>> took(cand.size());
     for (int round = 0; round < 3; ++round)
         for (size_t c = 0; c < cand.size(); ++c) {
-            float med = 0;
-            int rc = time_walk(cand[c].second, 5, &med);
+            const int rc = time_walk(cand[c].second, 5, &took[c][round]);
             if (rc) return rc;
-            sum[c] += med;
         }
-    bt = cand[std::min_element(sum.begin(), sum.end()) - sum.begin()].second;
+    size_t won = 0;
+    for (size_t c = 1; c < cand.size(); ++c)
+        if (took[c][0] + took[c][1] + took[c][2] < took[won][0] + took[won][1] + took[won][2]) won = c;
+    for (size_t c = 0; c < cand.size(); ++c)
+        if (walk_launch_is_auto(cand[c].second) &&
+            *std::max_element(took[won].begin(), took[won].end()) >= *std::min_element(took[c].begin(), took[c].end()))
+            won = c;
+    bt = cand[won].second;
     // DeepWalk: groups per warp x column layout (extended / name-paired /
     // plain), timed on a short fixed-length walk each.
     {

@@ -392,6 +392,9 @@ struct WalkLaunch {
 };
 // The launch parameters a graph is built with.
 ptw_tune default_tune();
+// Walkers of one wave of k_walk_queued: launches of up to that many do not depend on
+// most launch parameters.
+uint64_t one_wave_walkers(const ptw_graph *g);
 // True when the fields of t that count and endpoint walks read are the ones
 // a graph is built with: the library then picks kernel and launch itself.
 bool walk_launch_is_auto(const ptw_tune &t);

@@ -828,10 +828,10 @@ void *pick_walk(bool endpoint, int ilp, bool hot, int min_blocks, int block, boo
 
 namespace ptw {
 
-// Walkers of one wave of k_walk_queued.
-constexpr uint64_t kColumnsStay = 192ull << 20;
-constexpr uint64_t kLocalBytes = 160 * 1024;
-static uint64_t queued_lanes(const ptw_graph *g) { return (uint64_t)g->num_sms * kQueuedBlock; }
+constexpr uint64_t kColumnsStay = 192ull << 20;  // columns up to here stay in L2 for the most part
+constexpr uint64_t kLocalBytes = 160 * 1024;     // row records and columns up to here are copied to shared memory
+
+uint64_t one_wave_walkers(const ptw_graph *g) { return (uint64_t)g->num_sms * kQueuedBlock; }
 
 ptw_tune default_tune()
 {
@@ -870,12 +870,12 @@ static bool paths_launch_is_auto(const ptw_tune &t)
 static bool walk_is_queued(const ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
 {
     return walk_launch_is_auto(t) ||
-           (n_walk <= queued_lanes(g) && !t.warp_agg && !t.gather_slots && !t.blocks_per_sm && t.cache_hints);
+           (n_walk <= one_wave_walkers(g) && !t.warp_agg && !t.gather_slots && !t.blocks_per_sm && t.cache_hints);
 }
 
 bool count_walk_by_name(ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
 {
-    if (walk_is_queued(g, t, n_walk)) return n_walk <= queued_lanes(g);
+    if (walk_is_queued(g, t, n_walk)) return n_walk <= one_wave_walkers(g);
     return !t.gather_slots && !t.warp_agg && (t.ext_columns & 1) && ensure_ext_columns(g);
 }
 
@@ -998,7 +998,7 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
     WalkArgs a = walk_args(g, wl);
     a.chunk = 32;
     if (wl.by_name) a.counts = wl.by_name;
-    const bool one_wave = a.n_walk <= queued_lanes(g);
+    const bool one_wave = a.n_walk <= one_wave_walkers(g);
     const uint64_t per_sm = (a.n_walk + g->num_sms - 1) / g->num_sms;
     const bool group = wl.start_mode == PTW_START_SOURCES && !wl.endpoint;
     // A small graph is copied to shared memory by every block (of 256 threads at
