@@ -14,7 +14,8 @@
 // A training step is 3.6 MFLOP at batch 256: its time is latency.  As five
 // launches per step with one thread per sample or parameter, each waiting on
 // its own loads, and a copy of the loss per step, a step took 155 us.  Now one
-// cluster of 16 CTAs runs the steps of several epochs in one launch (k_mlp_steps):
+// cluster of 16 CTAs runs the steps of several epochs in one launch (k_mlp_steps; one CTA
+// where no such cluster fits):
 // samples are spread over the CTAs in tiles of 16 (a thread makes four of the 64
 // sums of a layer for two samples, weights in shared memory), then every
 // CTA sums the gradients of a sixteenth of the parameters over the whole
@@ -318,11 +319,26 @@ __device__ __forceinline__ void sum_one(float &acc, const float *u, const float 
     }
 }
 
+// f(0) .. f(V - 1).
+template <int V, typename F> __device__ __forceinline__ void each(F f)
+{
+    if constexpr (V == 1) {
+        f(0);
+    } else {
+#pragma unroll 1
+        for (int v = 0; v < V; ++v) f(v);
+    }
+}
+
 // TRAIN: one Adam step per batch of positions; otherwise the gradient of the
-// first batch, into G.
-template <bool TRAIN>
+// first batch, into G.  CTAS: kCluster, the work of one rank each, or 1 where no
+// such cluster fits (a partition of the device): one CTA does that of all ranks in
+// turn, with the same sums in the same order.
+template <bool TRAIN, int CTAS>
 __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a, const __grid_constant__ Norm nm)
 {
+    constexpr int V = kCluster / CTAS;  // ranks per CTA
+    static_assert(V == 1 || CTAS == 1, "one rank per CTA or all in one");
     extern __shared__ __align__(16) float smem[];
     float *w = smem;                     // parameters
     float *w2t = w + kParamsPadded;      // W2 transposed
@@ -331,30 +347,37 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a,
     float *ones = stage + kStageRows * kChunkRow;  // a row of ones
     float *grad = ones + kChunkRow;      // sums, one per thread
     Tile &t = *reinterpret_cast<Tile *>(grad + kStepThreads);
-    const int rank = blockIdx.x;  // one cluster
+    auto rank_of = [](int v) { return V == 1 ? (int)blockIdx.x : v; };  // one cluster
     const int tid = threadIdx.x;
     const uint64_t pol = l2_policy(0);
     for (int i = tid; i < kChunkRow; i += kStepThreads) ones[i] = 1.f;
 
-    // This thread's parameter, with its optimiser state.
-    const int param = param_of(rank, tid);
-    float pP = 0.f, pM = 0.f, pV = 0.f;
-    if (TRAIN && param >= 0) {
-        pP = a.P[param];
-        pM = a.M[param];
-        pV = a.V[param];
-    }
+    // This thread's parameter (of each rank), with its optimiser state.
+    const int own = param_of(rank_of(0), tid);
+    auto param_at = [&](int v) { return V == 1 ? own : param_of(v, tid); };
+    float pP[V] = {}, pM[V] = {}, pV[V] = {};
+    each<V>([&](int v) {
+        const int param = param_at(v);
+        if (TRAIN && param >= 0) {
+            pP[v] = a.P[param];
+            pM[v] = a.M[param];
+            pV[v] = a.V[param];
+        }
+    });
 
     // What it copies of a tile's terms: 16 bytes of row r for r = tid / 64, + 5, ...
     // of tile tid % 64 / 4.
     constexpr int kRowStep = kStepThreads / (4 * kCluster), kRowRounds = (kStageRows + kRowStep - 1) / kRowStep;
     const int c_row = tid / (4 * kCluster), c_tile = tid / 4 % kCluster, c_part = 4 * (tid % 4);
     uint16_t c_from[kRowRounds];
+    auto copied_rows = [&](int rank) {
 #pragma unroll
-    for (int i = 0; i < kRowRounds; ++i) {
-        const int r = c_row + i * kRowStep;
-        c_from[i] = (uint16_t)(r < kStageRows ? staged_row(rank, r) : 0);
-    }
+        for (int i = 0; i < kRowRounds; ++i) {
+            const int r = c_row + i * kRowStep;
+            c_from[i] = (uint16_t)(r < kStageRows ? staged_row(rank, r) : 0);
+        }
+    };
+    if (V == 1) copied_rows(rank_of(0));
 
     // What this thread adds up: threads 0 .. 63 W2 rows i, i + 8 and columns j, j + 8,
     // threads 64 .. 95 W1, threads 96 .. 108 b1, b2, w3 and b3 (sums of d1, d2, a2 e
@@ -380,7 +403,7 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a,
     uint32_t ix = 0, it = 0;  // their samples
     float xv = 0.f, tv = 0.f;
     // position b of epoch ep (the first of the next epoch behind the last)
-    auto ahead_index = [&](uint32_t ep, uint32_t b) {
+    auto ahead_index = [&](int rank, uint32_t ep, uint32_t b) {
         if (b >= a.n) {
             if (!TRAIN || ++ep >= a.epochs) return;
             b = 0;
@@ -394,8 +417,10 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a,
         if (tid < kTileThreads) xv = a.x[(uint64_t)ix * IN + xk];
         if (tid < kTile) tv = a.t[it];
     };
-    ahead_index(0, 0);
-    ahead_values();
+    if (V == 1) {
+        ahead_index(rank_of(0), 0, 0);
+        ahead_values();
+    }
 
     uint32_t flip = 0;
     for (uint32_t ep = 0, step = 0; ep < a.epochs; ++ep)
@@ -412,13 +437,19 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a,
         copy_async(w2t, a.PT, H * H, pol);
         asm volatile("cp.async.commit_group;" ::: "memory");
         asm volatile("cp.async.wait_group 1;" ::: "memory");
-        float acc[2][2] = {};
+        float accs[V][2][2] = {};
         for (uint32_t k0 = 0; k0 < B; k0 += kChunk, flip ^= 1) {
             float *const all = a.terms + (uint64_t)flip * (kCluster * kTermRows * kTile);
             const uint32_t n = B - k0 < kChunk ? (B - k0 + kTile - 1) / kTile * kTile : kChunk;
-            const uint32_t t0 = k0 + rank * kTile;  // first sample of this CTA's tile within the batch
             // ---- forward and backward of this CTA's tile ------------------------------
-            if (t0 < B) {
+            each<V>([&](int v) {
+                const int rank = rank_of(v);
+                const uint32_t t0 = k0 + rank * kTile;  // its first sample within the batch
+                if (t0 >= B) return;
+                if (V != 1) {
+                    ahead_index(rank, ep, b0 + k0);
+                    ahead_values();
+                }
                 if (tid < kTileThreads) t.x[xs][xk] = t0 + xs < B ? (xv - mu) / sd : 0.f;
                 __syncthreads();
                 tile_forward(t, w);
@@ -476,74 +507,86 @@ __global__ void __launch_bounds__(kStepThreads, 1) k_mlp_steps(const StepArgs a,
                     __stcg(reinterpret_cast<float4 *>(all + (uint64_t)rank * (kTermRows * kTile)) + i,
                            make_float4(f[0], f[1], f[2], f[3]));
                 }
-            }
+            });
             asm volatile("cp.async.wait_group 0;" ::: "memory");
             cluster_arrive();
-            ahead_index(ep, k0 + kChunk < B ? b0 + k0 + kChunk : b0 + a.batch);
+            if (V == 1) ahead_index(rank_of(0), ep, k0 + kChunk < B ? b0 + k0 + kChunk : b0 + a.batch);
             cluster_wait();
-            ahead_values();
+            if (V == 1) ahead_values();
             // ---- gradient of this CTA's share, samples in order -----------------------
             // (the next chunk's terms go to the other half of a.terms; whoever writes to
             // this one again has passed the barrier after this copy in every CTA)
-            if (c_tile * kTile < n) {
-                const float *from = all + c_tile * (kTermRows * kTile) + c_part;
-                float *to = stage + c_row * kChunkRow + c_tile * kTile + c_part;
+            each<V>([&](int i_rank) {
+                float(&acc)[2][2] = accs[i_rank];
+                if (V != 1) copied_rows(rank_of(i_rank));
+                if (c_tile * kTile < n) {
+                    const float *from = all + c_tile * (kTermRows * kTile) + c_part;
+                    float *to = stage + c_row * kChunkRow + c_tile * kTile + c_part;
 #pragma unroll
-                for (int i = 0; i < kRowRounds; ++i)
-                    if (c_row + i * kRowStep < kStageRows)
-                        cp_async16(to + i * (kRowStep * kChunkRow), from + c_from[i] * kTile, pol);
-            }
-            cp_async_wait_all();
-            __syncthreads();
-            const float *u = stage + ru * kChunkRow, *v = rv < 0 ? ones : stage + rv * kChunkRow;
-            if (tid < 64) {
-                // A sample whose a1 is 0 adds 0 times d2, which only differs from
-                // leaving it out where d2 is not finite: then the sum is NaN and is
-                // made again with the others only (a test per sample doubles it).
-                float q[2][2] = {{acc[0][0], acc[0][1]}, {acc[1][0], acc[1][1]}};
-                sum_quad<false>(q, u, v, n);
-                if (isnan(q[0][0]) || isnan(q[0][1]) || isnan(q[1][0]) || isnan(q[1][1])) sum_quad<true>(acc, u, v, n);
-                else {
-                    acc[0][0] = q[0][0];
-                    acc[0][1] = q[0][1];
-                    acc[1][0] = q[1][0];
-                    acc[1][1] = q[1][1];
+                    for (int i = 0; i < kRowRounds; ++i)
+                        if (c_row + i * kRowStep < kStageRows)
+                            cp_async16(to + i * (kRowStep * kChunkRow), from + c_from[i] * kTile, pol);
                 }
-            } else if (tid < 96) {
-                sum_one<false>(acc[0][0], u, v, n);
+                cp_async_wait_all();
+                __syncthreads();
+                const float *u = stage + ru * kChunkRow, *v = rv < 0 ? ones : stage + rv * kChunkRow;
+                if (tid < 64) {
+                    // A sample whose a1 is 0 adds 0 times d2, which only differs from
+                    // leaving it out where d2 is not finite: then the sum is NaN and is
+                    // made again with the others only (a test per sample doubles it).
+                    float q[2][2] = {{acc[0][0], acc[0][1]}, {acc[1][0], acc[1][1]}};
+                    sum_quad<false>(q, u, v, n);
+                    if (isnan(q[0][0]) || isnan(q[0][1]) || isnan(q[1][0]) || isnan(q[1][1])) sum_quad<true>(acc, u, v, n);
+                    else {
+                        acc[0][0] = q[0][0];
+                        acc[0][1] = q[0][1];
+                        acc[1][0] = q[1][0];
+                        acc[1][1] = q[1][1];
+                    }
+                } else if (tid < 96) {
+                    sum_one<false>(acc[0][0], u, v, n);
+                } else if (tid < 96 + 13) {
+                    float q = acc[0][0];
+                    sum_one<false>(q, u, v, n);
+                    if (isnan(q)) sum_one<true>(acc[0][0], u, v, n);
+                    else acc[0][0] = q;
+                }
+                if (V != 1) __syncthreads();
+            });
+        }
+        each<V>([&](int v) {
+            const float(&acc)[2][2] = accs[v];
+            const int param = param_at(v);
+            if (tid < 64) {
+                float *g = grad + tid / 8 * 16 + tid % 8;
+                g[0] = acc[0][0];
+                g[8] = acc[0][1];
+                g[8 * 16] = acc[1][0];
+                g[8 * 16 + 8] = acc[1][1];
             } else if (tid < 96 + 13) {
-                float q = acc[0][0];
-                sum_one<false>(q, u, v, n);
-                if (isnan(q)) sum_one<true>(acc[0][0], u, v, n);
-                else acc[0][0] = q;
+                grad[kW2 + tid - 64] = acc[0][0];
             }
-        }
-        if (tid < 64) {
-            float *g = grad + tid / 8 * 16 + tid % 8;
-            g[0] = acc[0][0];
-            g[8] = acc[0][1];
-            g[8 * 16] = acc[1][0];
-            g[8 * 16 + 8] = acc[1][1];
-        } else if (tid < 96 + 13) {
-            grad[kW2 + tid - 64] = acc[0][0];
-        }
-        __syncthreads();
-        if (!TRAIN) {
-            if (param >= 0) a.G[param] = grad[tid];
-            return;
-        }
-        if (param >= 0) {
-            adam(pP, pM, pV, grad[tid], a.lr, a.b1, a.b2, a.eps, c1, c2);
-            __stcg(a.P + param, pP);
-            if (tid < kW2) __stcg(a.PT + (param - OW2) % H * H + (param - OW2) / H, pP);
-        }
+            __syncthreads();
+            if (!TRAIN) {
+                if (param >= 0) a.G[param] = grad[tid];
+            } else if (param >= 0) {
+                adam(pP[v], pM[v], pV[v], grad[tid], a.lr, a.b1, a.b2, a.eps, c1, c2);
+                __stcg(a.P + param, pP[v]);
+                if (tid < kW2) __stcg(a.PT + (param - OW2) % H * H + (param - OW2) / H, pP[v]);
+            }
+            if (V != 1) __syncthreads();
+        });
+        if (!TRAIN) return;
         cluster_arrive();
         cluster_wait();
     }
-    if (TRAIN && param >= 0) {
-        a.M[param] = pM;
-        a.V[param] = pV;
-    }
+    each<V>([&](int v) {
+        const int param = param_at(v);
+        if (TRAIN && param >= 0) {
+            a.M[param] = pM[v];
+            a.V[param] = pV[v];
+        }
+    });
 }
 
 constexpr size_t kStepSmem =
@@ -646,26 +689,46 @@ struct MlpScratch {
     }
 };
 
-// Launches k_mlp_steps as one cluster.
-template <bool TRAIN> int launch_steps(const StepArgs &a, const Norm &nm, cudaStream_t st)
-{
-    const void *fn = (const void *)k_mlp_steps<TRAIN>;
-    PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem));
-    PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+// A launch of k_mlp_steps: one cluster, or one CTA where the device (a partition of
+// it) has no room for a cluster of that size.  Made once per call, used for each
+// of its launches.
+template <bool TRAIN> struct StepLaunch {
     cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = kCluster;
-    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(kCluster);
-    cfg.blockDim = dim3(kStepThreads);
-    cfg.dynamicSmemBytes = kStepSmem;
-    cfg.stream = st;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    PTW_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_steps<TRAIN>, a, nm));
-    return PTW_OK;
-}
+    int init(cudaStream_t st)
+    {
+        const void *fn = (const void *)k_mlp_steps<TRAIN, kCluster>;
+        PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStepSmem));
+        PTW_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr.id = cudaLaunchAttributeClusterDimension;
+        attr.val.clusterDim.x = kCluster;
+        attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+        cfg.gridDim = dim3(kCluster);
+        cfg.blockDim = dim3(kStepThreads);
+        cfg.dynamicSmemBytes = kStepSmem;
+        cfg.stream = st;
+        cfg.attrs = &attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess) {
+            cudaGetLastError();
+            clusters = 0;
+        }
+        if (clusters) return PTW_OK;
+        cfg.gridDim = dim3(1);
+        cfg.attrs = nullptr;
+        cfg.numAttrs = 0;
+        PTW_CUDA(cudaFuncSetAttribute((const void *)k_mlp_steps<TRAIN, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)kStepSmem));
+        return PTW_OK;
+    }
+    int run(const StepArgs &a, const Norm &nm) const
+    {
+        if (cfg.numAttrs) PTW_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_steps<TRAIN, kCluster>, a, nm));
+        else PTW_CUDA(cudaLaunchKernelEx(&cfg, k_mlp_steps<TRAIN, 1>, a, nm));
+        return PTW_OK;
+    }
+};
 
 // Sum of n squared errors as the loss of a batch takes it.
 double mean_loss(const float *lt, uint32_t n)
@@ -833,8 +896,9 @@ try {
     a.loss_terms = s.lt;
     a.n = a.batch = B;
     a.epochs = 1;
-    const int rc = launch_steps<false>(a, host_norm(m), st);
-    if (rc) return rc;
+    StepLaunch<false> steps;
+    if (const int rc = steps.init(st)) return rc;
+    if (const int rc = steps.run(a, host_norm(m))) return rc;
     std::vector<float> lt(h_loss ? B : 0);
     if (h_loss) PTW_CUDA(cudaMemcpyAsync(lt.data(), s.lt, B * 4ull, cudaMemcpyDeviceToHost, st));
     if (h_grad) PTW_CUDA(cudaMemcpyAsync(h_grad, m->grad, PTW_MLP_NPARAMS * 4, cudaMemcpyDeviceToHost, st));
@@ -911,6 +975,8 @@ try {
     a.b2 = 0.999f;
     a.eps = 1e-8f;
     const Norm nm = host_norm(m);
+    StepLaunch<true> steps;
+    if (const int rc = steps.init(st)) return rc;
     std::vector<uint32_t> plan(most * words), order(N);
     std::vector<float> lt((uint64_t)run * N);
     for (uint32_t i = 0; i < N; ++i) order[i] = i;
@@ -938,8 +1004,7 @@ try {
         a.corr = reinterpret_cast<const float *>(d_plan + (uint64_t)E * N);
         a.loss_terms = run ? s.lt + (uint64_t)(ep - ep0) * N : nullptr;
         a.epochs = E;
-        const int rc = launch_steps<true>(a, nm, st);
-        if (rc) return rc;
+        if (const int rc = steps.run(a, nm)) return rc;
         ep += E;
         if (run && (ep == epochs || ep - ep0 == run)) {
             PTW_CUDA(cudaMemcpyAsync(lt.data(), s.lt, (uint64_t)(ep - ep0) * N * 4, cudaMemcpyDeviceToHost, st));
