@@ -1,11 +1,14 @@
-"""Training where the device has no room for a cluster of 16 blocks: gradients and
-parameters bit for bit as elsewhere."""
+"""Training where the device has no room for a cluster of 16 blocks, and where copies
+from pageable memory read it late: gradients and parameters bit for bit as elsewhere."""
 import pytest
 
 import failing_lib
 
 pytestmark = pytest.mark.gpu
 
+# The epochs of a launch double (1, 2, 4, ...): 2^k - 1 of them leave no shorter
+# launch at the end, so that a plan copied too late would still hold sample indices
+# where the launch before it reads them.
 TRAIN = """
     import hashlib
     from ptwalker_gb300 import learned
@@ -29,7 +32,7 @@ def failing(gpu, tmp_path_factory):
     return failing_lib.build("mlp.cu", tmp_path_factory.mktemp("lib"))
 
 
-@pytest.mark.parametrize("what", [failing_lib.NO_CLUSTERS])
+@pytest.mark.parametrize("what", [failing_lib.NO_CLUSTERS, failing_lib.LATE_COPIES])
 def test_training(failing, what):
     want = failing_lib.run(None, TRAIN.format(what=what))
     assert failing_lib.run(failing, TRAIN.format(what=what)) == want
