@@ -310,8 +310,10 @@ typedef struct ptw_batch ptw_batch; /* the sparse results of one batch (host mem
 /* Launch parameters of the batched walker kernel (ptw_ppr_batch only; the
  * serving loop keeps the defaults).  Zero fields take the defaults. */
 typedef struct ptw_batch_tune {
-    uint32_t desc_walkers;  /* walker ranks per work descriptor, 32 .. 65536; 0 = 256 */
-    uint32_t blocks_per_sm; /* walker-kernel blocks (256 threads) per SM; 0 = as many as fit */
+    uint32_t desc_walkers;  /* walker ranks per work descriptor, 32 .. 65536; 0 = by the number of
+                               walkers, 256 at most */
+    uint32_t blocks_per_sm; /* walker-kernel blocks (of 256 threads, or as many threads in fewer
+                               blocks) per SM; 0 = as many as fit */
     uint64_t group_bytes;   /* descriptors interleave over groups of consecutive queries whose
                                count tables add up to about this many bytes, group after group;
                                0 = 384 MiB; UINT64_MAX = all queries in one group */

@@ -487,7 +487,7 @@ int run_wave(ptw_graph *g, const std::vector<WaveQuery> &wq, const ptw_batch_cfg
     if (nd >= (1ull << 32)) return fail(PTW_EINVAL, "wave too large");
     BatchLaunch bl;
     if (const int rc0 = batch_launch(g, ext, a, bl)) return rc0;
-    if (bt.blocks_per_sm) bl.per_sm = std::min<int>(bl.per_sm, (int)bt.blocks_per_sm);
+    limit_blocks(bl, bt.blocks_per_sm);
     const unsigned grid = batch_grid(g, bl, nd);
     // Full lists: host buffers of an estimated size are faulted in on host
     // threads while the walk runs (about 1.1 distinct entries per walker on

@@ -331,9 +331,24 @@ __global__ void __launch_bounds__(kBatchRowsBlock, 2) k_batch_rows(const BatchAr
 struct BatchLaunch {
     const void *fn;
     int block;
+    int most;    // threads of a block at most (row table kernel)
     size_t smem;
     int per_sm;  // blocks per SM
 };
+
+// Holds a launch to `blocks` blocks of 256 threads per SM (0: no limit): the row
+// table kernel to as many threads, in as few blocks as hold them.
+inline void limit_blocks(BatchLaunch &l, uint32_t blocks)
+{
+    if (!blocks) return;
+    if (l.smem) {
+        const int threads = 256 * (int)blocks;
+        l.per_sm = std::min(l.per_sm, (threads + l.most - 1) / l.most);
+        l.most = std::min(l.most, threads / l.per_sm / 32 * 32);
+    } else {
+        l.per_sm = std::min(l.per_sm, (int)blocks);
+    }
+}
 
 // Walker ranks per descriptor for a launch of `walkers` walkers: a warp per
 // descriptor on the whole GPU (48 per SM) before a descriptor gets a second
@@ -350,7 +365,7 @@ inline unsigned batch_grid(const ptw_graph *g, BatchLaunch &l, uint64_t nd)
 {
     if (l.smem) {
         const uint64_t per_sm = (nd + g->num_sms - 1) / g->num_sms;
-        l.block = (int)std::max<uint64_t>(1, std::min<uint64_t>(per_sm, kBatchRowsBlock / 32)) * 32;
+        l.block = (int)std::max<uint64_t>(1, std::min<uint64_t>(per_sm, l.most / 32)) * 32;
     }
     const uint64_t warps = l.block / 32;
     return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)g->num_sms * l.per_sm, (nd + warps - 1) / warps));
@@ -360,7 +375,7 @@ inline int batch_launch(const ptw_graph *g, bool ext, BatchArgs &a, BatchLaunch 
 {
     const bool rows = !ext && g->dg.rows;
     l.fn = ext ? (const void *)k_batch<true> : rows ? (const void *)k_batch_rows : (const void *)k_batch<false>;
-    l.block = rows ? kBatchRowsBlock : 256;  // at most: batch_grid
+    l.block = l.most = rows ? kBatchRowsBlock : 256;  // at most: batch_grid
     l.smem = 0;
     a.col_ext = g->dg.col_ext;
     if (rows) {
