@@ -532,9 +532,7 @@ int run_node2vec(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t L, double p, do
     if (rc) return rc;
     PTW_CUDA(mark(g, 3, timed));
     PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 5 * sizeof(unsigned long long), g->stream));
-    if (cfg->n_walkers && L && !(ensure_ext_columns(g) && ensure_edge_filter(g)))
-        return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
-                                "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
+    if (cfg->n_walkers && L && (rc = ensure_node2vec(g, cfg->n_walkers, p, q))) return rc;
     PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers && L) {
         const uint64_t w0 = cfg->first_walker;
@@ -1104,9 +1102,7 @@ try {
     if (rc) return rc;
     PTW_CUDA(cudaEventRecord(g->ev[3], g->stream));
     PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 5 * sizeof(unsigned long long), g->stream));
-    if (cfg->n_walkers && L && !(ensure_ext_columns(g) && ensure_edge_filter(g)))
-        return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
-                                "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
+    if (cfg->n_walkers && L && (rc = ensure_node2vec(g, cfg->n_walkers, p, q))) return rc;
     const uint32_t ns = cfg->start_mode == PTW_START_SOURCES ? cfg->n_sources : 0;
     rc = paths_to_host(g, cfg, L, h_paths, (int32_t *)stage, [&](uint64_t b, uint64_t e, int32_t *d) -> int {
         // each chunk draws walker ids from a fresh cursor; the counters add up

@@ -522,16 +522,26 @@ LaneArgs lane_args(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, u
 
 }  // namespace
 
+// Every first draw is accepted: the plain columns, while the names stay in L2
+// beside them (scale 18 273 -> 160 us, 20 1,086 -> 719, 22 4,119 -> 3,838; 24
+// 15.3 ms against 18.4).
+static bool first_draw_paths(const ptw_graph *g, uint64_t n_walk, double p, double q)
+{
+    return p == 1.0 && q == 1.0 && g->dg.n <= kFirstDrawNames && paths_rows_apply(g, n_walk);
+}
+
+int ensure_node2vec(ptw_graph *g, uint64_t n_walk, double p, double q)
+{
+    if (first_draw_paths(g, n_walk, p, q) || (ensure_ext_columns(g) && ensure_edge_filter(g))) return PTW_OK;
+    return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
+                            "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
+}
+
 int launch_node2vec(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
                     int start_mode, uint32_t n_sources, double p, double q, const uint64_t thr[3], int32_t *paths)
 {
-    if (!ensure_ext_columns(g) || !ensure_edge_filter(g))
-        return fail(PTW_ENOMEM, "node2vec needs the extended column copy (16 bytes per CSR entry) and "
-                                "the edge filter (2 bytes per CSR entry), which do not fit in device memory");
-    // Every first draw is accepted: the plain columns, while the names stay in L2
-    // beside them (scale 18 273 -> 160 us, 20 1,086 -> 719, 22 4,119 -> 3,838; 24
-    // 15.3 ms against 18.4).
-    if (p == 1.0 && q == 1.0 && g->dg.n <= kFirstDrawNames && paths_rows_apply(g, w_end - w_begin))
+    if (const int rc = ensure_node2vec(g, w_end - w_begin, p, q)) return rc;
+    if (first_draw_paths(g, w_end - w_begin, p, q))
         return launch_paths(g, w_begin, w_end, L, seed, start_mode, n_sources, paths, PTW_TAG_N2V, g->sc.ctrl + 1);
     LaneArgs a = lane_args(g, w_begin, w_end, L, seed, start_mode, n_sources, paths);
     a.thr_ret = thr[0];

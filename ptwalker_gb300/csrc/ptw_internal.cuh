@@ -412,8 +412,11 @@ bool paths_rows_apply(const ptw_graph *g, uint64_t n_walk);
 // Second-order (node2vec) paths (node2vec.cu): thr = acceptance thresholds
 // {return, neighbour of the previous vertex, other} for the envelope
 // max(1/p, 1, 1/q) (p and q pick the folded form on simple symmetric
-// graphs); needs the extended column copy (PTW_ENOMEM when it does not fit).  Moves, candidate draws and
-// row probes accumulate in ctrl[1..3].
+// graphs).  Moves, candidate draws, filter tests and row probes accumulate in
+// ctrl[1..4].  ensure_node2vec builds what the walk of n_walk walkers reads beside
+// the CSR: the extended column copy and the edge filter (PTW_ENOMEM when they do
+// not fit), or nothing for the p = q = 1 walks that k_paths_rows takes.
+int ensure_node2vec(ptw_graph *g, uint64_t n_walk, double p, double q);
 int launch_node2vec(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uint64_t seed,
                     int start_mode, uint32_t n_sources, double p, double q, const uint64_t thr[3],
                     int32_t *paths);
