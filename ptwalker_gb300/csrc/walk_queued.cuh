@@ -166,23 +166,18 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
     }
 
     // ---- while there are more: one walker queued behind each lane's own -----------
-    if (!exhausted) {
+    // (counting by name and LOCAL are launches of one wave, which has no more)
+    if constexpr (!BYNAME && !LOCAL) if (!exhausted) {
         uint64_t qwid = 0;
         uint32_t qv = 0;
         bool queued = false;
-        // Names on the way, of the move's and the adopted start's visit, or
-        // (ENDPOINT) of the end and start of a walk.
-        bool pend = false, spend = false;
-        uint32_t pname = 0, sname = 0, pinc = 0, sinc = 0;
+        // ENDPOINT: the names of a walk's start and end on the way.
+        bool pend = false;
+        uint32_t pname = 0, sname = 0;
         uint64_t pj = 0;
         auto flush_names = [&] {
-            if (ENDPOINT) {
-                if (pend) *reinterpret_cast<uint2 *>(&a.pairs[2 * pj]) = make_uint2(sname, pname);
-            } else if (BYNAME) {
-                if (pend) add_name(pname, pinc);
-                if (spend) add_name(sname, sinc);
-            }
-            pend = spend = false;
+            if (pend) *reinterpret_cast<uint2 *>(&a.pairs[2 * pj]) = make_uint2(sname, pname);
+            pend = false;
         };
         for (;;) {
             // 1. the move's gather
@@ -192,7 +187,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
             const bool done = act && (!go || (uint64_t)ry < a.thr || (a.max_moves && step + 1 >= a.max_moves));
 
             // 2. names that arrived
-            if (ENDPOINT || BYNAME) flush_names();
+            if (ENDPOINT) flush_names();
 
             // 3. the queue
             {
@@ -239,15 +234,8 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
                 if (ENDPOINT) v = nb;
             }
             if (!ENDPOINT) {
-                pinc = visit(go, nb);
-                if (pinc) {
-                    if (BYNAME) {
-                        pname = name_of(nb);
-                        pend = true;
-                    } else {
-                        add(nb, pinc);
-                    }
-                }
+                const uint32_t inc = visit(go, nb);
+                if (inc) add(nb, inc);
             } else if (done) {
                 pj = wid - a.w_begin;
                 sname = name_of(s0);
@@ -255,15 +243,8 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
                 pend = true;
             }
             if (count_start) {
-                sinc = visit(adopt, qv);
-                if (sinc) {
-                    if (BYNAME) {
-                        sname = name_of(qv);
-                        spend = true;
-                    } else {
-                        add(qv, sinc);
-                    }
-                }
+                const uint32_t inc = visit(adopt, qv);
+                if (inc) add(qv, inc);
             }
             if (done) act = false;
             if (adopt) {
@@ -275,7 +256,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
             }
             if (exhausted && !__any_sync(kFull, queued || next < end)) break;
         }
-        if (ENDPOINT || BYNAME) flush_names();
+        if (ENDPOINT) flush_names();
     }
 
     // ---- no more: every lane walks on by itself -------------------------------------
