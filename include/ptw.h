@@ -245,7 +245,8 @@ int ptw_deepwalk_dev(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t L, int32_t 
  * p and q must be positive and finite with max(1/p, 1, 1/q) / min(1/p, 1, 1/q)
  * <= 1024 (PTW_EINVAL otherwise).  Needs the extended column copy (16 bytes
  * per CSR entry) and an edge filter (a blocked Bloom filter, about 2 bytes
- * per CSR entry), both built on first use (PTW_ENOMEM when they do not fit).
+ * per CSR entry), both built on first use (PTW_ENOMEM when they do not fit);
+ * with p = q = 1, untouched path parameters and up to 2^23 vertices the CSR is enough.
  * cfg->sp and cfg->max_moves are ignored. */
 typedef struct ptw_node2vec_stats {
     uint64_t walkers;

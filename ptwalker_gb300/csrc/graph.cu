@@ -514,10 +514,13 @@ std::vector<uint32_t> row_table_image(const std::vector<uint4> &found, uint32_t 
     return img;
 }
 
-// The arrays of a graph.  Those of a small one are one allocation (seven were a fifth
-// of its build); from 1 MB per vertex array on each has its own, in the order in which
-// walks read them: in one block with the row records, names cost DeepWalk 6% (R-MAT
-// scale 22 4,027 against 3,800 us).
+// The arrays of a graph: one allocation up to 1 MB per vertex array, from there on one
+// each, in the order in which walks read them.  The line lies about where the walks'
+// times cross, for a reason not known: DeepWalk, one walker per vertex, 80 positions, apart
+// against in one, R-MAT scale 17 63 against 65 us, 18 (0.7 MB) 142 / 138, 19 (1.3 MB)
+// 266 / 264, 20 565 / 576, 22 3,723 / 3,740; count walks the same up to 18, 19 74 / 76,
+// 22 331 / 342.  One allocation spares a build of scale 10 20 us of 400 and its close
+// 17 of 97, at scale 18 140 of 1,420 and 110 of 195.
 int alloc_arrays(ptw_graph *g, uint32_t n, uint64_t m, uint32_t max_runs)
 {
     DeviceGraph &dg = g->dg;
@@ -556,7 +559,7 @@ int alloc_arrays(ptw_graph *g, uint32_t n, uint64_t m, uint32_t max_runs)
 // from a table over the name range 0.26 ms (sorting all endpoints for the distinct
 // ones and searching those for every endpoint: 1.6 ms), the sort of the keys 1.0
 // ms (six passes at 1.7 TB/s of reads and writes), rows and columns 0.3 ms.
-// R-MAT scale 20 7.8 -> 3.6 ms, 22 29 -> 16, 24 119 -> 68; 1,087 edges 449 -> 300 us.
+// R-MAT scale 20 7.8 -> 3.6 ms, 22 29 -> 16, 24 119 -> 69; 1,087 edges 449 -> 300 us.
 int build_graph_from_device_edges(ptw_graph *g, uint32_t *d_src, uint32_t *d_dst, uint64_t m, bool as_undirected,
                                   bool clean, bool compact_names)
 {

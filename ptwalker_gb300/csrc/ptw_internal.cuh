@@ -387,8 +387,8 @@ struct WalkLaunch {
     uint32_t max_moves = 0;
     bool endpoint = false;     // RWR endpoint app instead of counting
     uint32_t *pairs = nullptr; // endpoint output by walker (names)
-    uint32_t *by_name = nullptr; // count walks: count straight into this by-name array (extended
-                                 // columns; see count_walk_by_name), else into the graph's scratch
+    uint32_t *by_name = nullptr; // count walks: count straight into this by-name array (the launches
+                                 // that count_walk_by_name names), else into the graph's scratch
 };
 // The launch parameters a graph is built with.
 ptw_tune default_tune();

@@ -418,6 +418,7 @@ try {
         a.key1 = (uint32_t)(cfg->seed >> 32);
         a.max_moves = cfg->max_moves;
         a.app = cfg->app;
+        // (columns as effective_tune picks them)
         const bool ext = !g->dg.rows && (g->tune.ext_columns & 1) && ensure_ext_columns(g);
         rc = batch_launch(g, ext, a, s->launch);
         s->uses_ext = ext;
