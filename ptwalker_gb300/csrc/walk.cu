@@ -510,14 +510,6 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
     const uint64_t n_groups = (a.n_walk + 31) / 32;
     const uint64_t warps = (uint64_t)gridDim.x * kPathWarps;
 
-    WalkArgs sa;  // start-vertex helper view
-    sa.start_map = a.start_map;
-    sa.sources = a.sources;
-    sa.n = a.n;
-    sa.key0 = a.key0;
-    sa.key1 = a.key1;
-    sa.n_sources = a.n_sources;
-    sa.start_mode = a.start_mode;
     const uint64_t pol_keep = l2_policy(a.hints ? 1 : 0);   // row records, names
     const uint64_t pol_stream = l2_policy(a.hints ? 2 : 0); // column array
 
@@ -533,7 +525,7 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
             const bool valid = j < a.n_walk;
             wid[g] = a.w_begin + j;
             rows[g] = grp < n_groups ? (uint32_t)umin64(32, a.n_walk - grp * 32) : 0;
-            v[g] = valid ? start_vertex(sa, wid[g]) : 0;
+            v[g] = valid ? walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid[g]) : 0;
             dead[g] = !valid;
             stage[wib][g][lane][0] = valid ? (int32_t)a.int2name[v[g]] : -1;
         }
