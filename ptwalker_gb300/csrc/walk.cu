@@ -1031,10 +1031,7 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
 {
     int rc = check_tune(t);
     if (rc) return rc;
-    if (walk_is_queued(g, t, wl.w_end - wl.w_begin)) {
-        if (t.ext_columns & 1) ensure_ext_columns(g);  // for the launches that read them
-        return launch_walk_queued(g, wl);
-    }
+    if (walk_launch_is_auto(t)) return launch_walk_queued(g, wl);
     const DeviceGraph &dg = g->dg;
     WalkArgs a = walk_args(g, wl);
     a.chunk = (uint32_t)t.chunk;
@@ -1046,14 +1043,6 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     const bool ext = !slots && (t.ext_columns & 1) && ensure_ext_columns(g);
     a.col_ext = g->dg.col_ext;
     a.vtx_ext = g->dg.vtx_ext;
-    // extended columns carry each neighbour's name: count straight into the
-    // caller's by-name array (no scatter after the walk)
-    a.by_name = 0;
-    if (wl.by_name) {
-        if (!(ext && !t.warp_agg && !wl.endpoint)) return fail(PTW_EINVAL, "counting by name needs the plain walk on extended columns");
-        a.by_name = 1;
-        a.counts = wl.by_name;
-    }
     void *fn = slots ? pick_walk_async(wl.endpoint, hot, t.gather_slots)
                : (t.warp_agg && !wl.endpoint) ? pick_walk_agg(t.ilp, hot, ext)
                                               : pick_walk(wl.endpoint, t.ilp, hot, t.min_blocks, t.block, ext);
@@ -1063,6 +1052,16 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     int per_sm = 0;
     PTW_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, t.block, smem));
     if (per_sm < 1) return fail(PTW_EINVAL, "walk kernel does not fit on an SM with this tune");
+    // (a launch that does not fit is refused whatever the number of walkers)
+    if (walk_is_queued(g, t, a.n_walk)) return launch_walk_queued(g, wl);
+    // extended columns carry each neighbour's name: count straight into the
+    // caller's by-name array (no scatter after the walk)
+    a.by_name = 0;
+    if (wl.by_name) {
+        if (!(ext && !t.warp_agg && !wl.endpoint)) return fail(PTW_EINVAL, "counting by name needs the plain walk on extended columns");
+        a.by_name = 1;
+        a.counts = wl.by_name;
+    }
     if (t.blocks_per_sm > 0) per_sm = std::min(per_sm, (int)t.blocks_per_sm);
     uint64_t grid = (uint64_t)g->num_sms * per_sm;
     // No more warps than walker ranges to hand out.
