@@ -49,9 +49,8 @@ struct WalkArgs {
     const uint4 *__restrict__ vtx_ext;       // {id, first column, degree, name} by canonical index
     const uint32_t *__restrict__ start_map;  // canonical index -> internal
     const uint32_t *__restrict__ int2idx;    // internal -> canonical index
-    const uint32_t *__restrict__ sources;    // internal ids (more than one source)
+    const uint32_t *__restrict__ sources;    // internal ids
     const uint32_t *__restrict__ int2name;
-    const uint32_t *__restrict__ rows;       // k_walk_queued: row table (row_table.cuh)
     uint32_t *__restrict__ counts;
     uint32_t *__restrict__ pairs;            // endpoint app: [2 * walkers] names
     unsigned long long *__restrict__ ctrl;   // [0] cursor, [1] moves; k_walk_queued: [8] cursor, [9] moves so far,
@@ -63,25 +62,28 @@ struct WalkArgs {
     uint32_t n;
     uint32_t key0, key1;
     uint32_t n_sources;
-    uint32_t source0;  // the only source
     uint32_t max_moves;
     uint32_t chunk;
     uint32_t hot_k;
-    uint32_t row_runs, row_words;
     int start_mode;
     int hints;  // L2 eviction priorities on (see l2_policy)
     int by_name;  // EXT count walks: counts[] is indexed by vertex name (the caller's output)
 };
 
+// (of its own: k_walk's registers and time depend on the fields beside its own, up to 7%)
+struct QueuedArgs : WalkArgs {
+    const uint32_t *__restrict__ rows;  // row table (row_table.cuh)
+    uint32_t row_runs, row_words;
+    uint32_t source0;  // the only source (sources: more than one)
+};
+
 __device__ __forceinline__ uint32_t start_vertex(const WalkArgs &a, uint64_t wid)
 {
-    if (a.start_mode == PTW_START_SOURCES && a.n_sources == 1) return a.source0;
     return walker_start(a.start_mode, a.start_map, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
 }
 
 __device__ __forceinline__ uint32_t start_index(const WalkArgs &a, uint64_t wid)
 {
-    if (a.start_mode == PTW_START_SOURCES && a.n_sources == 1) return a.int2idx[a.source0];
     return walker_start_index(a.start_mode, a.int2idx, a.sources, a.n, a.n_sources, a.key0, a.key1, wid);
 }
 
@@ -468,13 +470,6 @@ inline size_t async_smem(int slots, int block, uint32_t hot_k)
 struct PathArgs {
     const uint2 *__restrict__ adj;
     const uint32_t *__restrict__ col;
-    const uint32_t *__restrict__ rows;    // k_paths_rows: row table
-    uint32_t row_runs, row_words;
-    unsigned long long *counters;         // k_paths_rows: {moves, draws} of node2vec, or null
-    uint32_t tag;                         // draw tag: "WALK" or "N2"
-    const uint4 *__restrict__ col_ext;    // extended columns: {id, first column, degree, name} per entry
-    const uint4 *__restrict__ vtx_ext;    // and per vertex, by canonical index
-    const uint32_t *__restrict__ int2idx;
     const uint2 *__restrict__ col_named;  // {internal id, name} per column entry
     const uint32_t *__restrict__ start_map;
     const uint32_t *__restrict__ sources;
@@ -488,6 +483,18 @@ struct PathArgs {
     uint32_t n_sources;
     int start_mode;
     int hints;
+};
+
+// (of its own: with these fields among the others k_paths<2> takes 67 registers
+// instead of 52, and 10% longer)
+struct PathRowsArgs : PathArgs {
+    const uint32_t *__restrict__ rows;    // row table
+    uint32_t row_runs, row_words;
+    unsigned long long *counters;         // {moves, draws} of node2vec, or null
+    uint32_t tag;                         // draw tag: "WALK" or "N2"
+    const uint4 *__restrict__ col_ext;    // extended columns: {id, first column, degree, name} per entry
+    const uint4 *__restrict__ vtx_ext;    // and per vertex, by canonical index
+    const uint32_t *__restrict__ int2idx;
 };
 
 constexpr int kPathWarps = 4;  // warps per block
@@ -617,7 +624,7 @@ constexpr uint32_t kPathStage = 32;   // positions collected before they are wri
 // part (kPathExtBytes) k_lane_paths reads more (scale 22 4.1 against 4.7 ms).
 // node2vec with p = q = 1 accepts every first draw: the same walk with its tag.
 template <bool MANY, bool EXT>
-__global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_paths_rows(const PathArgs a)
+__global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_paths_rows(const PathRowsArgs a)
 {
     extern __shared__ __align__(16) uint32_t s_rows[];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -716,6 +723,9 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
         }
     }
 }
+
+// A single source as a list (queued on the stream, as a copy from the host is not).
+__global__ void k_set_source(uint32_t *sources, uint32_t id) { *sources = id; }
 
 __global__ void k_name_columns(const uint32_t *col, const uint32_t *int2name, uint64_t m, uint2 *col_named)
 {
@@ -976,7 +986,6 @@ WalkArgs walk_args(ptw_graph *g, const WalkLaunch &wl)
     a.key0 = (uint32_t)wl.seed;
     a.key1 = (uint32_t)(wl.seed >> 32);
     a.n_sources = wl.n_sources;
-    a.source0 = wl.source0;
     a.max_moves = wl.max_moves;
     a.start_mode = wl.start_mode;
     return a;
@@ -987,8 +996,10 @@ WalkArgs walk_args(ptw_graph *g, const WalkLaunch &wl)
 // that takes, so that all SMs share the walkers.
 int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
 {
-    WalkArgs a = walk_args(g, wl);
+    QueuedArgs a{};
+    static_cast<WalkArgs &>(a) = walk_args(g, wl);
     a.chunk = 32;
+    a.source0 = wl.source0;
     if (wl.by_name) a.counts = wl.by_name;
     const bool one_wave = a.n_walk <= one_wave_walkers(g);
     const uint64_t per_sm = (a.n_walk + g->num_sms - 1) / g->num_sms;
@@ -1069,6 +1080,15 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     const uint64_t max_blocks = std::max<uint64_t>(1, (warps_needed + t.block / 32 - 1) / (t.block / 32));
     grid = std::min(grid, max_blocks);
 
+    if (wl.start_mode == PTW_START_SOURCES && wl.n_sources == 1) {
+        if (!g->sc.sources_cap) {
+            PTW_CUDA(device_malloc(&g->sc.sources, 4));
+            g->sc.sources_cap = 1;
+        }
+        k_set_source<<<1, 1, 0, g->stream>>>(g->sc.sources, wl.source0);
+        PTW_CUDA(cudaGetLastError());
+        a.sources = g->sc.sources;
+    }
     PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 2 * sizeof(unsigned long long), g->stream));
     void *args[] = {&a};
     PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(t.block), args, smem, g->stream));
@@ -1101,7 +1121,7 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
                  int start_mode, uint32_t n_sources, int32_t *paths, uint32_t tag, unsigned long long *counters)
 {
     const DeviceGraph &dg = g->dg;
-    PathArgs a{};
+    PathRowsArgs a{};
     a.adj = dg.adj;
     a.col = dg.col;
     a.start_map = dg.idx2int;
@@ -1178,7 +1198,8 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
     const uint64_t per_block = (uint64_t)kPathWarps * G;
     uint64_t grid = std::min<uint64_t>((uint64_t)g->num_sms * per_sm, (groups + per_block - 1) / per_block);
     grid = std::max<uint64_t>(grid, 1);
-    void *args[] = {&a};
+    PathArgs pa = a;
+    void *args[] = {&pa};
     PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(kPathWarps * 32), args, 0, g->stream));
     return PTW_OK;
 }

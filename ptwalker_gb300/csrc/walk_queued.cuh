@@ -58,10 +58,16 @@ __host__ __device__ __forceinline__ uint64_t local_words(uint32_t n, uint64_t m)
     return local_adj_words(n) + ((m + 3) & ~3ull);
 }
 
+__device__ __forceinline__ uint32_t queued_start(const QueuedArgs &a, uint64_t wid)
+{
+    if (a.start_mode == PTW_START_SOURCES && a.n_sources == 1) return a.source0;
+    return start_vertex(a, wid);
+}
+
 // ROWS: row records from the row table in shared memory instead of adj; LOCAL: row
 // records and columns from shared memory.
 template <bool ENDPOINT, bool HOT, bool BYNAME, bool GROUP, bool ROWS, bool LOCAL = false>
-__global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs a)
+__global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const QueuedArgs a)
 {
     extern __shared__ __align__(16) uint32_t s_mem[];
     const uint32_t *s_rows = s_mem;
@@ -151,7 +157,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
     {
         uint32_t x = 0;
         if (act) {
-            x = start_vertex(a, wid);
+            x = queued_start(a, wid);
             draw(wid, 0);
             rec = row(x);
             v = s0 = x;
@@ -216,7 +222,7 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const WalkArgs 
                 }
                 if (my != ~0ull) {
                     qwid = a.w_begin + my;
-                    qv = start_vertex(a, qwid);
+                    qv = queued_start(a, qwid);
                     queued = true;
                 }
             }
