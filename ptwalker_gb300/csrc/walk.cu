@@ -495,6 +495,7 @@ struct PathRowsArgs : PathArgs {
     const uint4 *__restrict__ col_ext;    // extended columns: {id, first column, degree, name} per entry
     const uint4 *__restrict__ vtx_ext;    // and per vertex, by canonical index
     const uint32_t *__restrict__ int2idx;
+    bool hot_cols;                        // columns through L1
 };
 
 constexpr int kPathWarps = 4;  // warps per block
@@ -587,8 +588,8 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
                 int32_t out = -1;
                 if (!dead[g])
                     out = MODE != 0 ? (int32_t)nm[g]
-                                    : (int32_t)ld_hint_u32(&a.int2name[PTW_IDX(v[g], a.n, a.check, kCheckCounter)],
-                                                           pol_keep);
+                                    : (int32_t)ld_hot_u32(&a.int2name[PTW_IDX(v[g], a.n, a.check, kCheckCounter)],
+                                                          pol_keep);
                 stage[wib][g][lane][p - c0] = out;
             }
         }
@@ -598,6 +599,7 @@ __global__ void __launch_bounds__(kPathWarps * 32) k_paths(const PathArgs a)
 constexpr int kPathRowsBlock = 768;   // many waves: 768 threads per SM (1,024: 5-15% slower)
 constexpr int kPathWaveBlock = 1024;  // one wave
 constexpr uint64_t kPathExtBytes = 512ull << 20;  // extended columns up to here: k_paths_rows
+constexpr uint64_t kPathHotBytes = 1ull << 20;    // columns up to here: through L1
 constexpr uint32_t kPathStage = 32;   // positions collected before they are written
 
 // DeepWalk of a graph whose path parameters are the ones it was built with
@@ -687,11 +689,11 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
                 if (alive) {
                     const uint64_t e = PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, a.check, kCheckColumn);
                     if (EXT) {
-                        const uint4 x = ld_hint_u4(&a.col_ext[e], pol_col);
+                        const uint4 x = ld_line_u4(&a.col_ext[e], pol_col);
                         rec = make_uint2(x.y, x.z);
                         next_name = x.w;
                     } else {
-                        v = ld_line_u32(&a.col[e], pol_col);
+                        v = a.hot_cols ? ld_hot_u32(&a.col[e], pol_col) : ld_line_u32(&a.col[e], pol_col);
                     }
                 }
             }
@@ -1159,6 +1161,7 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
         a.col_ext = g->dg.col_ext;
         a.vtx_ext = g->dg.vtx_ext;
         a.int2idx = dg.int2idx;
+        a.hot_cols = dg.m * sizeof(uint32_t) <= kPathHotBytes || start_mode == PTW_START_SOURCES;
         if (smem > 48 * 1024) PTW_CUDA(allow_shared(fn));
         void *args[] = {&a};
         PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)blocks), dim3(block), args, smem, g->stream));

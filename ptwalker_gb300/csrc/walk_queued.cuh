@@ -122,11 +122,11 @@ __global__ void __launch_bounds__(kQueuedBlock, 1) k_walk_queued(const QueuedArg
     };
     auto gather = [&]() -> uint32_t {
         if (LOCAL) return s_col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)];
-        return ld_line_u32(&a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)],
-                           pol_stream);
+        return ld_hot_u32(&a.col[PTW_IDX((uint64_t)rec.x + __umulhi(rx, rec.y), a.m, &a.ctrl[7], kCheckColumn)],
+                          pol_stream);
     };
     auto name_of = [&](uint32_t x) -> uint32_t {
-        return ld_hint_u32(&a.int2name[PTW_IDX(x, a.n, &a.ctrl[7], kCheckCounter)], pol_keep);
+        return ld_hot_u32(&a.int2name[PTW_IDX(x, a.n, &a.ctrl[7], kCheckCounter)], pol_keep);
     };
     // How much this lane has to add to the count of x (0: another lane adds
     // it, or shared memory took it).

@@ -1,0 +1,50 @@
+"""Walks whose gathers all go to a few lines: their time, and layouts at the sizes where
+the kernels and the way through L1 change."""
+import numpy as np
+import pytest
+
+import oracle
+from oracle.replay import START_SOURCES, START_UNIFORM
+
+pytestmark = pytest.mark.gpu
+
+PATHS = dict(deepwalk=lambda gpu, G, W, src: gpu.deepwalk(G, W, 40, 3, "sources", src, stats=True),
+             deepwalk_one_wave=lambda gpu, G, W, src: gpu.deepwalk(G, 120_000, 80, 3, "sources", src, stats=True),
+             node2vec=lambda gpu, G, W, src: gpu.node2vec(G, W, 10, 0.25, 4.0, 3, "sources", sources=src, stats=True),
+             first_draw=lambda gpu, G, W, src: gpu.node2vec(G, W, 40, 1.0, 1.0, 3, "sources", sources=src, stats=True),
+             pagerank=lambda gpu, G, W, src: gpu.pagerank(G, 4 * W, 0.3, 3, "sources", src, stats=True),
+             rwr=lambda gpu, G, W, src: gpu.rwr(G, 4 * W, 0.3, 3, "sources", src, stats=True))
+
+
+# A graph of some hundred vertices is in L1 of every SM, one of 47,000 (7 MB of columns) is not:
+# the same walks take 0.5 to 1.1 times as long on the small one.  With gathers past
+# L1 they took 1.5 to 7 times as long.
+@pytest.mark.parametrize("ext", [0, 3])
+@pytest.mark.parametrize("call", sorted(PATHS))
+def test_small_graphs_are_no_slower(gpu, call, ext):
+    if ext and call in ("first_draw", "node2vec"):
+        pytest.skip("node2vec reads the extended columns whatever the launch")
+    ms = []
+    for scale in (8, 16):
+        with gpu.Graph.rmat(scale, 8, 0.57, 0.19, 0.19, seed=1, clean=True) as G:
+            if ext:
+                G.tune = gpu.Tune(ext_columns=ext & 2)
+            ms.append(min(PATHS[call](gpu, G, 600_000, [1])[1].kernel_ms for _ in range(5)))
+    assert ms[0] <= 1.35 * ms[1], ms
+
+
+# Entries on both sides of 512 KB (DeepWalk of many walkers: which kernel) and 1 MB
+# (columns through L1) of columns, walkers on both sides of a wave; path lengths with a
+# remainder of a row's 32 staged positions.
+@pytest.mark.parametrize("m", [131_072, 131_073, 262_144, 262_145])
+def test_layout_lines(gpu, m):
+    rng = np.random.default_rng(m)
+    s, d = rng.integers(0, 3000, m).astype(np.uint32), rng.integers(0, 3000, m).astype(np.uint32)
+    canon = oracle.canonical_from_edges(s, d)
+    with gpu.Graph.from_edges(s, d) as G:
+        assert G.m == m
+        for W, L in ((155_648, 33), (155_649, 2), (160_001, 5), (160_001, 31), (156_000, 40)):
+            for start, mode, src in (("uniform", START_UNIFORM, None), ("sources", START_SOURCES, canon.names[[7]])):
+                want = oracle.replay_paths(canon, 0, W, L, 3, mode, src, threads=8)
+                want = np.where(want < 0, -1, canon.names[np.maximum(want, 0)].astype(np.int32))
+                assert np.array_equal(gpu.deepwalk(G, W, L, 3, start, src), want), (W, L, start)
