@@ -600,6 +600,7 @@ constexpr int kPathRowsBlock = 768;   // many waves: 768 threads per SM (1,024: 
 constexpr int kPathWaveBlock = 1024;  // one wave
 constexpr uint64_t kPathExtBytes = 512ull << 20;  // extended columns up to here: k_paths_rows
 constexpr uint64_t kPathHotBytes = 1ull << 20;    // columns up to here: through L1
+constexpr uint64_t kPathPairBytes = 512ull << 10; // columns up to here, many walkers: k_paths
 constexpr uint32_t kPathStage = 32;   // positions collected before they are written
 
 // DeepWalk of a graph whose path parameters are the ones it was built with
@@ -667,14 +668,20 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
             if (!MANY) out.start(a.paths + j * a.L);
         }
         // Writes positions [c0, p) of the group's rows, consecutive lanes
-        // consecutive positions of one row.
+        // consecutive positions of one row (fewer than 32: and of the next rows).
         auto flush = [&](uint32_t c0, uint32_t p) {
             __syncwarp();
-            const uint32_t rows = (uint32_t)umin64(32, a.n_walk - g * 32);
-            int32_t *o = a.paths + g * 32 * a.L + c0 + lane;
-            if (c0 + lane < p)
+            const uint32_t rows = (uint32_t)umin64(32, a.n_walk - g * 32), cols = p - c0;
+            int32_t *o = a.paths + g * 32 * a.L + c0;
+            if (cols == 32) {
 #pragma unroll 4
-                for (uint32_t r = 0; r < rows; ++r) st_hint_s32(o + (uint64_t)r * a.L, stage[r][lane], pol_out);
+                for (uint32_t r = 0; r < rows; ++r) st_hint_s32(o + (uint64_t)r * a.L + lane, stage[r][lane], pol_out);
+            } else {
+                for (uint32_t i = lane; i < rows * cols; i += 32) {
+                    const uint32_t r = i / cols, c = i - r * cols;
+                    st_hint_s32(o + (uint64_t)r * a.L + c, stage[r][c], pol_out);
+                }
+            }
             __syncwarp();
         };
         const bool valid = alive;
@@ -1145,7 +1152,9 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
     a.counters = counters;
     const bool ext = (g->tune.ext_columns & 2) && ensure_ext_columns(g);
     const bool many = path_rows_many(g, a.n_walk);
-    if (paths_rows_apply(g, a.n_walk) || (ext && (!many || dg.m * sizeof(uint4) <= kPathExtBytes))) {
+    // On a small graph with walkers for many waves, the pairs of k_paths are in L1.
+    const bool pairs = many && tag == PTW_TAG_WALK && dg.m * sizeof(uint32_t) <= kPathPairBytes;
+    if ((!pairs && paths_rows_apply(g, a.n_walk)) || (ext && (!many || dg.m * sizeof(uint4) <= kPathExtBytes))) {
         // One wave: as few threads per SM as the walkers take, so that all SMs
         // share them.
         const uint64_t sm_walkers = (a.n_walk + g->num_sms - 1) / g->num_sms;
