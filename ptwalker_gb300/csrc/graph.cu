@@ -743,26 +743,24 @@ try {
     PTW_CUDA(cudaSetDevice(g->device));
     PoolKeep pool(st);
     AsyncBufs tmp(st);
-    uint32_t *deg = nullptr, *off = nullptr;
-    PTW_CUDA(tmp.alloc(&deg, dg.n + 1ull));
-    PTW_CUDA(tmp.alloc(&off, dg.n + 1ull));
-    k_deg_by_index<<<grid_for(dg.n + 1ull), kThreads, 0, st>>>(dg.adj, dg.idx2int, dg.n, deg);
+    // row offsets as the caller takes them, degrees, offsets, columns: one allocation
+    const uint64_t n1 = dg.n + 1ull;
+    unsigned long long *rows = nullptr;
+    PTW_CUDA(tmp.alloc(&rows, (h_row_ptr ? n1 : 0) + n1 + (h_col ? (dg.m + 1) / 2 : 0)));
+    uint32_t *const deg = reinterpret_cast<uint32_t *>(rows + (h_row_ptr ? n1 : 0)), *const off = deg + n1, *const c = off + n1;
+    k_deg_by_index<<<grid_for(n1), kThreads, 0, st>>>(dg.adj, dg.idx2int, dg.n, deg);
     PTW_CUDA(cub_call([&](void *t, size_t &b) {
-        return cub::DeviceScan::ExclusiveSum(t, b, deg, off, (int64_t)dg.n + 1, st);
+        return cub::DeviceScan::ExclusiveSum(t, b, deg, off, (int64_t)n1, st);
     }, st));
-    uint32_t *c = nullptr;
     if (h_col) {
-        PTW_CUDA(tmp.alloc(&c, dg.m));
         const uint64_t tiles = (dg.m + kExportTile - 1) / kExportTile;
         k_export<<<grid_for(tiles * 32), kThreads, 0, st>>>(dg.adj, dg.col, dg.int2idx, off, dg.n, dg.m, c);
         PTW_CUDA(cudaGetLastError());
     }
     if (h_row_ptr) {
-        unsigned long long *rows = nullptr;
-        PTW_CUDA(tmp.alloc(&rows, dg.n + 1ull));
-        k_widen<<<grid_for(dg.n + 1ull), kThreads, 0, st>>>(off, dg.n + 1ull, rows);
+        k_widen<<<grid_for(n1), kThreads, 0, st>>>(off, n1, rows);
         PTW_CUDA(cudaGetLastError());
-        PTW_CUDA(cudaMemcpyAsync(h_row_ptr, rows, (dg.n + 1ull) * 8, cudaMemcpyDeviceToHost, st));
+        PTW_CUDA(cudaMemcpyAsync(h_row_ptr, rows, n1 * 8, cudaMemcpyDeviceToHost, st));
     }
     if (h_col) PTW_CUDA(cudaMemcpyAsync(h_col, c, dg.m * 4, cudaMemcpyDeviceToHost, st));
     if (h_names) std::memcpy(h_names, g->h_names, (uint64_t)dg.n * 4);
