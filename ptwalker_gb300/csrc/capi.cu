@@ -1138,9 +1138,9 @@ try {
     const int hintss[] = {0, 1};
     const int exts[] = {0, 1};
     // Walks of one wave hardly depend on the launch, later ones of more do: for a
-    // request of one wave four waves are timed as well, and both times count.
+    // request of one wave two waves are timed as well, and both times count.
     std::vector<uint64_t> sizes{cfg.n_walkers};
-    if (cfg.n_walkers <= one_wave_walkers(g)) sizes.push_back(4 * one_wave_walkers(g));
+    if (cfg.n_walkers <= one_wave_walkers(g)) sizes.push_back(2 * one_wave_walkers(g));
     // Median time per launch of `reps` timings after one warm-up (the warm-up
     // also builds a column copy the candidate asks for); each timing runs
     // three walks back to back, as a caller's loop of walks does, so the
@@ -1149,9 +1149,21 @@ try {
     // on extended columns, a scatter by name otherwise.  A negative time
     // marks a candidate that does not launch.
     if (!g->sc.by_name) PTW_CUDA(device_malloc(&g->sc.by_name, std::max<uint64_t>((uint64_t)g->dg.id_bound * 4, 4)));
+    // A candidate whose warm-up takes twice the fastest so far is not timed
+    // further (unless the warm-up built the columns), nor the one launch that most
+    // take for a request of one wave.
+    float fastest[2] = {1e30f, 1e30f};  // per size
+    float one_wave_ms = 0.f;
     auto time_walk = [&](const ptw_tune &t, int reps, float *med) -> int {
         *med = 0.f;
-        for (uint64_t walkers : sizes) {
+        for (size_t z = 0; z < sizes.size(); ++z) {
+            const uint64_t walkers = sizes[z];
+            const bool had_ext = g->dg.col_ext != nullptr;
+            const bool common = sizes.size() > 1 && z == 0 && walk_is_queued(g, t, walkers);
+            if (common && one_wave_ms > 0.f) {
+                *med += one_wave_ms;
+                continue;
+            }
             std::vector<float> ms(reps);
             const bool by_name = count_walk_by_name(g, t, walkers);
             cfg.n_walkers = walkers;
@@ -1173,9 +1185,16 @@ try {
                 float x = 0;
                 PTW_CUDA(cudaEventElapsedTime(&x, g->ev[0], g->ev[1]));
                 if (rep >= 0) ms[rep] = x / 3.f;
+                else if (x / 3.f > 2.f * fastest[z] && had_ext == (g->dg.col_ext != nullptr)) {
+                    std::fill(ms.begin(), ms.end(), x / 3.f);
+                    break;
+                }
             }
             std::sort(ms.begin(), ms.end());
-            *med += reps % 2 ? ms[reps / 2] : 0.5f * (ms[reps / 2 - 1] + ms[reps / 2]);
+            const float m = reps % 2 ? ms[reps / 2] : 0.5f * (ms[reps / 2 - 1] + ms[reps / 2]);
+            fastest[z] = std::min(fastest[z], m);
+            if (common) one_wave_ms = m;
+            *med += m;
         }
         return PTW_OK;
     };

@@ -399,6 +399,8 @@ ptw_tune default_tune();
 // Walkers of one wave of k_walk_queued: launches of up to that many do not depend on
 // most launch parameters.
 uint64_t one_wave_walkers(const ptw_graph *g);
+// True when k_walk_queued takes a walk of n_walk walkers under t.
+bool walk_is_queued(const ptw_graph *g, const ptw_tune &t, uint64_t n_walk);
 // True when the fields of t that count and endpoint walks read are the ones
 // a graph is built with: the library then picks kernel and launch itself.
 bool walk_launch_is_auto(const ptw_tune &t);

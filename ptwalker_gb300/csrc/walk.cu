@@ -878,7 +878,7 @@ static bool paths_launch_is_auto(const ptw_tune &t)
 // walkers on R-MAT scales 10 to 22 (30,000 at scale 16 77 us against 54, 100,000 at
 // scale 20 94 against 73; of 300,000 on either may win).  Merged visits, walkers in
 // shared memory and a limit on blocks stay what they say.
-static bool walk_is_queued(const ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
+bool walk_is_queued(const ptw_graph *g, const ptw_tune &t, uint64_t n_walk)
 {
     return walk_launch_is_auto(t) ||
            (n_walk <= one_wave_walkers(g) && !t.warp_agg && !t.gather_slots && !t.blocks_per_sm && t.cache_hints);
