@@ -600,7 +600,7 @@ constexpr int kPathRowsBlock = 768;   // many waves: 768 threads per SM (1,024: 
 constexpr int kPathWaveBlock = 1024;  // one wave
 constexpr uint64_t kPathExtBytes = 512ull << 20;  // extended columns up to here: k_paths_rows
 constexpr uint64_t kPathHotBytes = 1ull << 20;    // columns up to here: through L1
-constexpr uint64_t kPathPairBytes = 512ull << 10; // columns up to here, many walkers: k_paths
+constexpr uint64_t kPathPairBytes = 512ull << 10; // columns up to here, many walkers: k_paths (short paths: twice)
 constexpr uint32_t kPathStage = 32;   // positions collected before they are written
 
 // DeepWalk of a graph whose path parameters are the ones it was built with
@@ -1157,7 +1157,7 @@ int launch_paths(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_t L, uin
     const bool ext = (g->tune.ext_columns & 2) && ensure_ext_columns(g);
     const bool many = path_rows_many(g, a.n_walk);
     // On a small graph with walkers for many waves, the pairs of k_paths are in L1.
-    const bool pairs = many && tag == PTW_TAG_WALK && dg.m * sizeof(uint32_t) <= kPathPairBytes;
+    const bool pairs = many && tag == PTW_TAG_WALK && dg.m * sizeof(uint32_t) <= (L <= 8 ? 2 : 1) * kPathPairBytes;
     if ((!pairs && paths_rows_apply(g, a.n_walk)) || (ext && (!many || dg.m * sizeof(uint4) <= kPathExtBytes))) {
         // One wave: as few threads per SM as the walkers take, so that all SMs
         // share them.
