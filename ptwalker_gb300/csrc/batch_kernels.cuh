@@ -259,7 +259,10 @@ __device__ __forceinline__ void batch_body(const BatchArgs &a, const uint32_t *s
                     nrec[k] = make_uint2(x.y, x.z);
                     nidx[k] = x.w;  // the neighbour's name: its canonical index when a.ext_idx
                 } else {
-                    nb[k] = ld_line_u32(&a.col[PTW_IDX(e, a.m, a.check, kCheckColumn)], pol_col);
+                    // (columns up to 1 MB through L1: 300 queries on 213 vertices 1,861 -> 1,367 us,
+                    // 895 and more vertices the same; of large graphs 0.5% slower)
+                    const uint32_t *p = &a.col[PTW_IDX(e, a.m, a.check, kCheckColumn)];
+                    nb[k] = a.m <= (1u << 18) ? ld_hot_u32(p, pol_col) : ld_line_u32(p, pol_col);
                 }
             }
         }
