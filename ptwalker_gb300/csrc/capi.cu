@@ -118,13 +118,15 @@ uint64_t pool_held()
     return held;
 }
 
-void release_pool_above(cudaStream_t st, uint64_t keep)
+void release_pool_above(cudaStream_t st, uint64_t keep, uint64_t spare)
 {
     int dev = 0;
-    if (pool_held() <= keep || cudaGetDevice(&dev) != cudaSuccess) return;
+    if (pool_held() <= std::max(keep, spare) || cudaGetDevice(&dev) != cudaSuccess) return;
     cudaStreamSynchronize(st);  // frees queued on st have happened
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    cudaMemPoolTrimTo(g_pools[dev], keep);
+    uint64_t used = 0;
+    if (cudaMemPoolGetAttribute(g_pools[dev], cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) used = 0;
+    cudaMemPoolTrimTo(g_pools[dev], std::max(keep, used + spare));
 }
 
 cudaError_t device_malloc_bytes(void **p, size_t bytes)

@@ -438,18 +438,19 @@ int launch_lane_deepwalk(ptw_graph *g, uint64_t w_begin, uint64_t w_end, uint32_
 cudaError_t pooled_alloc_async(void **p, size_t bytes, cudaStream_t st);
 // Bytes that the current device's pool holds mapped.
 uint64_t pool_held();
-// Waits for st and unmaps what the pool holds unused above keep bytes.
-void release_pool_above(cudaStream_t st, uint64_t keep);
+// Waits for st and unmaps what the pool holds above keep bytes and above spare bytes
+// that are not in use.
+void release_pool_above(cudaStream_t st, uint64_t keep, uint64_t spare);
 // Around a graph's construction or export on st: their buffers come from the pool too
 // (mapping fresh memory takes longer than a small build), and what a large one
-// added to it is handed back at the end, down to 1 GB or what it held before.
-// Declared before the first such allocation, destroyed after the last free.
+// added to it is handed back at the end, down to 1 GB not in use or what it held
+// before.  Declared before the first such allocation, destroyed after the last free.
 struct PoolKeep {
     cudaStream_t st;
-    uint64_t keep;
-    explicit PoolKeep(cudaStream_t s) : st(s), keep(std::max<uint64_t>(pool_held(), 1ull << 30)) {}
+    uint64_t before;
+    explicit PoolKeep(cudaStream_t s) : st(s), before(pool_held()) {}
     PoolKeep(const PoolKeep &) = delete;
-    ~PoolKeep() { release_pool_above(st, keep); }
+    ~PoolKeep() { release_pool_above(st, before, 1ull << 30); }
 };
 // Hands the pools' cached memory back to the CUDA driver.
 void trim_pools();
