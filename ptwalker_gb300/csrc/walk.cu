@@ -609,7 +609,8 @@ constexpr uint32_t kPathStage = 32;   // positions collected before they are wri
 // gather from the plain columns; no column copy is built or read.  The
 // neighbour's name is loaded beside the next gather, through L1 (the hubs'
 // names are asked for by all SMs), and the draw of a move is made while the
-// gather before it is on its way.
+// gather before it is on its way.  The columns come through L1 where their lines
+// are shared (hot_cols): on small graphs and from given sources.
 // MANY (more walkers than one wave): the row comes from the row table in shared
 // memory, and a warp's paths are collected there and written 32 positions of
 // one row at a time, first to be evicted from L2: in pieces of 16 bytes they
@@ -626,6 +627,10 @@ constexpr uint32_t kPathStage = 32;   // positions collected before they are wri
 // 216, 19 606 -> 475, 20 1,127 -> 1,080 us; of columns that DRAM holds for the most
 // part (kPathExtBytes) k_lane_paths reads more (scale 22 4.1 against 4.7 ms).
 // node2vec with p = q = 1 accepts every first draw: the same walk with its tag.
+// Many walkers on columns of up to kPathPairBytes are left to k_paths, whose id and
+// name come with one read that hits L1: 2 M walkers, 20 positions, scale 8 208 against
+// 238 us, 11 247 / 282, 12 267 / 286; scale 13 (0.8 MB) 283 / 285, but 5 positions
+// 94 / 104.
 template <bool MANY, bool EXT>
 __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_paths_rows(const PathRowsArgs a)
 {

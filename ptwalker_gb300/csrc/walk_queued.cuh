@@ -19,7 +19,7 @@
 //    steps;
 //  - ROWS: with more walkers than lanes the row of a vertex comes from the row
 //    table in shared memory (row_table.cuh), which leaves one gather per move;
-//    a 4-byte one, from the plain columns.  In one wave the L2 load of
+//    a 4-byte one, from the plain columns, through L1 (ld_hot_u32).  In one wave the L2 load of
 //    adj[v] is as quick as the lookup and the table need not be copied;
 //  - LOCAL: in one wave on a small graph, row records and columns are copied to
 //    shared memory, and the chain of a move is its draw and two reads there;
