@@ -313,8 +313,8 @@ int check_cfg(const ptw_graph *g, const ptw_walk_cfg *cfg, bool needs_sp)
 }
 
 // Maps source names to internal ids and uploads them to the scratch table.
-// With `only`, a single source's id is stored there instead (it travels as a
-// kernel argument, without a copy to wait for).
+// With `only`, a single source's canonical index is stored there instead (it travels
+// with the launch, without a copy to wait for).
 int upload_sources(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *only = nullptr)
 {
     if (cfg->start_mode != PTW_START_SOURCES) return PTW_OK;
@@ -325,11 +325,11 @@ int upload_sources(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *only = nullp
         const uint32_t *p = std::lower_bound(g->h_names, g->h_names + n, nm);
         if (p == g->h_names + n || *p != nm)
             return fail(PTW_EINVAL, "source " + std::to_string(nm) + " is not a vertex of the graph");
+        if (only && cfg->n_sources == 1) {
+            *only = (uint32_t)(p - g->h_names);
+            return PTW_OK;
+        }
         ids[i] = g->h_idx2int[p - g->h_names];
-    }
-    if (only && ids.size() == 1) {
-        *only = ids[0];
-        return PTW_OK;
     }
     if (g->sc.sources_cap < cfg->n_sources) {
         cudaFree(g->sc.sources);
@@ -358,10 +358,10 @@ int stage_bytes(ptw_graph *g, size_t bytes, void **out)
     return PTW_OK;
 }
 
-WalkLaunch make_launch(const ptw_walk_cfg *cfg, uint32_t source0 = 0)
+WalkLaunch make_launch(const ptw_walk_cfg *cfg, uint32_t source_index = 0)
 {
     WalkLaunch wl;
-    wl.source0 = source0;
+    wl.source_index = source_index;
     wl.w_begin = cfg->first_walker;
     wl.w_end = wl.w_begin + cfg->n_walkers;
     wl.thr = stop_threshold(cfg->sp);
@@ -400,8 +400,8 @@ cudaError_t mark(ptw_graph *g, int ev, bool timed)
 // into d_by_name.  Events (timed): ev3 first, ev0 before, ev1 after the kernel.
 int run_count(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_by_name, bool timed)
 {
-    uint32_t source0 = 0;
-    int rc = upload_sources(g, cfg, &source0);
+    uint32_t source = 0;
+    int rc = upload_sources(g, cfg, &source);
     if (rc) return rc;
     // on extended columns the walk counts by name into d_by_name itself;
     // otherwise by internal id into the scratch, scattered by name after
@@ -411,7 +411,7 @@ int run_count(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_by_name, bool t
     else PTW_CUDA(cudaMemsetAsync(g->sc.counts, 0, (uint64_t)g->dg.n * 4, g->stream));
     PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers) {
-        WalkLaunch wl = make_launch(cfg, source0);
+        WalkLaunch wl = make_launch(cfg, source);
         if (by_name) wl.by_name = d_by_name;
         rc = launch_walk(g, wl, g->tune);
         if (rc) return rc;
@@ -424,13 +424,13 @@ int run_count(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_by_name, bool t
 
 int run_endpoint(ptw_graph *g, const ptw_walk_cfg *cfg, uint32_t *d_pairs, bool timed)
 {
-    uint32_t source0 = 0;
-    int rc = upload_sources(g, cfg, &source0);
+    uint32_t source = 0;
+    int rc = upload_sources(g, cfg, &source);
     if (rc) return rc;
     PTW_CUDA(mark(g, 3, timed));
     PTW_CUDA(mark(g, 0, timed));
     if (cfg->n_walkers) {
-        WalkLaunch wl = make_launch(cfg, source0);
+        WalkLaunch wl = make_launch(cfg, source);
         wl.endpoint = true;
         wl.pairs = d_pairs;
         rc = launch_walk(g, wl, g->tune);

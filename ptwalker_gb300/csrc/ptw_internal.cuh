@@ -387,7 +387,7 @@ struct WalkLaunch {
     uint64_t seed = 0;
     int start_mode = 0;
     uint32_t n_sources = 0;
-    uint32_t source0 = 0;      // the only source's internal id (n_sources == 1: no list on the device)
+    uint32_t source_index = 0; // the only source's canonical index (n_sources == 1: no list on the device)
     uint32_t max_moves = 0;
     bool endpoint = false;     // RWR endpoint app instead of counting
     uint32_t *pairs = nullptr; // endpoint output by walker (names)

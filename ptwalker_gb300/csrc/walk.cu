@@ -738,9 +738,6 @@ __global__ void __launch_bounds__(MANY ? kPathRowsBlock : kPathWaveBlock, 1) k_p
     }
 }
 
-// A single source as a list (queued on the stream, as a copy from the host is not).
-__global__ void k_set_source(uint32_t *sources, uint32_t id) { *sources = id; }
-
 __global__ void k_name_columns(const uint32_t *col, const uint32_t *int2name, uint64_t m, uint2 *col_named)
 {
     for (uint64_t e = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; e < m; e += (uint64_t)gridDim.x * blockDim.x) {
@@ -1017,7 +1014,7 @@ int launch_walk_queued(ptw_graph *g, const WalkLaunch &wl)
     // with 128; 600,000 47, 41, 41); of longer walks (sp 0.15) all three are alike.
     const uint64_t per_lane = a.n_walk / one_wave_walkers(g);
     a.chunk = per_lane >= 4 ? 128 : per_lane >= 2 ? 64 : 32;
-    a.source0 = wl.source0;
+    a.source0 = g->h_idx2int[wl.source_index];
     if (wl.by_name) a.counts = wl.by_name;
     const bool one_wave = a.n_walk <= one_wave_walkers(g);
     const uint64_t per_sm = (a.n_walk + g->num_sms - 1) / g->num_sms;
@@ -1098,15 +1095,8 @@ int launch_walk(ptw_graph *g, const WalkLaunch &wl, const ptw_tune &t)
     const uint64_t max_blocks = std::max<uint64_t>(1, (warps_needed + t.block / 32 - 1) / (t.block / 32));
     grid = std::min(grid, max_blocks);
 
-    if (wl.start_mode == PTW_START_SOURCES && wl.n_sources == 1) {
-        if (!g->sc.sources_cap) {
-            PTW_CUDA(device_malloc(&g->sc.sources, 4));
-            g->sc.sources_cap = 1;
-        }
-        k_set_source<<<1, 1, 0, g->stream>>>(g->sc.sources, wl.source0);
-        PTW_CUDA(cudaGetLastError());
-        a.sources = g->sc.sources;
-    }
+    // a single source: its entry of the index table is the list
+    if (wl.start_mode == PTW_START_SOURCES && wl.n_sources == 1) a.sources = dg.idx2int + wl.source_index;
     PTW_CUDA(cudaMemsetAsync(g->sc.ctrl, 0, 2 * sizeof(unsigned long long), g->stream));
     void *args[] = {&a};
     PTW_CUDA(cudaLaunchKernel(fn, dim3((unsigned)grid), dim3(t.block), args, smem, g->stream));
